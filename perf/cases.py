@@ -30,7 +30,7 @@ DENSITY, RC, SKIN, DT = 0.85, 2.5, 0.3, 0.001
 FENE_K, FENE_R0, ANGLE_K = 30.0, 1.5, 5.0
 LANGEVIN = "nvt_langevin 1.0 1.0 1.0 {seed}"
 NVT = "nvt_nh 1.0 1.0 0.5 3"
-NPT = "npt_nh 1.0 1.0 0.1 0.0 0.0 1.0 3"
+NPT = "npt_nh 1.0 1.0 0.5 0.0 0.0 10.0 3"
 # two-type pair parameters of the NPT workload: (i, j) -> (epsilon, sigma)
 TWO_TYPES = {(0, 0): (1.0, 1.0), (0, 1): (0.8, 1.0), (1, 1): (1.0, 1.0)}
 TABLE_POINTS, TABLE_LO, TABLE_HI = 2001, 0.05, 2.5
@@ -358,9 +358,9 @@ class _Exact:
         self.listed_at = None
         self.ens, self.step_no = case["ensemble"], 0
         # Nose-Hoover chain of three and the barostat
-        tdamp = {"langevin": 1.0, "nvt": 0.5, "npt": 0.1}[self.ens]
+        tdamp = {"langevin": 1.0, "nvt": 0.5, "npt": 0.5}[self.ens]
         self.M, self.Qr, self.Q1 = 3, tdamp * tdamp, 3.0 * self.n * tdamp * tdamp
-        self.W, self.V0 = 3.0 * self.n + 3.0, self.L ** 3
+        self.W, self.V0 = (3.0 * self.n + 3.0) * 100.0, self.L ** 3  # Pdamp 10
         self.c1 = math.exp(-DT / tdamp)
         self.xi, self.vxi, self.eps_V, self.veps, self.pending = [0.0] * 3, [0.0] * 3, 0.0, 0.0, 1.0
         self.Lpos = self.L
