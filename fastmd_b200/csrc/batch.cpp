@@ -20,6 +20,8 @@
 namespace fmd {
 namespace mixed {
 
+constexpr int kReadPiece = 32768;  // atoms per piece of a state readout (2 MB)
+
 // ------------------------------------------------------------- allocator
 int64_t SegAlloc::alloc(int64_t n) {
   if (n <= 0) n = 1;
@@ -187,6 +189,8 @@ Batch::Batch(const fmd_batch_opts& o, const BatchCaps* exact) {
 Batch::~Batch() {
   if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
   for (auto& e : ev_)
+    if (e) cudaEventDestroy(e);
+  for (auto& e : read_ev_)
     if (e) cudaEventDestroy(e);
   if (st_) cudaStreamDestroy(st_);
   if (side_) cudaStreamDestroy(side_);
@@ -1078,44 +1082,41 @@ void Batch::force_frame(int r, double* xyz, double* box) {
   if (box) *box = rep(r).Lpos;
 }
 
+// The reference wraps positions in the box of the last pre-force update
+// (Lpos); an NPT barostat has changed L since, and positions are reported
+// re-wrapped into the current box L (two wraps, the first one in Lpos).  A
+// replica is read in pieces, each ordered and converted on the device
+// (k_read_state): while one piece is copied into the caller's arrays the next
+// crosses the bus.
 void Batch::read_state(int r, double* xyz, double* vel, int32_t* image, bool rewrap) {
-  const Rep& R = rep(r);
-  const int n = R.natoms;
-  std::vector<float4> hp(n), hv(n);
-  std::vector<int4> hi(n);
-  FMD_CUDA(cudaMemcpyAsync(hp.data(), pos_.p + R.slot_base, n * sizeof(float4), cudaMemcpyDeviceToHost, st_));
-  FMD_CUDA(cudaMemcpyAsync(hv.data(), vel_.p + R.slot_base, n * sizeof(float4), cudaMemcpyDeviceToHost, st_));
-  FMD_CUDA(cudaMemcpyAsync(hi.data(), img_.p + R.slot_base, n * sizeof(int4), cudaMemcpyDeviceToHost, st_));
-  FMD_CUDA(cudaStreamSynchronize(st_));
-  // The reference wraps positions in the box of the last pre-force update
-  // (Lpos); an NPT barostat has changed L since, and positions are reported
-  // re-wrapped into the current box L (two wraps, the first one in Lpos).
-  const double Lp = R.Lpos, L = R.L, h = R.h;
-  for (int s = 0; s < n; ++s) {
-    const int id = hi[s].w;
-    const uint32_t u = w_bits(hp[s].w);
-    const int c[3] = {w_cx(u), w_cy(u), w_cz(u)};
-    const float o[3] = {hp[s].x, hp[s].y, hp[s].z};
-    const int im[3] = {hi[s].x, hi[s].y, hi[s].z};
-    for (int a = 0; a < 3; ++a) {
-      double x = (double)c[a] * h + (double)o[a];
-      int ia = im[a];
-      double fl = std::floor(x / Lp);
-      x -= fl * Lp;
-      ia += (int)fl;
-      if (rewrap) {
-        fl = std::floor(x / L);
-        x -= fl * L;
-        ia += (int)fl;
-      }
-      if (xyz) xyz[3 * id + a] = x;
-      if (image) image[3 * id + a] = ia;
+  const int n = rep(r).natoms, piece = std::min(n, kReadPiece);
+  const size_t bytes = (size_t)piece * kReadBytes;
+  const int pieces = (n + piece - 1) / piece;
+  for (int k = 0; k < std::min(2, pieces); ++k) {
+    if (read_dev_[k].n < bytes) {
+      FMD_CUDA(cudaStreamSynchronize(st_));
+      read_dev_[k].alloc(bytes);
+      read_pin_[k].alloc(bytes);
     }
-    if (vel) {
-      vel[3 * id] = (double)hv[s].x * R.pending_scale;
-      vel[3 * id + 1] = (double)hv[s].y * R.pending_scale;
-      vel[3 * id + 2] = (double)hv[s].z * R.pending_scale;
-    }
+    if (!read_ev_[k]) FMD_CUDA(cudaEventCreateWithFlags(&read_ev_[k], cudaEventDisableTiming));
+  }
+  const Dev d = dev();
+  auto fetch = [&](int k) {
+    const int a0 = k * piece, m = std::min(piece, n - a0);
+    launch_read_state(d, r, a0, m, rewrap, reinterpret_cast<double*>(read_dev_[k & 1].p), st_);
+    FMD_CUDA_LAUNCH();
+    FMD_CUDA(cudaMemcpyAsync(read_pin_[k & 1].p, read_dev_[k & 1].p, (size_t)m * kReadBytes, cudaMemcpyDeviceToHost, st_));
+    FMD_CUDA(cudaEventRecord(read_ev_[k & 1], st_));
+  };
+  fetch(0);
+  for (int k = 0; k < pieces; ++k) {
+    if (k + 1 < pieces) fetch(k + 1);
+    FMD_CUDA(cudaEventSynchronize(read_ev_[k & 1]));
+    const size_t a0 = (size_t)k * piece, m = std::min<size_t>(piece, n - a0);
+    const char* src = read_pin_[k & 1].p;
+    if (xyz) std::memcpy(xyz + 3 * a0, src, m * 24);
+    if (vel) std::memcpy(vel + 3 * a0, src + m * 24, m * 24);
+    if (image) std::memcpy(image + 3 * a0, src + m * 48, m * 12);
   }
 }
 

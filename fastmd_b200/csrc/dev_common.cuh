@@ -57,6 +57,25 @@ struct DevBuf {
   operator T*() const { return p; }
 };
 
+// Page-locked host bytes.
+struct PinBuf {
+  char* p = nullptr;
+  size_t n = 0;
+  PinBuf() = default;
+  PinBuf(const PinBuf&) = delete;
+  PinBuf& operator=(const PinBuf&) = delete;
+  ~PinBuf() {
+    if (p) cudaFreeHost(p);
+  }
+  void alloc(size_t bytes) {
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+    n = 0;
+    FMD_CUDA(cudaMallocHost(&p, bytes));
+    n = bytes;
+  }
+};
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, o);

@@ -339,6 +339,10 @@ void launch_force(const Dev& d, int nchunks, bool ev, int variant, cudaStream_t 
 // Positions (3 floats per atom, id order) of replica r, wrapped in its
 // last pre-force box, into out.
 void launch_pack_frame(const Dev& d, int r, int natoms, float* out, cudaStream_t st);
+// State of atoms [a0, a0 + n) of replica r in id order, in FP64: positions
+// (3 n), velocities (3 n), image flags (3 n ints), packed into out.
+constexpr int kReadBytes = 6 * 8 + 3 * 4;  // per atom
+void launch_read_state(const Dev& d, int r, int a0, int n, bool rewrap, double* out, cudaStream_t st);
 // Work-list offsets of the listed replicas (a step where none rebuilds).
 void launch_rb_plan(const Dev& d, cudaStream_t st);
 // Filters of the listed replicas' pruned lists after their plan, without a

@@ -2532,6 +2532,49 @@ __global__ void __launch_bounds__(256) k_pack_frame(Dev d, int r, float* out) {
   }
 }
 
+// Atoms [a0, a0 + n) of a replica in id order, as the host reads them: the
+// position wrapped in the box of the last pre-force (and, rewrap, then in the
+// current box), the velocity with the pending thermostat scale, the image
+// flags; each operation rounded by itself.  out: 3 n doubles, 3 n doubles, 3 n
+// ints.  One gather per atom through slot_of, coalesced stores; the host loop
+// it replaces (three raw copies, then a scatter by id) took 1.1 ms of a
+// 30,000-bead replica's readout.
+__global__ void __launch_bounds__(256) k_read_state(Dev d, int r, int a0, int n, int rewrap, double* out) {
+  const Rep& R = d.reps[r];
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const int s = R.slot_base + d.slot_of[R.slot_base + a0 + t];
+  const float4 p = d.pos[s], v = d.vel[s];
+  const int4 im = d.img[s];
+  double* const x_out = out + 3 * (size_t)t;
+  double* const v_out = out + 3 * (size_t)n + 3 * (size_t)t;
+  int* const i_out = reinterpret_cast<int*>(out + 6 * (size_t)n) + 3 * (size_t)t;
+  const uint32_t u = w_bits(p.w);
+  const int c[3] = {w_cx(u), w_cy(u), w_cz(u)};
+  const float o[3] = {p.x, p.y, p.z}, vv[3] = {v.x, v.y, v.z};
+  const int ia[3] = {im.x, im.y, im.z};
+  const double h = (double)R.h, Lp = R.Lpos, L = R.L, scale = R.pending_scale;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    double x = __dadd_rn(__dmul_rn((double)c[a], h), (double)o[a]);
+    double fl = floor(__ddiv_rn(x, Lp));
+    int w = ia[a] + (int)fl;
+    x = __dsub_rn(x, __dmul_rn(fl, Lp));
+    if (rewrap) {
+      fl = floor(__ddiv_rn(x, L));
+      x = __dsub_rn(x, __dmul_rn(fl, L));
+      w += (int)fl;
+    }
+    x_out[a] = x;
+    v_out[a] = __dmul_rn((double)vv[a], scale);
+    i_out[a] = w;
+  }
+}
+
+void launch_read_state(const Dev& d, int r, int a0, int n, bool rewrap, double* out, cudaStream_t st) {
+  k_read_state<<<(n + 255) / 256, 256, 0, st>>>(d, r, a0, n, rewrap ? 1 : 0, out);
+}
+
 void launch_pack_frame(const Dev& d, int r, int natoms, float* out, cudaStream_t st) {
   k_pack_frame<<<(natoms + 255) / 256, 256, 0, st>>>(d, r, out);
 }
