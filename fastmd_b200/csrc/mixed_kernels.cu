@@ -2266,37 +2266,66 @@ __global__ void __launch_bounds__(kChunk) k_table(Dev d, int sel) {
     const uint32_t* lst = (pruned ? d.pnbr : d.nbr) + R.nbr_base + ((size_t)(local >> 5) * R.M) * 32 + (local & 31);
     const float4* pbase = d.pos + R.slot_base;
     float fx = 0, fy = 0, fz = 0, pe = 0, v0 = 0, v1 = 0, v2 = 0, v3 = 0, v4 = 0, v5 = 0;
-    for (int k = 0; k < nn; ++k) {
-      const uint32_t w = __ldg(lst + (size_t)k * 32);
-      const float4 pj = __ldg(pbase + (w & kIdxMask));
-      const float3 sh = entry_shift<0>(w, s_shift, nullptr);
-      const float dx = __fsub_rn(__fsub_rn(pi.x, pj.x), sh.x);
-      const float dy = __fsub_rn(__fsub_rn(pi.y, pj.y), sh.y);
-      const float dz = __fsub_rn(__fsub_rn(pi.z, pj.z), sh.z);
-      const float r2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-      const int tid = R.table_of[ti * nt + w_type(w_bits(pj.w))];
-      if (!(r2 < rc2 && r2 > 1e-10f) || tid < 0) continue;
-      const float rmin = R.tab_rmin[tid], rmax = R.tab_rmax[tid], dr = R.tab_dr[tid], inv_dr = R.tab_inv_dr[tid];
-      const int np = R.tab_n[tid];
-      const float rr = fminf(fmaxf(__fsqrt_rn(r2), rmin), rmax);
-      int idx = (int)__fmul_rn(__fsub_rn(rr, rmin), inv_dr);
-      idx = max(0, min(idx, np - 2));
-      const float t = __fmul_rn(__fsub_rn(rr, __fadd_rn(rmin, __fmul_rn((float)idx, dr))), inv_dr);
-      const float2 p0 = __ldg(d.tab + R.tab_off[tid] + idx), p1 = __ldg(d.tab + R.tab_off[tid] + idx + 1);
-      const float fs = __fadd_rn(p0.x, __fmul_rn(t, __fsub_rn(p1.x, p0.x)));
-      const float fxij = __fmul_rn(fs, dx), fyij = __fmul_rn(fs, dy), fzij = __fmul_rn(fs, dz);
-      fx = __fadd_rn(fx, fxij);
-      fy = __fadd_rn(fy, fyij);
-      fz = __fadd_rn(fz, fzij);
-      if (EV) {
-        const float e = __fadd_rn(p0.y, __fmul_rn(t, __fsub_rn(p1.y, p0.y)));
-        pe += 0.5f * e;
-        v0 += 0.5f * fxij * dx;
-        v1 += 0.5f * fxij * dy;
-        v2 += 0.5f * fxij * dz;
-        v3 += 0.5f * fyij * dy;
-        v4 += 0.5f * fyij * dz;
-        v5 += 0.5f * fzij * dz;
+    // Batches of B entries: the list words (loaded a batch ahead), then the
+    // positions, then the table points, each B loads in flight together; the
+    // pairs are added in list order.  (One entry at a time, the pass waits
+    // four dependent loads per entry: 72 us for 24,000 beads.)
+    constexpr int B = 4;
+    uint32_t wn[B];
+#pragma unroll
+    for (int q = 0; q < B; ++q) wn[q] = nn > 0 ? lst[(size_t)q * 32] : 0u;
+    for (int k = 0; k < nn; k += B) {
+      uint32_t w[B];
+#pragma unroll
+      for (int q = 0; q < B; ++q) w[q] = wn[q];
+      if (k + B < nn) {
+#pragma unroll
+        for (int q = 0; q < B; ++q) wn[q] = lst[(size_t)(k + B + q) * 32];
+      }
+      float4 pj[B];
+#pragma unroll
+      for (int q = 0; q < B; ++q) pj[q] = pbase[w[q] & kIdxMask];
+      float dx[B], dy[B], dz[B], t[B];
+      float2 p0[B], p1[B];
+      bool on[B];
+#pragma unroll
+      for (int q = 0; q < B; ++q) {
+        const float3 sh = entry_shift<0>(w[q], s_shift, nullptr);
+        dx[q] = __fsub_rn(__fsub_rn(pi.x, pj[q].x), sh.x);
+        dy[q] = __fsub_rn(__fsub_rn(pi.y, pj[q].y), sh.y);
+        dz[q] = __fsub_rn(__fsub_rn(pi.z, pj[q].z), sh.z);
+        const float r2 = __fadd_rn(__fadd_rn(__fmul_rn(dx[q], dx[q]), __fmul_rn(dy[q], dy[q])), __fmul_rn(dz[q], dz[q]));
+        const int tid = R.table_of[ti * nt + w_type(w_bits(pj[q].w))];
+        on[q] = r2 < rc2 && r2 > 1e-10f && tid >= 0;
+        if (on[q]) {
+          const float rmin = R.tab_rmin[tid], rmax = R.tab_rmax[tid], dr = R.tab_dr[tid], inv_dr = R.tab_inv_dr[tid];
+          const float rr = fminf(fmaxf(__fsqrt_rn(r2), rmin), rmax);
+          int idx = (int)__fmul_rn(__fsub_rn(rr, rmin), inv_dr);
+          idx = max(0, min(idx, R.tab_n[tid] - 2));
+          t[q] = __fmul_rn(__fsub_rn(rr, __fadd_rn(rmin, __fmul_rn((float)idx, dr))), inv_dr);
+          const float2* const points = d.tab + R.tab_off[tid] + idx;
+          p0[q] = __ldg(points);
+          p1[q] = __ldg(points + 1);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < B; ++q) {
+        if (!on[q]) continue;
+        const float fs = __fadd_rn(p0[q].x, __fmul_rn(t[q], __fsub_rn(p1[q].x, p0[q].x)));
+        const float fxij = __fmul_rn(fs, dx[q]), fyij = __fmul_rn(fs, dy[q]), fzij = __fmul_rn(fs, dz[q]);
+        fx = __fadd_rn(fx, fxij);
+        fy = __fadd_rn(fy, fyij);
+        fz = __fadd_rn(fz, fzij);
+        if (EV) {
+          const float e = __fadd_rn(p0[q].y, __fmul_rn(t[q], __fsub_rn(p1[q].y, p0[q].y)));
+          pe += 0.5f * e;
+          v0 += 0.5f * fxij * dx[q];
+          v1 += 0.5f * fxij * dy[q];
+          v2 += 0.5f * fxij * dz[q];
+          v3 += 0.5f * fyij * dy[q];
+          v4 += 0.5f * fyij * dz[q];
+          v5 += 0.5f * fzij * dz[q];
+        }
       }
     }
     float4 f = d.force[s];
