@@ -20,7 +20,14 @@
 namespace fmd {
 namespace mixed {
 
-constexpr int kReadPiece = 32768;  // atoms per piece of a state readout (2 MB)
+// Chunks per resident block up to which k_steps takes a batch (one where a
+// replica has a Nose-Hoover chain).  Measured per 200 steps, graph against
+// resident: 200 x 1,000 beads (2 chunks per block) 21.9 / 19.0 ms, 64 uneven
+// replicas of 342,000 beads in all (4 per block) 40.4 / 38.3 ms; 16 x 30,000
+// NVT (5 per block) 42.4 / 52.2 ms.
+constexpr int kResidentChunks = 4;
+constexpr int kResidentSteps = 1000;  // steps per k_steps launch
+constexpr int kReadPiece = 32768;     // atoms per piece of a state readout (2 MB)
 
 // ------------------------------------------------------------- allocator
 int64_t SegAlloc::alloc(int64_t n) {
@@ -603,15 +610,7 @@ void Batch::finish_pushoffs() {
     h_reps_[r].stop_step = info_[r].pending_pushoff;
   }
   upload_reps();
-  int64_t direct = steps;
-  if (graph_steps_ > 0 && steps >= graph_steps_) {
-    ensure_graph();
-    for (int64_t k = 0; k < steps / graph_steps_; ++k) FMD_CUDA(cudaGraphLaunch(graph_exec_, st_));
-    direct = steps % graph_steps_;
-  }
-  const Dev d = dev();
-  for (int64_t k = 0; k < direct; ++k) launch_step(d, shape(), &host_mode_, st_);
-  FMD_CUDA_LAUNCH();
+  advance(steps);
   FMD_CUDA(cudaStreamSynchronize(st_));
   download_reps();
   complete_pushoffs(pend);
@@ -710,11 +709,88 @@ void Batch::check_status(int r, bool throw_on_fault) {
   throw Error(FMD_ERR_FAULT, "replica fault");
 }
 
-void Batch::advance_direct(int64_t nsteps) {
+// Lanes per atom with which k_steps takes the replicas for which runs(r)
+// holds, 0 where the graph's grids are the better form; their chunks in all.
+template <typename F>
+int Batch::resident_lanes(F runs, int64_t* chunks) const {
+  int groups = 0;
+  bool chained = false;  // a Nose-Hoover chain: a second barrier and a reduction every step
+  *chunks = 0;
+  for (int r = 0; r < max_reps_; ++r) {
+    if (!runs(r)) continue;
+    *chunks += h_reps_[r].nchunks;
+    chained |= h_reps_[r].mode == kModeRun && h_reps_[r].ensemble != FMD_LANGEVIN;
+    ++groups;
+  }
+  if (graph_steps_ <= 0 || groups == 0) return 0;
+  const int lpa = *chunks <= steps_resident_blocks(4) ? 4 : 1;
+  const int cap = steps_resident_blocks(lpa);
+  return groups <= cap && *chunks <= (int64_t)(chained ? 1 : kResidentChunks) * cap ? lpa : 0;
+}
+
+// The replicas with steps left as groups of resident blocks (k_steps): the
+// fewest chunks per block for which every group fits the GPU at once.  False
+// where the step graph is used instead.
+bool Batch::plan_resident() {
+  if (!steps_variant(force_variant_)) return false;
+  auto runs = [&](int r) { return info_[r].used && h_reps_[r].active && h_reps_[r].step < h_reps_[r].stop_step; };
+  int64_t chunks = 0;
+  const int lpa = resident_lanes(runs, &chunks);
+  if (!lpa) return false;
+  const int cap = steps_resident_blocks(lpa);
+  int most = 0;
+  for (int r = 0; r < max_reps_; ++r)
+    if (runs(r)) most = std::max(most, h_reps_[r].nchunks);
+  int per = (int)((chunks + cap - 1) / cap);
+  for (; per < most; ++per) {
+    int64_t blocks = 0;
+    for (int r = 0; r < max_reps_; ++r)
+      if (runs(r)) blocks += (h_reps_[r].nchunks + per - 1) / per;
+    if (blocks <= cap) break;
+  }
+  new_plan_.clear();
+  for (int r = 0; r < max_reps_; ++r) {
+    if (!runs(r)) continue;
+    const int nb = (h_reps_[r].nchunks + per - 1) / per, first = (int)new_plan_.size();
+    for (int b = 0; b < nb; ++b) new_plan_.push_back(make_int4(r, b, nb, first));
+  }
+  const size_t room = std::max(steps_resident_blocks(1), steps_resident_blocks(4));
+  if (plan_.n < room) {
+    plan_.alloc(room);
+    flags_.alloc(2 * room);
+    h_plan_.clear();
+  }
+  lpa_ = lpa;
+  const bool same = new_plan_.size() == h_plan_.size() &&
+                    std::memcmp(new_plan_.data(), h_plan_.data(), h_plan_.size() * sizeof(int4)) == 0;
+  if (!same) {
+    h_plan_ = new_plan_;
+    seq_ = 0;  // no word of another layout stays behind
+    FMD_CUDA(cudaMemsetAsync(flags_, 0, flags_.bytes(), st_));
+    FMD_CUDA(cudaMemcpyAsync(plan_, h_plan_.data(), h_plan_.size() * sizeof(int4), cudaMemcpyHostToDevice, st_));
+  }
+  return true;
+}
+
+// Queue nsteps steps (each replica stops at its own stop_step, as uploaded).
+void Batch::advance(int64_t nsteps) {
   const Dev d = dev();
-    for (int64_t k = 0; k < nsteps; ++k) launch_step(d, shape(), &host_mode_, st_);
+  if (plan_resident()) {
+    while (nsteps > 0) {
+      const int k = (int)std::min<int64_t>(nsteps, kResidentSteps);
+      launch_steps(d, plan_, (int)h_plan_.size(), lpa_, flags_, seq_, force_variant_, k, st_);
+      seq_ += (unsigned)k * kStepBarriers;
+      nsteps -= k;
+    }
+    return;
+  }
+  if (graph_steps_ > 0 && nsteps >= graph_steps_) {
+    ensure_graph();
+    for (int64_t k = 0; k < nsteps / graph_steps_; ++k) FMD_CUDA(cudaGraphLaunch(graph_exec_, st_));
+    nsteps %= graph_steps_;
+  }
+  for (int64_t k = 0; k < nsteps; ++k) launch_step(d, shape(), &host_mode_, st_);
   FMD_CUDA_LAUNCH();
-  FMD_CUDA(cudaStreamSynchronize(st_));
 }
 
 static bool same_shape(const StepShape& a, const StepShape& b) {
@@ -775,17 +851,7 @@ void Batch::run(int64_t nsteps, bool respect_nsteps) {
     return;
   }
   upload_reps();
-  if (graph_steps_ > 0 && need >= graph_steps_) {
-    ensure_graph();
-    const int64_t reps = need / graph_steps_;
-    for (int64_t k = 0; k < reps; ++k) FMD_CUDA(cudaGraphLaunch(graph_exec_, st_));
-    need -= reps * graph_steps_;
-  }
-  if (need > 0) {
-    const Dev d = dev();
-    for (int64_t k = 0; k < need; ++k) launch_step(d, shape(), &host_mode_, st_);
-    FMD_CUDA_LAUNCH();
-  }
+  advance(need);
   FMD_CUDA(cudaStreamSynchronize(st_));
   download_reps();
   if (concurrent_pushoff_) complete_done_pushoffs();
@@ -924,9 +990,13 @@ int Batch::autotune(int iters, double* ms_out, int cap) {
   nbr_variant_ = nb;
   int best = 0;
   double best_ms = 0;
+  // a batch that k_steps takes keeps to the variants built in that form
+  int64_t chunks = 0;
+  const bool resident = resident_lanes([&](int r) { return info_[r].used && h_reps_[r].active; }, &chunks) != 0;
   for (int v = 0; v < kForceVariants; ++v) {
     const double ms = time_force(iters, v, true);
     if (ms_out && v < cap) ms_out[v] = ms;
+    if (resident && !steps_variant(v)) continue;
     if (v == 0 || ms < best_ms) {
       best = v;
       best_ms = ms;

@@ -134,7 +134,10 @@ class Batch {
   void freeze_others(int r);
   void upload_atoms(int r, const double* xyz, const double* vel, const int32_t* image);
   void setup(const std::vector<int>& rs);
-  void advance_direct(int64_t nsteps);
+  void advance(int64_t nsteps);
+  template <typename F>
+  int resident_lanes(F runs, int64_t* chunks) const;
+  bool plan_resident();
   void ensure_graph();
 
   int device_ = 0;
@@ -167,6 +170,11 @@ class Batch {
   DevBuf<float2> tab_;  // pair-table points of every replica (appended at add)
   std::vector<float2> tab_host_;
   DevBuf<int> rb_;  // rebuild work list
+  DevBuf<int4> plan_;      // resident steps: the block plan in use
+  DevBuf<unsigned long long> flags_;  // resident steps: group barrier words
+  unsigned seq_ = 0;                  // and the barriers counted so far
+  int lpa_ = 1;                       // lanes per atom of the plan
+  std::vector<int4> h_plan_, new_plan_;
   // state readout: two device and two pinned buffers of a piece of atoms each
   DevBuf<char> read_dev_[2];
   PinBuf read_pin_[2];

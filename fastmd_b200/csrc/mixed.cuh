@@ -361,6 +361,18 @@ void launch_forces_only(const Dev& d, int nchunks, int variant, bool has_table, 
 void launch_table(const Dev& d, int nchunks, bool ev, int sel, cudaStream_t st);
 void launch_reduce_only(const Dev& d, int nchunks, int nreps, cudaStream_t st, int mode);
 // Scalars of the next pre-force for replicas whose copy a host upload made stale.
+// Resident steps (k_steps): each replica with steps left is advanced by its
+// own group of blocks, up to max_steps steps in one cooperative launch.
+// plan: per block {replica, rank in its group, blocks of the group, first
+// block of the group}, at most steps_resident_blocks(lpa) blocks (lpa: lanes
+// per atom, 1 or 4); flags: 2 words per block, kept between launches; seq:
+// barriers counted so far, at most kStepBarriers per step of each launch.
+// Force variants with several lanes per atom are not built in this form.
+constexpr unsigned kStepBarriers = 16;
+int steps_resident_blocks(int lpa);
+bool steps_variant(int force_variant);
+void launch_steps(const Dev& d, const int4* plan, int blocks, int lpa, unsigned long long* flags, unsigned seq,
+                  int force_variant, int max_steps, cudaStream_t st);
 void launch_prepare(const Dev& d, int nreps, cudaStream_t st);  // 0 setup, 2 re-evaluation
 
 }  // namespace mixed

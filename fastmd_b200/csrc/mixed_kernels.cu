@@ -26,6 +26,9 @@
 // neighbor/skin_trigger.cuh:6-33, analysis/thermo.cu:88-138.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cstddef>
+
 #include "counter_rng.h"
 #include "dev_common.cuh"
 #include "mixed.cuh"
@@ -45,14 +48,21 @@ struct DSinh {
 };
 
 __device__ __forceinline__ double ramp(const Rep& R, int64_t step, double a, double b) {
+  if (a == b) return a;  // the usual constant set point: no division
   const double frac = (double)(step - 1) / (double)(R.nsteps > 0 ? R.nsteps : 1);
   return a + (b - a) * frac;
 }
+
+// a / b for a box ratio, exactly 1 for an unchanged box (no division).
+__device__ __forceinline__ double box_ratio(double a, double b) { return a == b ? 1.0 : a / b; }
 
 // Scalars of the step after R.step.  The single-thread commit kernels inline
 // this into a local and store the result once (next_scalars): through a
 // reference that may point into R (R.next), every store would order the
 // later reads of R behind it, one dependent memory round trip per field.
+// NH: also copy the chain state for a Langevin replica (which leaves it as it
+// is: a caller whose S holds it already does without).
+template <bool NH = true>
 __device__ __forceinline__ void step_scalars(const Rep& R, StepScalars& S) {
   S.adv = R.active && R.step < R.stop_step;
   S.step = R.step + 1;
@@ -67,10 +77,10 @@ __device__ __forceinline__ void step_scalars(const Rep& R, StepScalars& S) {
   S.dh = 0.0f;
   S.h_new = R.h;
   S.h_old = R.h;
-  S.inv_Lold = (float)(1.0 / R.Lpos);
+  S.inv_Lold = 0.0f;
   S.dW = 0.0f;
   S.L_new = R.L;
-  S.nh = R.nh;
+  if (NH || S.ens != FMD_LANGEVIN) S.nh = R.nh;
   if (S.ens == FMD_LANGEVIN) {
     const double kT = (R.mode == kModePushoff) ? R.T0 : ramp(R, S.step, R.T0, R.T1);
     const double c1 = (R.mode == kModePushoff) ? exp(-dt / R.Tdamp) : R.c1;
@@ -90,6 +100,7 @@ __device__ __forceinline__ void step_scalars(const Rep& R, StepScalars& S) {
     S.ev = (float)S.nh.exp_vW;
     S.fpos = (float)S.nh.fpos;
     S.L_new = S.nh.L;
+    S.inv_Lold = (float)(1.0 / R.Lpos);
     const double hn = (double)(float)(S.nh.L / R.G);
     S.h_new = (float)hn;
     S.dh = (float)((double)R.h * S.nh.exp_vW - hn);
@@ -338,13 +349,17 @@ __global__ void __launch_bounds__(32) k_commit(Dev d, StepConds cond) {
   if (cond.use && mode == kRbPrune) cudaGraphSetConditional(cond.prune, 1u);
 }
 
-__device__ void commit_replica(const Dev& d, Rep& R, int r, const StepConds& cond) {
-  StepScalars S;
-  if (R.next_valid) S = R.next;
-  else step_scalars(R, S);
+// What a committed step does with its neighbor lists (Rep::rebuild_now).
+enum ListAction : int { kListKeep = 0, kListRebuild = 1, kListFilter = 2 };
+
+// The pre-force commit on a replica's record R, without side effects outside
+// it: step counter, chain / barostat state, box, and the list decision (also
+// stored in R.rebuild_now).  S: the scalars of the step taken.
+template <bool NH = true>
+__device__ __forceinline__ int commit_state(Rep& R, const StepScalars& S) {
   R.next_valid = 0;
   R.step = S.step;
-  R.nh = S.nh;
+  if (NH || S.ens != FMD_LANGEVIN) R.nh = S.nh;
   R.pending_scale = 1.0;
   if (S.ens == FMD_NPT_NH) {
     R.L = S.L_new;
@@ -365,7 +380,7 @@ __device__ void commit_replica(const Dev& d, Rep& R, int r, const StepConds& con
     R.filter_scale *= (double)S.ev;
   }
   const float maxd2 = __uint_as_float(R.maxdisp_bits);
-  const double s = fmin(R.L / R.L_list, R.list_scale);
+  const double s = fmin(box_ratio(R.L, R.L_list), R.list_scale);
   const float hs = (float)(s < 1.0 ? 0.5 * (s * (R.rc + R.skin) - R.rc) : 0.5 * R.skin);
   const bool trig = hs <= 0.f || maxd2 > hs * hs;
   // With a pruned list (pairs within rc + prune_delta), maxd2 is the
@@ -377,7 +392,7 @@ __device__ void commit_replica(const Dev& d, Rep& R, int r, const StepConds& con
   bool rtrig = trig;
   const float dmax = sqrtf(maxd2);
   if (R.disp_acc > 0.f) rtrig = hs <= 0.f || dmax + R.disp_acc > hs;
-  const double sp = fmin(R.L / R.L_filter, R.filter_scale);
+  const double sp = fmin(box_ratio(R.L, R.L_filter), R.filter_scale);
   const float hp = (float)(sp < 1.0 ? 0.5 * (sp * (R.rc + (double)R.prune_delta) - R.rc) : 0.5 * R.prune_delta);
   const bool ptrig = R.prune_delta > 0.f && (hp <= 0.f || dmax > hp);
   if (rtrig || R.since >= R.max_between) {
@@ -389,25 +404,36 @@ __device__ void commit_replica(const Dev& d, Rep& R, int r, const StepConds& con
     R.maxdisp_bits = 0u;
     R.disp_acc = 0.f;
     R.rebuilds += 1;
-    R.rebuild_now = 1;
-    atomicAdd(d.rb + kRbRebuilds, 1);
-    d.rb[kRbHead + atomicAdd(d.rb + kRbCount, 1)] = r;
+    R.rebuild_now = kListRebuild;
   } else if (ptrig) {
     R.disp_acc += dmax;
     R.maxdisp_bits = 0u;
     R.L_filter = R.L;
     R.filter_scale = 1.0;
-    R.rebuild_now = 2;
-    d.rb[kRbHead + atomicAdd(d.rb + kRbCount, 1)] = r;
+    R.rebuild_now = kListFilter;
   } else {
-    R.rebuild_now = 0;
+    R.rebuild_now = kListKeep;
   }
-  // Langevin steps inside a graph leave their post-force kick to the next
-  // pre-force (the post-force kernel then has nothing else to do); the post
-  // runs on energy steps, for the Nose-Hoover chains and on a replica's last
-  // step of the run, so every state the host can read is complete.
+  return R.rebuild_now;
+}
+
+// Langevin steps leave their post-force kick to the next pre-force (the
+// post-force pass then has nothing else to do); it runs on energy steps, for
+// the Nose-Hoover chains and on a replica's last step of the run, so every
+// state the host can read is complete.
+__device__ __forceinline__ bool post_needed(const Rep& R) {
   const bool langevin = R.mode == kModePushoff || R.ensemble == FMD_LANGEVIN;
-  const bool post = !cond.use || !langevin || need_ev(R) || R.step >= R.stop_step;
+  return !langevin || need_ev(R) || R.step >= R.stop_step;
+}
+
+__device__ void commit_replica(const Dev& d, Rep& R, int r, const StepConds& cond) {
+  StepScalars S;
+  if (R.next_valid) S = R.next;
+  else step_scalars(R, S);
+  const int action = commit_state(R, S);
+  if (action == kListRebuild) atomicAdd(d.rb + kRbRebuilds, 1);
+  if (action != kListKeep) d.rb[kRbHead + atomicAdd(d.rb + kRbCount, 1)] = r;
+  const bool post = !cond.use || post_needed(R);
   R.defer = post ? 0 : 1;
   if (cond.use) {
     // any replica that needs a force variant / a post switches it on
@@ -571,8 +597,8 @@ __device__ __forceinline__ void for_rebuild_chunks(const Dev& d, F body) {
   }
 }
 
-__device__ __forceinline__ void bin_chunk(const Dev& d, const Rep& R, int ci) {
-  const int local = ci * kChunk + threadIdx.x;
+__device__ __forceinline__ void bin_chunk(const Dev& d, const Rep& R, int ci, int t) {
+  const int local = ci * kChunk + t;
   if (local >= R.natoms) return;
   const int s = R.slot_base + local;
   const float4 p = d.pos[s];
@@ -617,7 +643,7 @@ __device__ __forceinline__ void bin_chunk(const Dev& d, const Rep& R, int ci) {
 
 __global__ void __launch_bounds__(kChunk) k_bin(Dev d) {
   count_launch(d, kKBin);
-  for_rebuild_chunks(d, [&](const Rep& R, int, int ci) { bin_chunk(d, R, ci); });
+  for_rebuild_chunks(d, [&](const Rep& R, int, int ci) { bin_chunk(d, R, ci, threadIdx.x); });
 }
 
 // Exclusive scan of the replica's cell counts; one block per replica.
@@ -716,15 +742,17 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(Dev d) {
   }
 }
 
+__device__ __forceinline__ void scatter_chunk(const Dev& d, const Rep& R, int ci, int t) {
+  const int local = ci * kChunk + t;
+  if (local >= R.natoms) return;
+  const int s = R.slot_base + local;
+  const int at = atomicAdd(&d.cell_fill[R.cell_base + d.key[s]], 1);
+  d.bucket[R.slot_base + at] = local;
+}
+
 __global__ void __launch_bounds__(kChunk) k_scatter(Dev d) {
   count_launch(d, kKScatter);
-  for_rebuild_chunks(d, [&](const Rep& R, int, int ci) {
-    const int local = ci * kChunk + threadIdx.x;
-    if (local >= R.natoms) return;
-    const int s = R.slot_base + local;
-    const int at = atomicAdd(&d.cell_fill[R.cell_base + d.key[s]], 1);
-    d.bucket[R.slot_base + at] = local;
-  });
+  for_rebuild_chunks(d, [&](const Rep& R, int, int ci) { scatter_chunk(d, R, ci, threadIdx.x); });
 }
 
 // Per cell: order members by atom id (deterministic), write the permutation.
@@ -772,8 +800,8 @@ __global__ void __launch_bounds__(32 * kCellGroup) k_cellsort(Dev d) {
   }
 }
 
-__device__ __forceinline__ void permute_chunk(const Dev& d, const Rep& R, int ci) {
-  const int local = ci * kChunk + threadIdx.x;
+__device__ __forceinline__ void permute_chunk(const Dev& d, const Rep& R, int ci, int t) {
+  const int local = ci * kChunk + t;
   const int s = R.slot_base + local;
   if (local >= R.natoms) {
     d.ncnt[s] = 0;
@@ -791,13 +819,13 @@ __device__ __forceinline__ void permute_chunk(const Dev& d, const Rep& R, int ci
 
 __global__ void __launch_bounds__(kChunk) k_permute(Dev d) {
   count_launch(d, kKPermute);
-  for_rebuild_chunks(d, [&](const Rep& R, int, int ci) { permute_chunk(d, R, ci); });
+  for_rebuild_chunks(d, [&](const Rep& R, int, int ci) { permute_chunk(d, R, ci, threadIdx.x); });
 }
 
 // Per-slot bonded tables for the new order: partner slots instead of atom
 // ids, so the force kernel reaches a partner's position in one load.
-__device__ __forceinline__ void topo_chunk(const Dev& d, const Rep& R, int ci) {
-  const int local = ci * kChunk + threadIdx.x;
+__device__ __forceinline__ void topo_chunk(const Dev& d, const Rep& R, int ci, int t) {
+  const int local = ci * kChunk + t;
   const int s = R.slot_base + local;
   if (local >= R.natoms) {
     d.tcnt[s] = 0;
@@ -828,14 +856,14 @@ __device__ __forceinline__ void topo_chunk(const Dev& d, const Rep& R, int ci) {
 
 __global__ void __launch_bounds__(kChunk) k_topo(Dev d) {
   count_launch(d, kKTopo);
-  for_rebuild_chunks(d, [&](const Rep& R, int, int ci) { topo_chunk(d, R, ci); });
+  for_rebuild_chunks(d, [&](const Rep& R, int, int ci) { topo_chunk(d, R, ci, threadIdx.x); });
 }
 
 // Verlet list for boxes of fewer than three cells per axis (L < 3 (rc +
 // skin)): one warp per home cell, the distinct neighbor cells de-duplicated,
 // each pair's periodic shift derived from the two cells and offsets.
 // Candidates are broadcast 32 at a time with shuffles.
-__device__ int neighbors_small_box(const Dev& d, Rep& R, int lc, int lane, int first = 0, int stride = 32) {
+__device__ int neighbors_small_box(const Dev& d, const Rep& R, int lc, int lane, int first = 0, int stride = 32) {
   const int G = R.G;
   const float h = R.h, inv_h = 1.0f / h;
   const float dL = (float)(R.L - (double)G * (double)h);
@@ -938,10 +966,11 @@ __device__ int neighbors_small_box(const Dev& d, Rep& R, int lc, int lane, int f
 
 
 constexpr int kNbrWarps = kNbrThreads / 32;
-constexpr int kNbrWin = 1024;     // staged candidates per window
+constexpr int kNbrWin = 1024;     // staged candidates per window (a multiple of 64)
 constexpr int kNbrGroup = 64;     // home atoms per pass
 
-__device__ void neighbors_cell_ballot(const Dev& d, Rep& R, int lc) {
+template <int WIN, int WARPS>
+__device__ __forceinline__ void neighbors_cell_ballot(const Dev& d, const Rep& R, int* status, int lc) {
   const int G = R.G;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (G < 3) return;  // boxes under three cells per axis: k_neighbors_small
@@ -954,15 +983,15 @@ __device__ void neighbors_cell_ballot(const Dev& d, Rep& R, int lc) {
   const float rcs = (float)(R.rc + R.skin);
   const float rcs2 = rcs * rcs;
 
-  __shared__ float4 s_c[kNbrWin];
+  __shared__ float4 s_c[WIN];
   __shared__ int s_ns[27], s_off[28], s_cnt[kNbrGroup];
   __shared__ float s_sx[27], s_sy[27], s_sz[27];
   __shared__ uint32_t s_code[27];
   constexpr int kExcl = 1 + kMaxBondsPerAtom;  // the atom itself and its bonded partners
   __shared__ float4 s_hp[kNbrGroup];            // home atoms' positions
   __shared__ int s_xk[kNbrGroup][kExcl];        // and their excluded candidates (index, or -1)
-  __shared__ uint32_t s_xm[kNbrWarps][kNbrWin / 32];  // per warp: excluded candidates of the window
-  for (int k = threadIdx.x; k < kNbrWarps * (kNbrWin / 32); k += blockDim.x) (&s_xm[0][0])[k] = 0u;
+  __shared__ uint32_t s_xm[WARPS][WIN / 32];  // per warp: excluded candidates of the window
+  for (int k = threadIdx.x; k < WARPS * (WIN / 32); k += blockDim.x) (&s_xm[0][0])[k] = 0u;
   const int hx = lc % G, hy = (lc / G) % G, hz = lc / (G * G);
   if (warp == 0) {
     // the 27 cells (one lane each) and their candidate offsets (warp scan)
@@ -1030,21 +1059,21 @@ __device__ void neighbors_cell_ballot(const Dev& d, Rep& R, int lc) {
         s_xk[a][1 + b] = k;
       }
     }
-    for (int w0 = 0; w0 < total; w0 += kNbrWin) {
-      const int wn = min(kNbrWin, total - w0);
-      if (hg == 0 || total > kNbrWin) {
+    for (int w0 = 0; w0 < total; w0 += WIN) {
+      const int wn = min(WIN, total - w0);
+      if (hg == 0 || total > WIN) {
         if (w0 > 0) __syncthreads();  // the previous window is no longer read
         // candidates of the window, each warp taking cells warp, warp + 4, ...:
         // asynchronous copies first (all in flight together), then each
         // thread adds the cell shifts to the candidates it copied
-        for (int t = warp; t < 27; t += kNbrWarps) {
+        for (int t = warp; t < 27; t += WARPS) {
           const int o0 = s_off[t], o1 = s_off[t + 1];
           const int lo = max(o0, w0), hi = min(o1, w0 + wn);
           const float4* src = d.pos + base + s_ns[t] - o0;
           for (int k = lo + lane; k < hi; k += 32) cp_async16(&s_c[k - w0], src + k);
         }
         cp_async_wait_all();
-        for (int t = warp; t < 27; t += kNbrWarps) {
+        for (int t = warp; t < 27; t += WARPS) {
           const int o0 = s_off[t], o1 = s_off[t + 1];
           const int lo = max(o0, w0), hi = min(o1, w0 + wn);
           const float sx = s_sx[t], sy = s_sy[t], sz = s_sz[t];
@@ -1060,7 +1089,7 @@ __device__ void neighbors_cell_ballot(const Dev& d, Rep& R, int lc) {
       const int wnp = (wn + 63) & ~63;
       for (int k = wn + threadIdx.x; k < wnp; k += blockDim.x) s_c[k] = make_float4(1e30f, 1e30f, 1e30f, 0.0f);
       __syncthreads();  // window (and home data) staged
-      for (int a = warp; a < gn; a += kNbrWarps) {
+      for (int a = warp; a < gn; a += WARPS) {
         const int i = hs + hg + a;
         const float4 pi = s_hp[a];
         // this atom's excluded candidates in the window, as bits
@@ -1088,7 +1117,7 @@ __device__ void neighbors_cell_ballot(const Dev& d, Rep& R, int lc) {
         __syncwarp();
         if (xk >= 0) s_xm[warp][xk >> 5] = 0u;
         __syncwarp();
-        if (w0 + kNbrWin >= total) {
+        if (w0 + WIN >= total) {
           if (count <= M) {
             const int padded = (count + kListPad - 1) & ~(kListPad - 1);
             if (lane < padded - count)
@@ -1104,7 +1133,7 @@ __device__ void neighbors_cell_ballot(const Dev& d, Rep& R, int lc) {
       }
     }
   }
-  if (overflow) atomicOr(&R.status, overflow);
+  if (overflow) atomicOr(status, overflow);
 }
 
 // Verlet list (G >= 3): one block per row of up to kNbrRow home cells along
@@ -1258,9 +1287,10 @@ __global__ void __launch_bounds__(kNbrThreads, MINB) k_neighbors(Dev d) {
   for (int item = blockIdx.x; item < total; item += gridDim.x) {
     cur.seek(item);
     __syncthreads();  // the previous item's shared staging is no longer read
-    if (V == 0)
-      neighbors_cell_ballot(d, d.reps[rb_rep(d, cur.i)], item - cur.lo);
-    else
+    if (V == 0) {
+      Rep& R = d.reps[rb_rep(d, cur.i)];
+      neighbors_cell_ballot<kNbrWin, kNbrWarps>(d, R, &R.status, item - cur.lo);
+    } else
       neighbors_row(d, d.reps[rb_rep(d, cur.i)], item - cur.lo);
   }
 }
@@ -1325,12 +1355,15 @@ __device__ __forceinline__ float3 bonded_dr(float4 pi, float4 pj, int G, float h
                      bonded_axis(w_cz(ui), w_cz(uj), pi.z, pj.z, G, h, inv_h, dL));
 }
 
+// Sums of the first BS threads' values (a block may be wider).
 template <int BS>
 __device__ __forceinline__ void block_partials(double* vals, int nv, double* out, int64_t stride) {
   __shared__ double sm[BS / 32][8];
-  for (int c = 0; c < nv; ++c) vals[c] = warp_sum(vals[c]);
-  if ((threadIdx.x & 31) == 0)
-    for (int c = 0; c < nv; ++c) sm[threadIdx.x >> 5][c] = vals[c];
+  if (threadIdx.x < BS) {
+    for (int c = 0; c < nv; ++c) vals[c] = warp_sum(vals[c]);
+    if ((threadIdx.x & 31) == 0)
+      for (int c = 0; c < nv; ++c) sm[threadIdx.x >> 5][c] = vals[c];
+  }
   __syncthreads();
   if (threadIdx.x < nv) {
     double t = 0.0;
@@ -1477,7 +1510,7 @@ __device__ __forceinline__ void lj_loop(const uint32_t* lst, int nn, const float
   uint32_t wn[B];
   if (PF) {
 #pragma unroll
-    for (int q = 0; q < B; ++q) wn[q] = nn > k0 ? __ldg(lst + (size_t)(k0 + q) * 32) : 0u;
+    for (int q = 0; q < B; ++q) wn[q] = nn > k0 ? lst[(size_t)(k0 + q) * 32] : 0u;
   }
   // plain sums over KB batches (KB * B <= 8 pairs), then one compensated add
   PairAcc g = {0, 0, 0, acc.pe, acc.v0, acc.v1, acc.v2, acc.v3, acc.v4, acc.v5};
@@ -1489,15 +1522,15 @@ __device__ __forceinline__ void lj_loop(const uint32_t* lst, int nn, const float
       for (int q = 0; q < B; ++q) w[q] = wn[q];
       if (k + STEP < nn) {
 #pragma unroll
-        for (int q = 0; q < B; ++q) wn[q] = __ldg(lst + (size_t)(k + STEP + q) * 32);
+        for (int q = 0; q < B; ++q) wn[q] = lst[(size_t)(k + STEP + q) * 32];
       }
     } else {
 #pragma unroll
-      for (int q = 0; q < B; ++q) w[q] = __ldg(lst + (size_t)(k + q) * 32);
+      for (int q = 0; q < B; ++q) w[q] = lst[(size_t)(k + q) * 32];
     }
     float4 pj[B];
 #pragma unroll
-    for (int q = 0; q < B; ++q) pj[q] = __ldg(pbase + (w[q] & kIdxMask));
+    for (int q = 0; q < B; ++q) pj[q] = pbase[w[q] & kIdxMask];
     if (P2 && ONE && !EV) {
 #pragma unroll
       for (int q = 0; q < B; q += 2)
@@ -1580,7 +1613,7 @@ __device__ __forceinline__ void lj_loop_ring(const uint32_t* tile_rows, uint32_t
     for (int q = 0; q < B; ++q) w[q] = k + q < nn ? slot[q * 32 + lane] : pad;
     float4 pj[B];
 #pragma unroll
-    for (int q = 0; q < B; ++q) pj[q] = __ldg(pbase + (w[q] & kIdxMask));
+    for (int q = 0; q < B; ++q) pj[q] = pbase[w[q] & kIdxMask];
     if (P2 && ONE && !EV) {
 #pragma unroll
       for (int q = 0; q < B; q += 2)
@@ -1635,7 +1668,7 @@ __device__ __forceinline__ int lj_loop_filter(const uint32_t* lst, int nn, uint3
   uint32_t wn[B];
   if (PF) {
 #pragma unroll
-    for (int q = 0; q < B; ++q) wn[q] = nn > 0 ? __ldg(lst + (size_t)q * 32) : 0u;
+    for (int q = 0; q < B; ++q) wn[q] = nn > 0 ? lst[(size_t)q * 32] : 0u;
   }
   PairAcc g = {0, 0, 0, acc.pe, acc.v0, acc.v1, acc.v2, acc.v3, acc.v4, acc.v5};
   int pc = 0;
@@ -1646,15 +1679,15 @@ __device__ __forceinline__ int lj_loop_filter(const uint32_t* lst, int nn, uint3
       for (int q = 0; q < B; ++q) w[q] = wn[q];
       if (k + B < nn) {
 #pragma unroll
-        for (int q = 0; q < B; ++q) wn[q] = __ldg(lst + (size_t)(k + B + q) * 32);
+        for (int q = 0; q < B; ++q) wn[q] = lst[(size_t)(k + B + q) * 32];
       }
     } else {
 #pragma unroll
-      for (int q = 0; q < B; ++q) w[q] = __ldg(lst + (size_t)(k + q) * 32);
+      for (int q = 0; q < B; ++q) w[q] = lst[(size_t)(k + q) * 32];
     }
     float4 pj[B];
 #pragma unroll
-    for (int q = 0; q < B; ++q) pj[q] = __ldg(pbase + (w[q] & kIdxMask));
+    for (int q = 0; q < B; ++q) pj[q] = pbase[w[q] & kIdxMask];
 #pragma unroll
     for (int q = 0; q < B; ++q) {
       const float3 sh = entry_shift<SH>(w[q], s_shift, s_axis);
@@ -1702,9 +1735,8 @@ __device__ __forceinline__ int lj_loop_filter(const uint32_t* lst, int nn, uint3
 // in different roles follow one path.  EV: a third of the energy per member,
 // the angle's virial carried by the vertex.
 template <bool EV>
-__device__ __forceinline__ void angle_term(float4 ri, float4 rj, float4 rk, int role, float kt, float th0, int G,
-                                           float h, float inv_h, float dL, KahanF& fx, KahanF& fy, KahanF& fz,
-                                           float& pe, float* bv) {
+__device__ __forceinline__ float3 angle_term(float4 ri, float4 rj, float4 rk, int role, float kt, float th0, int G,
+                                             float h, float inv_h, float dL, float& pe, float* bv) {
   const float3 dij = bonded_dr(ri, rj, G, h, inv_h, dL);
   const float3 dkj = bonded_dr(rk, rj, G, h, inv_h, dL);
   const float rij2 = dij.x * dij.x + dij.y * dij.y + dij.z * dij.z;
@@ -1724,9 +1756,6 @@ __device__ __forceinline__ void angle_term(float4 ri, float4 rj, float4 rk, int 
   const float fkx = __fmul_rn(pref, fmaf(dij.x, rr, -__fmul_rn(ck2, dkj.x)));
   const float fky = __fmul_rn(pref, fmaf(dij.y, rr, -__fmul_rn(ck2, dkj.y)));
   const float fkz = __fmul_rn(pref, fmaf(dij.z, rr, -__fmul_rn(ck2, dkj.z)));
-  fx.add(role == 0 ? fix : (role == 2 ? fkx : -(fix + fkx)));
-  fy.add(role == 0 ? fiy : (role == 2 ? fky : -(fiy + fky)));
-  fz.add(role == 0 ? fiz : (role == 2 ? fkz : -(fiz + fkz)));
   if (EV) {
     if (role == 1) {
       bv[0] += fix * dij.x + fkx * dkj.x;
@@ -1737,6 +1766,97 @@ __device__ __forceinline__ void angle_term(float4 ri, float4 rj, float4 rk, int 
       bv[5] += fiz * dij.z + fkz * dkj.z;
     }
     pe += kt * dth * dth * (1.0f / 3.0f);
+  }
+  return make_float3(role == 0 ? fix : (role == 2 ? fkx : -(fix + fkx)),
+                     role == 0 ? fiy : (role == 2 ? fky : -(fiy + fky)),
+                     role == 0 ? fiz : (role == 2 ? fkz : -(fiz + fkz)));
+}
+
+// The push-off's cap on a non-bonded force.  Explicit roundings: the capped
+// values enter the force sums of every kernel that evaluates them.
+__device__ __forceinline__ void cap_force(float cap, float& lx, float& ly, float& lz) {
+  const float m2 = __fmaf_rn(lz, lz, __fmaf_rn(lx, lx, __fmul_rn(ly, ly)));
+  if (m2 > cap * cap) {
+    const float sc = __fmul_rn(cap, rsqrtf(m2));
+    lx = __fmul_rn(lx, sc);
+    ly = __fmul_rn(ly, sc);
+    lz = __fmul_rn(lz, sc);
+  }
+}
+
+template <bool EV>
+__device__ __forceinline__ float3 fene_term(const Rep& R, uint32_t bw, float4 pi, float4 pj, int G, float h,
+                                            float inv_h, float dL, float& pe, float* bv, int& status) {
+  // FENE + WCA (fene.cu:18-73): this atom's force; the bond's energy is split
+  // half per atom and its virial carried by the first atom.
+  const int bt = (bw >> 26) & 0xF;
+  const float3 dr = bonded_dr(pi, pj, G, h, inv_h, dL);
+  const float r2 = dr.x * dr.x + dr.y * dr.y + dr.z * dr.z;
+  const float kf = R.fene[4 * bt], R02 = R.fene[4 * bt + 1], eps = R.fene[4 * bt + 2], sig2 = R.fene[4 * bt + 3];
+  if (r2 >= R02 * 0.9999f) status |= kStatusFeneStretch;
+  const float r2s = fminf(fmaxf(r2, 1e-6f), R02 * 0.9999f);
+  float ff = -kf * R02 * __fdividef(1.0f, R02 - r2s);
+  float wpe = 0.0f;
+  if (r2s < sig2 * 1.2599210498948732f) {
+    const float r2inv = __fdividef(1.0f, r2s);
+    const float sr2 = sig2 * r2inv;
+    const float sr6 = sr2 * sr2 * sr2;
+    ff = fmaf(24.0f * eps * r2inv * sr6, 2.0f * sr6 - 1.0f, ff);
+    if (EV) wpe = 4.0f * eps * sr6 * (sr6 - 1.0f) + eps;
+  }
+  if (EV) {
+    pe += 0.5f * (-0.5f * kf * R02 * log1pf(-r2s / R02) + wpe);
+    if ((bw >> 30) & 1) {
+      bv[0] = fmaf(ff * dr.x, dr.x, bv[0]);
+      bv[1] = fmaf(ff * dr.x, dr.y, bv[1]);
+      bv[2] = fmaf(ff * dr.x, dr.z, bv[2]);
+      bv[3] = fmaf(ff * dr.y, dr.y, bv[3]);
+      bv[4] = fmaf(ff * dr.y, dr.z, bv[4]);
+      bv[5] = fmaf(ff * dr.z, dr.z, bv[5]);
+    }
+  }
+  return make_float3(__fmul_rn(ff, dr.x), __fmul_rn(ff, dr.y), __fmul_rn(ff, dr.z));
+}
+
+// The angle entry aw of the atom at pi: its force on that atom.
+template <bool EV>
+__device__ __forceinline__ float3 angle_of(const Rep& R, uint2 aw, float4 pi, const float4* pbase, int G, float h,
+                                           float inv_h, float dL, float& pe, float* bv) {
+  const int role = (aw.x >> 26) & 3, at = (aw.y >> 26) & 0xF;
+  const float4 p1 = pbase[aw.x & kSlotMask26];
+  const float4 p2 = pbase[aw.y & kSlotMask26];
+  const float kt = R.angp[2 * at], th0 = R.angp[2 * at + 1];
+  // members in angle order (i, j = vertex, k); the table holds the other two
+  const float4 ri = role == 0 ? pi : p1;
+  const float4 rj = role == 1 ? pi : (role == 0 ? p1 : p2);
+  const float4 rk = role == 2 ? pi : p2;
+  return angle_term<EV>(ri, rj, rk, role, kt, th0, G, h, inv_h, dL, pe, bv);
+}
+
+// Bonded terms of the atom in slot s, gathered: its bonds and angles
+// first, first + stride, ... (lanes that share an atom split them; one lane
+// per atom takes all with first = 0, stride = 1).
+template <bool EV>
+__device__ __forceinline__ void bonded_terms(const Dev& d, const Rep& R, int s, const float4* pbase, float4 pi, int G,
+                                             float h, float inv_h, float dL, int first, int stride, KahanF& fx,
+                                             KahanF& fy, KahanF& fz, float& pe, float* bv, int& status) {
+  const int tc = d.tcnt[s];
+  const int nbd = tc & 0xFF, nang = tc >> 8;
+  const uint32_t* bl = d.bnd + (size_t)s * kMaxBondsPerAtom;
+  for (int b = first; b < nbd; b += stride) {
+    const uint32_t bw = bl[b];
+    const float3 f = fene_term<EV>(R, bw, pi, pbase[bw & kSlotMask26], G, h, inv_h, dL, pe, bv, status);
+    fx.add(f.x);
+    fy.add(f.y);
+    fz.add(f.z);
+  }
+  // Harmonic angles this atom belongs to, by role.
+  const uint2* al = d.ang + (size_t)s * kMaxAnglesPerAtom;
+  for (int a = first; a < nang; a += stride) {
+    const float3 f = angle_of<EV>(R, al[a], pi, pbase, G, h, inv_h, dL, pe, bv);
+    fx.add(f.x);
+    fy.add(f.y);
+    fz.add(f.z);
   }
 }
 
@@ -1749,83 +1869,17 @@ __device__ __forceinline__ void angle_term(float4 ri, float4 rj, float4 rk, int 
 // LISTED: the work-list launch itself (replicas rebuilt or re-filtered this
 // step), which walks the rc + skin list and, where the replica keeps a
 // pruned list, writes it (the filter) and its displacement reference.
-// Bonded terms of the atom in slot s, gathered: its bonds and angles
-// first, first + stride, ... (lanes that share an atom split them; one lane
-// per atom takes all with first = 0, stride = 1).
-template <bool EV>
-__device__ __forceinline__ void bonded_terms(const Dev& d, const Rep& R, int s, const float4* pbase, float4 pi, int G,
-                                             float h, float inv_h, float dL, int first, int stride, KahanF& fx,
-                                             KahanF& fy, KahanF& fz, float& pe, float* bv, int& status) {
-  const int tc = d.tcnt[s];
-  const int nbd = tc & 0xFF, nang = tc >> 8;
-  // FENE + WCA (fene.cu:18-73), gathered: this atom's force; the bond's
-  // energy is split half per atom and its virial carried by the first atom.
-  const uint32_t* bl = d.bnd + (size_t)s * kMaxBondsPerAtom;
-  for (int b = first; b < nbd; b += stride) {
-    const uint32_t bw = bl[b];
-    const int bt = (bw >> 26) & 0xF;
-    const float4 pj = pbase[bw & kSlotMask26];
-    const float3 dr = bonded_dr(pi, pj, G, h, inv_h, dL);
-    const float r2 = dr.x * dr.x + dr.y * dr.y + dr.z * dr.z;
-    const float kf = R.fene[4 * bt], R02 = R.fene[4 * bt + 1], eps = R.fene[4 * bt + 2], sig2 = R.fene[4 * bt + 3];
-    if (r2 >= R02 * 0.9999f) status |= kStatusFeneStretch;
-    const float r2s = fminf(fmaxf(r2, 1e-6f), R02 * 0.9999f);
-    float ff = -kf * R02 * __fdividef(1.0f, R02 - r2s);
-    float wpe = 0.0f;
-    if (r2s < sig2 * 1.2599210498948732f) {
-      const float r2inv = __fdividef(1.0f, r2s);
-      const float sr2 = sig2 * r2inv;
-      const float sr6 = sr2 * sr2 * sr2;
-      ff = fmaf(24.0f * eps * r2inv * sr6, 2.0f * sr6 - 1.0f, ff);
-      if (EV) wpe = 4.0f * eps * sr6 * (sr6 - 1.0f) + eps;
-    }
-    fx.add(__fmul_rn(ff, dr.x));
-    fy.add(__fmul_rn(ff, dr.y));
-    fz.add(__fmul_rn(ff, dr.z));
-    if (EV) {
-      pe += 0.5f * (-0.5f * kf * R02 * log1pf(-r2s / R02) + wpe);
-      if ((bw >> 30) & 1) {
-        bv[0] = fmaf(ff * dr.x, dr.x, bv[0]);
-        bv[1] = fmaf(ff * dr.x, dr.y, bv[1]);
-        bv[2] = fmaf(ff * dr.x, dr.z, bv[2]);
-        bv[3] = fmaf(ff * dr.y, dr.y, bv[3]);
-        bv[4] = fmaf(ff * dr.y, dr.z, bv[4]);
-        bv[5] = fmaf(ff * dr.z, dr.z, bv[5]);
-      }
-    }
-  }
-  // Harmonic angles this atom belongs to, by role.
-  const uint2* al = d.ang + (size_t)s * kMaxAnglesPerAtom;
-  for (int a = first; a < nang; a += stride) {
-    const uint2 aw = al[a];
-    const int role = (aw.x >> 26) & 3, at = (aw.y >> 26) & 0xF;
-    const float4 p1 = pbase[aw.x & kSlotMask26];
-    const float4 p2 = pbase[aw.y & kSlotMask26];
-    const float kt = R.angp[2 * at], th0 = R.angp[2 * at + 1];
-    // members in angle order (i, j = vertex, k); the table holds the other two
-    const float4 ri = role == 0 ? pi : p1;
-    const float4 rj = role == 1 ? pi : (role == 0 ? p1 : p2);
-    const float4 rk = role == 2 ? pi : p2;
-    angle_term<EV>(ri, rj, rk, role, kt, th0, G, h, inv_h, dL, fx, fy, fz, pe, bv);
-  }
-}
-
 // PF: 0 = list words loaded with the batch, 1 = the next batch's words
 // loaded ahead into registers, D >= 2 = the ring of D batches (per-chunk
 // kernel; the work-list kernel then loads ahead into registers).
+// R: the replica's record, or a block's copy of it; ci the chunk's entry.
 template <bool EV, int B, int PF, int KB, bool LISTED, int SH, bool P2>
-__device__ __forceinline__ void force_chunk(const Dev& d, int chunk, bool skip_rebuilt) {
+__device__ __forceinline__ void force_chunk_of(const Dev& d, const Rep& R, const int4 ci, int chunk) {
   constexpr bool RING = PF >= 2 && !LISTED;
   constexpr bool PFR = PF != 0;  // register look-ahead in the loops below
   static_assert(!RING || B == 4, "the ring stages batches of 4 rows");
-  const int4 ci = d.chunk_rep[chunk];
-  const int r = ci.x;
-  if (r < 0) return;
-  const Rep& R = d.reps[r];
-  if (!R.adv) return;
-  if (need_ev(R) != EV) return;
-  if (skip_rebuilt && R.rebuild_now) return;
   constexpr bool ev = EV;
+  const int r = ci.x;
   __shared__ float4 s_shift[SH == 0 ? kShiftCodes : 1];
   __shared__ float s_axis[5];
   __shared__ float s_eps24[kMaxTypes * kMaxTypes], s_sig2[kMaxTypes * kMaxTypes];
@@ -1878,7 +1932,7 @@ __device__ __forceinline__ void force_chunk(const Dev& d, int chunk, bool skip_r
                                                            d.pos + base, pi, s_shift, s_axis, ti, nt, s_eps24,
                                                            s_sig2, rc2, fx, fy, fz, acc);
   }
-  if (local < R.natoms) {
+  if (threadIdx.x < kChunk && local < R.natoms) {
     const float4 pi = d.pos[s];
     const uint32_t ui = w_bits(pi.w);
     const int ti = w_type(ui);
@@ -1917,14 +1971,7 @@ __device__ __forceinline__ void force_chunk(const Dev& d, int chunk, bool skip_r
     float bv[6] = {0.5f * acc.v0, 0.5f * acc.v1, 0.5f * acc.v2, 0.5f * acc.v3, 0.5f * acc.v4, 0.5f * acc.v5};
     if (R.fcap > 0.0) {  // push-off caps the non-bonded force only
       float lx = fx.s - fx.c, ly = fy.s - fy.c, lz = fz.s - fz.c;
-      const float m2 = lx * lx + ly * ly + lz * lz;
-      const float cap = (float)R.fcap;
-      if (m2 > cap * cap) {
-        const float sc = cap * rsqrtf(m2);
-        lx *= sc;
-        ly *= sc;
-        lz *= sc;
-      }
+      cap_force((float)R.fcap, lx, ly, lz);
       fx = {lx, 0.0f};
       fy = {ly, 0.0f};
       fz = {lz, 0.0f};
@@ -1939,8 +1986,19 @@ __device__ __forceinline__ void force_chunk(const Dev& d, int chunk, bool skip_r
     }
   }
   status = __syncthreads_or(status);
-  if (threadIdx.x == 0 && status) atomicOr((int*)&d.reps[r].status, status);
+  if (threadIdx.x == 0 && status) atomicOr(&d.reps[r].status, status);
   if (EV) block_partials<kChunk>(vals, 7, d.part + chunk, d.part_stride);
+}
+
+template <bool EV, int B, int PF, int KB, bool LISTED, int SH, bool P2>
+__device__ __forceinline__ void force_chunk(const Dev& d, int chunk, bool skip_rebuilt) {
+  const int4 ci = d.chunk_rep[chunk];
+  if (ci.x < 0) return;
+  const Rep& R = d.reps[ci.x];
+  if (!R.adv) return;
+  if (need_ev(R) != EV) return;
+  if (skip_rebuilt && R.rebuild_now) return;
+  force_chunk_of<EV, B, PF, KB, LISTED, SH, P2>(d, R, ci, chunk);
 }
 
 // The list filter alone: the entries of the atom's rc + skin list (nn
@@ -1955,9 +2013,9 @@ __device__ __forceinline__ int filter_list(const uint32_t* lst, int nn, uint32_t
     uint32_t w[kListPad];
     float4 pj[kListPad];
 #pragma unroll
-    for (int q = 0; q < kListPad; ++q) w[q] = __ldg(lst + (size_t)(k + q) * 32);
+    for (int q = 0; q < kListPad; ++q) w[q] = lst[(size_t)(k + q) * 32];
 #pragma unroll
-    for (int q = 0; q < kListPad; ++q) pj[q] = __ldg(pbase + (w[q] & kIdxMask));
+    for (int q = 0; q < kListPad; ++q) pj[q] = pbase[w[q] & kIdxMask];
 #pragma unroll
     for (int q = 0; q < kListPad; ++q) {
       float dx, dy, dz;
@@ -2083,14 +2141,7 @@ __device__ __forceinline__ void force_chunk_lanes(const Dev& d, int chunk, bool 
       lanes_combine<LPA>(fy);
       lanes_combine<LPA>(fz);
       float lx = fx.s - fx.c, ly = fy.s - fy.c, lz = fz.s - fz.c;
-      const float m2 = lx * lx + ly * ly + lz * lz;
-      const float cap = (float)R.fcap;
-      if (m2 > cap * cap) {
-        const float sc = cap * rsqrtf(m2);
-        lx *= sc;
-        ly *= sc;
-        lz *= sc;
-      }
+      cap_force((float)R.fcap, lx, ly, lz);
       const bool own = g == 0;
       fx = {own ? lx : 0.0f, 0.0f};
       fy = {own ? ly : 0.0f, 0.0f};
@@ -2153,6 +2204,212 @@ __global__ void __launch_bounds__(kChunk, MINB) k_force_rb(Dev d) {
   }
 }
 
+// ---- four lanes per atom (resident steps of small batches).  Lane group
+// q = lane / 8 of a warp shares the warp's eight atoms (src = lane % 8; a
+// batch row read by one group is one whole sector): it evaluates the atom's
+// compensated-add units q, q + 4, ..., and every lane then adds all four
+// lanes' unit sums in list order, so the sums are bit for bit those of the
+// one-lane walk while a list's dependent chain (word -> position -> pair) is
+// a quarter as long.  The bonded terms are split and added the same way.
+__device__ __forceinline__ float quad_get(float v, int src, int j) {
+  return __shfl_sync(0xFFFFFFFFu, v, src + 8 * j);
+}
+
+template <int KB, bool ONE>
+__device__ __forceinline__ void lj_quads(const uint32_t* lst, int nn, const float4* pbase, float4 pi,
+                                         const float* s_axis, int ti, int nt, const float* s_eps24,
+                                         const float* s_sig2, float rc2, uint32_t pad, int q, int src, KahanF& fx,
+                                         KahanF& fy, KahanF& fz) {
+  constexpr int U = 4 * KB;  // entries per compensated add
+  const float e24_0 = s_eps24[0], sig2_0 = s_sig2[0];
+  const int nu = (nn + U - 1) / U;
+  const int rounds = __reduce_max_sync(0xFFFFFFFFu, (nu + 3) / 4);
+  uint32_t wn[U];
+#pragma unroll
+  for (int i = 0; i < U; ++i) wn[i] = q * U + i < nn ? lst[(size_t)(q * U + i) * 32] : pad;
+  for (int t = 0; t < rounds; ++t) {
+    uint32_t w[U];
+    const int k = (4 * (t + 1) + q) * U;
+#pragma unroll
+    for (int i = 0; i < U; ++i) {
+      w[i] = wn[i];
+      wn[i] = k + i < nn ? lst[(size_t)(k + i) * 32] : pad;
+    }
+    PairAcc g = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int b = 0; b < U; b += 4) {
+      float4 pj[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) pj[i] = pbase[w[b + i] & kIdxMask];
+      if (ONE) {
+#pragma unroll
+        for (int i = 0; i < 4; i += 2)
+          lj_pair2(g, pi, entry_shift<1>(w[b + i], nullptr, s_axis), pj[i],
+                   entry_shift<1>(w[b + i + 1], nullptr, s_axis), pj[i + 1], rc2, e24_0, sig2_0);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int pidx = ti * nt + w_type(w_bits(pj[i].w));
+          lj_pair<false>(g, pi, entry_shift<1>(w[b + i], nullptr, s_axis), pj[i], rc2, s_eps24[pidx], s_sig2[pidx]);
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float x = quad_get(g.fx, src, j), y = quad_get(g.fy, src, j), z = quad_get(g.fz, src, j);
+      if (4 * t + j < nu) {
+        fx.add(x);
+        fy.add(y);
+        fz.add(z);
+      }
+    }
+  }
+}
+
+// The list filter by four lanes per atom: the entries within rc +
+// prune_delta in list order, padded; returns their count in every lane.
+__device__ __forceinline__ int filter_quads(const uint32_t* lst, int nn, uint32_t* pout, float rcd2,
+                                            const float4* pbase, float4 pi, const float* s_axis, uint32_t pad, int q,
+                                            int src) {
+  const int rounds = __reduce_max_sync(0xFFFFFFFFu, (nn + 15) / 16);
+  uint32_t wn[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) wn[i] = 4 * q < nn ? lst[(size_t)(4 * q + i) * 32] : pad;
+  int pc = 0;
+  for (int t = 0; t < rounds; ++t) {
+    uint32_t w[4];
+    const int k = 16 * (t + 1) + 4 * q;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      w[i] = wn[i];
+      wn[i] = k < nn ? lst[(size_t)(k + i) * 32] : pad;
+    }
+    float4 pj[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) pj[i] = pbase[w[i] & kIdxMask];
+    bool keep[4];
+    int n = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float dx, dy, dz;
+      keep[i] = pair_r2(pi, entry_shift<1>(w[i], nullptr, s_axis), pj[i], dx, dy, dz) < rcd2;
+      n += keep[i] ? 1 : 0;
+    }
+    int at = pc;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int m = __shfl_sync(0xFFFFFFFFu, n, src + 8 * j);
+      at += j < q ? m : 0;
+      pc += m;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (keep[i]) pout[(size_t)(at++) * 32] = w[i];
+  }
+  const int padded = (pc + kPrunePad - 1) & ~(kPrunePad - 1);
+  if (pc + q < padded) pout[(size_t)(pc + q) * 32] = pad;
+  return pc;
+}
+
+// Forces without energies of one chunk by a block of 4 kChunk threads, four
+// lanes per atom; LISTED: the replica's pruned list is due (or it keeps none).
+template <int KB, bool LISTED>
+__device__ __forceinline__ void force_chunk_quads(const Dev& d, const Rep& R, int r, int c) {
+  __shared__ float s_axis[5];
+  __shared__ float s_eps24[kMaxTypes * kMaxTypes], s_sig2[kMaxTypes * kMaxTypes];
+  const int lane = threadIdx.x & 31, q = lane >> 3, src = lane & 7;
+  const int nt = R.ntypes;
+  const int G = R.G;
+  const float h = R.h, inv_h = 1.0f / h;
+  const float dL = (float)(R.L - (double)G * (double)h);
+  const int local = c * kChunk + (threadIdx.x >> 5) * 8 + src;
+  const int base = R.slot_base, s = base + local;
+  const bool valid = local < R.natoms;
+  const bool keeps = R.prune_delta > 0.f, pruned = keeps && !LISTED;
+  // the atom's own words, all in flight before the tables' barrier
+  const float4 pi = valid ? d.pos[s] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const int tc = valid ? d.tcnt[s] : 0;
+  int nn = valid ? (pruned ? d.pcnt[s] : d.ncnt[s]) : 0;
+  const uint32_t bw = valid ? d.bnd[(size_t)s * kMaxBondsPerAtom + q] : 0u;
+  const uint2 aw = valid ? d.ang[(size_t)s * kMaxAnglesPerAtom + q] : make_uint2(0u, 0u);
+  for (int k = threadIdx.x; k < nt * nt; k += blockDim.x) {
+    s_eps24[k] = R.lj_eps24[k];
+    s_sig2[k] = R.lj_sig2[k];
+  }
+  if (threadIdx.x < 5)
+    s_axis[threadIdx.x] = shift_term(axis_code_e(threadIdx.x), axis_code_k(threadIdx.x), h, dL);
+  __syncthreads();
+  const int padding = pruned ? kPrunePad : kListPad;
+  nn = (nn + padding - 1) & ~(padding - 1);
+  const float rc2 = (float)(R.rc * R.rc);
+  const uint32_t pad = (uint32_t)(valid ? local : 0) | kPadBits;
+  const size_t row = (size_t)R.nbr_base + ((size_t)(local >> 5) * R.M) * 32 + (local & 31);
+  const uint32_t* lst = (pruned ? d.pnbr : d.nbr) + row;
+  const float4* pbase = d.pos + base;
+  const int ti = w_type(w_bits(pi.w));
+  if (LISTED && keeps) {  // replica-uniform
+    const float rcd = (float)(R.rc + (double)R.prune_delta);
+    const int pc = filter_quads(lst, nn, d.pnbr + row, rcd * rcd, pbase, pi, s_axis, pad, q, src);
+    if (valid && q == 0) {
+      d.pcnt[s] = pc;
+      const float4 ref = d.ref[s];
+      d.ref[s] = make_float4(pi.x, pi.y, pi.z, ref.w);
+    }
+    __syncwarp();  // the other lanes' entries of the new list
+    nn = (pc + kPrunePad - 1) & ~(kPrunePad - 1);
+    lst = d.pnbr + row;
+  }
+  KahanF fx = {0, 0}, fy = {0, 0}, fz = {0, 0};
+  if (nt == 1)
+    lj_quads<KB, true>(lst, nn, pbase, pi, s_axis, ti, nt, s_eps24, s_sig2, rc2, pad, q, src, fx, fy, fz);
+  else
+    lj_quads<KB, false>(lst, nn, pbase, pi, s_axis, ti, nt, s_eps24, s_sig2, rc2, pad, q, src, fx, fy, fz);
+  if (R.fcap > 0.0) {  // push-off caps the non-bonded force only
+    float lx = fx.s - fx.c, ly = fy.s - fy.c, lz = fz.s - fz.c;
+    cap_force((float)R.fcap, lx, ly, lz);
+    fx = {lx, 0.0f};
+    fy = {ly, 0.0f};
+    fz = {lz, 0.0f};
+  }
+  int status = 0;
+  const int nbd = tc & 0xFF, nang = tc >> 8;
+  float pe = 0.f, bv[6];
+  float3 f = make_float3(0.f, 0.f, 0.f);
+  static_assert(kMaxBondsPerAtom <= 4, "one bond per lane");
+  if (q < nbd) f = fene_term<false>(R, bw, pi, pbase[bw & kSlotMask26], G, h, inv_h, dL, pe, bv, status);
+  const int most_b = __reduce_max_sync(0xFFFFFFFFu, nbd);
+  for (int j = 0; j < most_b; ++j) {
+    const float x = quad_get(f.x, src, j), y = quad_get(f.y, src, j), z = quad_get(f.z, src, j);
+    if (j < nbd) {
+      fx.add(x);
+      fy.add(y);
+      fz.add(z);
+    }
+  }
+  const int most_a = __reduce_max_sync(0xFFFFFFFFu, nang);
+  for (int a0 = 0; a0 < most_a; a0 += 4) {
+    f = make_float3(0.f, 0.f, 0.f);
+    if (a0 + q < nang)
+      f = angle_of<false>(R, a0 == 0 ? aw : d.ang[(size_t)s * kMaxAnglesPerAtom + a0 + q], pi, pbase, G, h, inv_h, dL,
+                          pe, bv);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float x = quad_get(f.x, src, j), y = quad_get(f.y, src, j), z = quad_get(f.z, src, j);
+      if (a0 + j < nang) {
+        fx.add(x);
+        fy.add(y);
+        fz.add(z);
+      }
+    }
+  }
+  if (valid && q == 0) {
+    const float ox = fx.s - fx.c, oy = fy.s - fy.c, oz = fz.s - fz.c;
+    if (!isfinite(ox + oy + oz)) status |= kStatusNonFinite;
+    d.force[s] = make_float4(ox, oy, oz, 0.0f);
+  }
+  if (status) atomicOr(&d.reps[r].status, status);
+}
+
 // ---------------------------------------------------------------- pruned list
 // Filter of the listed replicas' lists (after a rebuild, or when the
 // displacement since the last filter reached prune_delta / 2): the entries
@@ -2203,7 +2460,7 @@ __global__ void __launch_bounds__(kChunk) k_prune(Dev d) {
 #pragma unroll
       for (int q = 0; q < kListPad; ++q) w[q] = __ldg(in + (size_t)(k + q) * 32);
 #pragma unroll
-      for (int q = 0; q < kListPad; ++q) pj[q] = __ldg(pbase + (w[q] & kIdxMask));
+      for (int q = 0; q < kListPad; ++q) pj[q] = pbase[w[q] & kIdxMask];
 #pragma unroll
       for (int q = 0; q < kListPad; ++q) {
         const float3 sh = entry_shift<0>(w[q], s_shift, nullptr);
@@ -2231,15 +2488,7 @@ void launch_prune(const Dev& d, cudaStream_t st);
 // kernel for replicas with tables only; explicit roundings keep the energy
 // flavour's forces identical to the plain one's.
 template <bool EV>
-__global__ void __launch_bounds__(kChunk) k_table(Dev d, int sel) {
-  count_launch(d, kKTable);
-  const int chunk = blockIdx.x;
-  const int4 ci = d.chunk_rep[chunk];
-  const int r = ci.x;
-  if (r < 0) return;
-  const Rep& R = d.reps[r];
-  if (!R.adv || R.ntables == 0 || need_ev(R) != EV) return;
-  if ((sel == 1 && R.rebuild_now) || (sel == 2 && !R.rebuild_now)) return;
+__device__ __forceinline__ void table_chunk(const Dev& d, const Rep& R, const int4 ci, int chunk) {
   __shared__ float4 s_shift[kShiftCodes];
   const int G = R.G;
   const float h = R.h;
@@ -2257,7 +2506,7 @@ __global__ void __launch_bounds__(kChunk) k_table(Dev d, int sel) {
   const float rc2 = (float)(R.rc * R.rc);
   const int nt = R.ntypes;
   double vals[7] = {0, 0, 0, 0, 0, 0, 0};
-  if (local < R.natoms) {
+  if (threadIdx.x < kChunk && local < R.natoms) {
     const float4 pi = d.pos[s];
     const int ti = w_type(w_bits(pi.w));
     // the pruned list when the replica keeps one (same layout and bases)
@@ -2352,6 +2601,17 @@ __global__ void __launch_bounds__(kChunk) k_table(Dev d, int sel) {
   }
 }
 
+template <bool EV>
+__global__ void __launch_bounds__(kChunk) k_table(Dev d, int sel) {
+  count_launch(d, kKTable);
+  const int4 ci = d.chunk_rep[blockIdx.x];
+  if (ci.x < 0) return;
+  const Rep& R = d.reps[ci.x];
+  if (!R.adv || R.ntables == 0 || need_ev(R) != EV) return;
+  if ((sel == 1 && R.rebuild_now) || (sel == 2 && !R.rebuild_now)) return;
+  table_chunk<EV>(d, R, ci, blockIdx.x);
+}
+
 void launch_table(const Dev& d, int nchunks, bool ev, int sel, cudaStream_t st) {
   if (ev)
     k_table<true><<<nchunks, kChunk, 0, st>>>(d, sel);
@@ -2360,20 +2620,10 @@ void launch_table(const Dev& d, int nchunks, bool ev, int sel, cudaStream_t st) 
 }
 
 // ---------------------------------------------------------------- post-force
-__global__ void __launch_bounds__(kChunk, 7) k_post(Dev d, int kick) {
-  count_launch(d, kKPost);
-  const int chunk = blockIdx.x;
-  const int4 ci = d.chunk_rep[chunk];
-  if (ci.x < 0) return;
-  const int s = ci.y + threadIdx.x;
-  const bool have = (int)threadIdx.x < ci.z;
-  float4 v = make_float4(0, 0, 0, 1), f = make_float4(0, 0, 0, 0);
-  if (have) {
-    v = d.vel[s];
-    f = d.force[s];
-  }
-  Rep& R = d.reps[ci.x];
-  if (!R.adv || (kick == 1 && R.defer)) return;
+// The final half kick (kick == 1) and the KE-tensor partials of one chunk,
+// on its loaded velocity and force.
+__device__ __forceinline__ void post_chunk(const Dev& d, const Rep& R, int chunk, int s, bool have, float4 v,
+                                           const float4 f, int kick) {
   double vals[7] = {0, 0, 0, 0, 0, 0, 0};
   if (have) {
     if (kick == 1) {
@@ -2394,6 +2644,23 @@ __global__ void __launch_bounds__(kChunk, 7) k_post(Dev d, int kick) {
     vals[5] = m * vz * vz;
   }
   block_partials<kChunk>(vals, 6, d.part + 7 * d.part_stride + chunk, d.part_stride);
+}
+
+__global__ void __launch_bounds__(kChunk, 7) k_post(Dev d, int kick) {
+  count_launch(d, kKPost);
+  const int chunk = blockIdx.x;
+  const int4 ci = d.chunk_rep[chunk];
+  if (ci.x < 0) return;
+  const int s = ci.y + threadIdx.x;
+  const bool have = (int)threadIdx.x < ci.z;
+  float4 v = make_float4(0, 0, 0, 1), f = make_float4(0, 0, 0, 0);
+  if (have) {
+    v = d.vel[s];
+    f = d.force[s];
+  }
+  const Rep& R = d.reps[ci.x];
+  if (!R.adv || (kick == 1 && R.defer)) return;
+  post_chunk(d, R, chunk, s, have, v, f, kick);
 }
 
 // One pressure-tensor sample into a replica's multiple-tau correlator, by
@@ -2444,6 +2711,68 @@ __device__ void acf_push(double* st, const double* sample_in) {
   }
 }
 
+// One warp: a stress step's sample, the pressure tensor of the thermo row
+// (KE tensor with the pending thermostat scale, and the virial, in the
+// current box).
+__device__ __forceinline__ void acf_sample(const Dev& d, const Rep& R, int r) {
+  const double s2 = __dmul_rn(R.pending_scale, R.pending_scale);
+  const double V = __dmul_rn(__dmul_rn(R.L, R.L), R.L);
+  double smp[kAcfComps];
+  for (int c = 0; c < kAcfComps; ++c) smp[c] = __dadd_rn(__dmul_rn(R.ke[c], s2), R.vir[c]) / V;
+  acf_push(d.acf + (size_t)r * kAcfWords, smp);
+}
+
+// The post-force commit on a replica's record R (one thread): energies,
+// virial and KE of the step from the replica's reduced partials acc, the
+// post-force chain or barostat, and the scalars of the next pre-force.
+__device__ __forceinline__ void post_commit_state(Rep& R, const double* acc, int kick) {
+  if (need_ev(R)) {
+    R.pe = acc[0];
+    for (int q = 0; q < 6; ++q) R.vir[q] = acc[1 + q];
+  }
+  for (int q = 0; q < 6; ++q) R.ke[q] = acc[7 + q];
+  const double ke_raw = acc[7] + acc[10] + acc[12];
+  const double dt = (R.mode == kModePushoff) ? R.push_dt : R.dt;
+  const int ens = (R.mode == kModePushoff) ? FMD_LANGEVIN : R.ensemble;
+  if (need_ev(R)) R.ev_step = R.step;
+  R.force_ev = 0;
+  // the chain / barostat state is updated in a local copy and stored
+  // once: in place, its arrays' stores would order every later read of
+  // the record behind them
+  NHScalars nh = R.nh;
+  if (kick == 2) {
+    // re-evaluation of the current state: reductions only
+  } else if (!kick) {
+    // Setup: the chain carry starts at the current KE (main.cu:376-390).
+    nh.carry = 0.5 * ke_raw;
+    R.pending_scale = 1.0;
+  } else if (ens == FMD_NVT_NH) {
+    const double kT = ramp(R, R.step, R.T0, R.T1);
+    const double ke = 0.5 * ke_raw;
+    const double sc = nhc_half_step(nh.xi, nh.vxi, R.chain_M, R.Q1, R.Qr, kT, R.natoms, ke, 0.5 * dt,
+                                    nh.carry_dd ? nh.dd : nullptr);
+    nh.scale = sc;
+    nh.carry = ke * sc * sc;
+    R.pending_scale = sc;
+  } else if (ens == FMD_NPT_NH) {
+    const double kT = ramp(R, R.step, R.T0, R.T1), Pt = ramp(R, R.step, R.P0, R.P1);
+    const double vtr = R.vir[0] + R.vir[3] + R.vir[5];
+    npt_chain_baro(nh, false, ke_raw, vtr, R.chain_M, R.Q1, R.Qr, R.W, 0.5 * dt, dt, R.V0, R.natoms, kT, Pt,
+                   DExp(), DCbrt(), DSinh());
+    R.L = nh.L;
+    R.pending_scale = nh.bscale * nh.scale;
+  } else {
+    R.pending_scale = 1.0;
+  }
+  R.nh = nh;
+  R.thermo_step = R.step;
+  R.adv = 0;
+  R.rebuild_now = 0;
+  // scalars of the next pre-force, computed once here for all its blocks
+  next_scalars(R);
+  R.next_valid = 1;
+}
+
 // Per-replica commit of the post-force update (one warp per replica, after
 // every post-force block finished): reduce the chunk partials in chunk order
 // (deterministic), store energies / virial / KE, run the post-force chain or
@@ -2480,63 +2809,362 @@ __global__ void __launch_bounds__(kPostCommitThreads) k_post_commit(Dev d, int k
         for (int w = 1; w < nw; ++w) t += s_red[w][q];
         acc[q] = t;
       }
-      if (need_ev(R)) {
-        R.pe = acc[0];
-        for (int q = 0; q < 6; ++q) R.vir[q] = acc[1 + q];
-      }
-      for (int q = 0; q < 6; ++q) R.ke[q] = acc[7 + q];
-      const double ke_raw = acc[7] + acc[10] + acc[12];
-      const double dt = (R.mode == kModePushoff) ? R.push_dt : R.dt;
-      const int ens = (R.mode == kModePushoff) ? FMD_LANGEVIN : R.ensemble;
-      if (need_ev(R)) R.ev_step = R.step;
-      R.force_ev = 0;
-      // the chain / barostat state is updated in a local copy and stored
-      // once: in place, its arrays' stores would order every later read of
-      // the record behind them
-      NHScalars nh = R.nh;
-      if (kick == 2) {
-        // re-evaluation of the current state: reductions only
-      } else if (!kick) {
-        // Setup: the chain carry starts at the current KE (main.cu:376-390).
-        nh.carry = 0.5 * ke_raw;
-        R.pending_scale = 1.0;
-      } else if (ens == FMD_NVT_NH) {
-        const double kT = ramp(R, R.step, R.T0, R.T1);
-        const double ke = 0.5 * ke_raw;
-        const double sc = nhc_half_step(nh.xi, nh.vxi, R.chain_M, R.Q1, R.Qr, kT, R.natoms, ke, 0.5 * dt,
-                                        nh.carry_dd ? nh.dd : nullptr);
-        nh.scale = sc;
-        nh.carry = ke * sc * sc;
-        R.pending_scale = sc;
-      } else if (ens == FMD_NPT_NH) {
-        const double kT = ramp(R, R.step, R.T0, R.T1), Pt = ramp(R, R.step, R.P0, R.P1);
-        const double vtr = R.vir[0] + R.vir[3] + R.vir[5];
-        npt_chain_baro(nh, false, ke_raw, vtr, R.chain_M, R.Q1, R.Qr, R.W, 0.5 * dt, dt, R.V0, R.natoms, kT, Pt,
-                       DExp(), DCbrt(), DSinh());
-        R.L = nh.L;
-        R.pending_scale = nh.bscale * nh.scale;
-      } else {
-        R.pending_scale = 1.0;
-      }
-      R.nh = nh;
-      R.thermo_step = R.step;
-      R.adv = 0;
-      R.rebuild_now = 0;
-      // scalars of the next pre-force, computed once here for all its blocks
-      next_scalars(R);
-      R.next_valid = 1;
+      post_commit_state(R, acc, kick);
     }
     // Stress steps: the thermo row's pressure tensor, (KE tensor (with the
     // pending thermostat scale) + virial) / V in the current box, feeds the
     // correlator (main.cu:632-666).
     __syncwarp();
     if (kick == 1 && stress_step(R)) {
-      const double s2 = __dmul_rn(R.pending_scale, R.pending_scale);
-      const double V = __dmul_rn(__dmul_rn(R.L, R.L), R.L);
-      double smp[kAcfComps];
-      for (int c = 0; c < kAcfComps; ++c) smp[c] = __dadd_rn(__dmul_rn(R.ke[c], s2), R.vir[c]) / V;
-      acf_push(d.acf + (size_t)r * kAcfWords, smp);
+      acf_sample(d, R, r);
     }
+  }
+}
+
+// ---------------------------------------------------------------- resident steps
+// Many steps in one launch.  A replica is advanced by a group of resident
+// blocks (a cooperative launch), each owning a contiguous range of its
+// chunks; the group synchronises itself through flags in global memory, so
+// replicas do not wait for one another and one replica's pre-force or rebuild
+// runs beside another's forces on the same SM.  Every block keeps a copy of
+// the replica's record in shared memory and commits each step on it (the same
+// FP64 operations on the same values in every block), so a step needs no
+// serial kernel: a Langevin step is one group barrier (positions and the
+// displacement maximum complete), a Nose-Hoover or energy step two (the KE
+// partials complete).  Positions alternate between the two position buffers,
+// which the rebuild's scratch copy shares, so the next pre-force may start
+// while other blocks still read this step's positions.
+//
+// What bounds it: the latency of the per-step chain (loads of the pre-force,
+// barrier, list walk), where the graph's step pays a chain of kernel and
+// conditional nodes (about 40 us however small the system).  All arithmetic is
+// that of the per-kernel path's device functions in the same order, so the
+// trajectories are bit-identical to it.
+//
+// LPA lanes per atom (blocks of LPA * kChunk threads): 4 for batches whose
+// every chunk has a resident block of that width, 1 beyond.
+constexpr int kStepWin = 704;       // list candidates staged per window: one 27-cell stencil of a melt
+constexpr int kStepSpin = 1 << 22;  // polls of a group barrier before the replica is given up (seconds)
+constexpr int step_threads(int lpa) { return lpa * kChunk; }
+// 6 blocks of 128 threads (80 registers: the energy flavour and the list
+// build do not spill), 2 blocks of 512 (64 registers)
+constexpr int step_blocks_per_sm(int lpa) { return lpa == 1 ? 6 : 2; }
+
+// Relaxed polls (an acquire per poll would drop the SM's L1 lines each time);
+// a fence follows the last.
+__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// A replica's group of blocks within k_steps.
+struct StepGroup {
+  int r, rank, nb;            // replica, this block's rank, blocks
+  int c0, c1;                 // this block's chunks
+  unsigned long long* flags;  // the group's words: barrier number << 32 | value, two sets in turn
+  int stride;                 // from one set to the other
+  unsigned seq;               // number of the last barrier
+  int* dead;                  // shared: a barrier ran out of polls
+  uint32_t* s_max;            // shared: per-warp maxima
+};
+
+// Barrier over the group's blocks; memory written by them before it is
+// visible after it (the fence also drops this SM's stale L1 lines).  Each
+// block posts its number in its own word and polls every block's, so arrival
+// and release are one store and one load apart; a word carries a value
+// (value: thread 0's), and thread 0 gets the largest back in most.  A block
+// is at most one barrier ahead of another's reads: two sets of words are
+// enough.  False when the wait ran out: the replica is faulted and the block
+// gives up.
+__device__ __forceinline__ bool group_sync(StepGroup& g, uint32_t value = 0u, uint32_t* most = nullptr) {
+  const unsigned seq = ++g.seq;
+  __syncthreads();
+  uint32_t m = value;
+  if (g.nb > 1) {
+    unsigned long long* const f = g.flags + (seq & 1u) * g.stride;
+    if (threadIdx.x == 0) {
+      __threadfence();
+      st_relaxed(f + g.rank, ((unsigned long long)seq << 32) | value);
+    }
+    if ((int)(threadIdx.x & ~31u) < g.nb) {  // the warps that poll
+      for (int i = threadIdx.x; i < g.nb; i += blockDim.x) {
+        unsigned long long w = ld_relaxed(f + i);
+        for (int polls = 0; (int)((unsigned)(w >> 32) - seq) < 0; w = ld_relaxed(f + i))
+          if (++polls > kStepSpin) {
+            *g.dead = 1;
+            break;
+          }
+        m = max(m, (uint32_t)w);
+      }
+      __threadfence();
+      if (most) {
+        warp_max_u32(m);
+        if ((threadIdx.x & 31) == 0) g.s_max[threadIdx.x >> 5] = m;
+      }
+    }
+    __syncthreads();
+    if (most && threadIdx.x == 0)
+      for (int w = 0; w < (int)(blockDim.x >> 5) && 32 * w < g.nb; ++w) m = max(m, g.s_max[w]);
+  }
+  if (most) *most = m;
+  return *g.dead == 0;
+}
+
+// Exclusive scan of the replica's cell counts by one block of T threads (see k_scan).
+template <int T>
+__device__ __forceinline__ void scan_cells_block(const Dev& d, const Rep& R) {
+  constexpr int W = T / 32, per = 8;
+  __shared__ int s_w[W];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ncell = R.P * R.P * R.P;
+  int* const cnt = d.cell_cnt + R.cell_base;
+  int* const start = d.cell_start + R.cell_base;
+  int* const fill = d.cell_fill + R.cell_base;
+  int carry = 0;
+  for (int t0 = 0; t0 < ncell; t0 += T * per) {
+    const int c0 = t0 + threadIdx.x * per;
+    int v[per], sum = 0;
+#pragma unroll
+    for (int j = 0; j < per; ++j) {
+      v[j] = c0 + j < ncell ? cnt[c0 + j] : 0;
+      sum += v[j];
+    }
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane >= o) incl += x;
+    }
+    __syncthreads();  // the previous tile's totals are read
+    if (lane == 31) s_w[warp] = incl;
+    __syncthreads();
+    int run = carry + incl - sum;
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      if (w < warp) run += s_w[w];
+      carry += s_w[w];
+    }
+#pragma unroll
+    for (int j = 0; j < per; ++j)
+      if (c0 + j < ncell) {
+        start[c0 + j] = run;
+        fill[c0 + j] = run;
+        cnt[c0 + j] = 0;
+        run += v[j];
+      }
+  }
+}
+
+// The rebuild of a group's replica: the phases of launch_rebuild with a group
+// barrier in the place of each kernel boundary.
+template <int LPA>
+__device__ __noinline__ bool rebuild_group(const Dev& d, Rep& R, StepGroup& g) {
+  constexpr int T = step_threads(LPA), W = T / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int t = threadIdx.x % kChunk, cf = g.c0 + threadIdx.x / kChunk;  // LPA chunks at a time
+  for (int c = cf; c < g.c1; c += LPA) bin_chunk(d, R, c, t);
+  if (!group_sync(g)) return false;
+  if (g.rank == 0) scan_cells_block<T>(d, R);
+  if (threadIdx.x == 0) {
+    int Gn = (int)floor(R.L / ((R.rc + R.skin) * 1.0001));
+    Gn = Gn < 1 ? 1 : (Gn > R.G_alloc ? R.G_alloc : Gn);
+    R.G = Gn;
+    R.h = (float)(R.L / Gn);
+  }
+  if (!group_sync(g)) return false;
+  for (int c = cf; c < g.c1; c += LPA) scatter_chunk(d, R, c, t);
+  if (!group_sync(g)) return false;
+  const int ncell = R.P * R.P * R.P;
+  for (int c = g.rank * W + warp; c < ncell; c += g.nb * W) cellsort_cell(d, R, c, lane);
+  if (!group_sync(g)) return false;
+  for (int c = cf; c < g.c1; c += LPA) permute_chunk(d, R, c, t);
+  if (!group_sync(g)) return false;
+  for (int c = cf; c < g.c1; c += LPA) topo_chunk(d, R, c, t);
+  if (!group_sync(g)) return false;
+  int* const status = &d.reps[g.r].status;
+  const int home = R.G * R.G * R.G;
+  for (int lc = g.rank; lc < home; lc += g.nb) {
+    if (R.G >= 3) {
+      __syncthreads();  // the previous cell's staging is no longer read
+      neighbors_cell_ballot<kStepWin, W>(d, R, status, lc);
+    } else {
+      const int ov = neighbors_small_box(d, R, lc, lane, 32 * warp, T);
+      if (ov) atomicOr(status, ov);
+    }
+  }
+  return group_sync(g);
+}
+
+template <bool EV, int KB, int LPA>
+__device__ __forceinline__ void forces_group(const Dev& d, const Rep& R, const StepGroup& g) {
+  for (int c = g.c0; c < g.c1; ++c) {
+    const int4 ci = make_int4(g.r, R.slot_base + c * kChunk, 0, c);
+    const int chunk = R.chunk_base + c;
+    if (!EV && LPA == 4) {
+      if (R.rebuild_now)
+        force_chunk_quads<KB, true>(d, R, g.r, c);
+      else
+        force_chunk_quads<KB, false>(d, R, g.r, c);
+    } else if (R.rebuild_now) {
+      force_chunk_of<EV, 4, true, KB, true, 1, true>(d, R, ci, chunk);
+    } else {
+      force_chunk_of<EV, 4, true, KB, false, 1, true>(d, R, ci, chunk);
+    }
+    __syncthreads();  // the tables and the block partials' staging are free again
+    if (R.ntables) {
+      table_chunk<EV>(d, R, ci, chunk);
+      __syncthreads();
+    }
+  }
+}
+
+// The replica's partials (values q0 .. 12) summed in k_post_commit's order by
+// a block of T threads: thread t of its kPostCommitThreads adds chunks t,
+// t + kPostCommitThreads, ..., a shuffle tree per warp, then the warp totals
+// in order.
+template <int T>
+__device__ __forceinline__ void reduce_partials(const Dev& d, const Rep& R, int q0, double (*s_red)[13], double* s_acc) {
+  const int lane = threadIdx.x & 31;
+  constexpr int nw = kPostCommitThreads / 32;
+  for (int vt = threadIdx.x; vt < kPostCommitThreads; vt += T) {
+    if (vt - lane >= R.nchunks) {  // warp-uniform: no chunks, zero totals
+      if (lane < 13) s_red[vt >> 5][lane] = 0.0;
+      continue;
+    }
+    double acc[13];
+#pragma unroll
+    for (int q = 0; q < 13; ++q) acc[q] = 0.0;
+    for (int c = vt; c < R.nchunks; c += kPostCommitThreads)
+#pragma unroll
+      for (int q = 0; q < 13; ++q)
+        if (q >= q0) acc[q] += d.part[q * d.part_stride + R.chunk_base + c];
+#pragma unroll
+    for (int q = 0; q < 13; ++q) {
+      if (q >= q0) acc[q] = warp_sum(acc[q]);
+      if (lane == 0) s_red[vt >> 5][q] = acc[q];
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < 13) {
+    double t = s_red[0][threadIdx.x];
+#pragma unroll
+    for (int w = 1; w < nw; ++w) t += s_red[w][threadIdx.x];
+    s_acc[threadIdx.x] = t;
+  }
+  __syncthreads();
+}
+
+template <int KB, int LPA>
+__global__ void __launch_bounds__(step_threads(LPA), step_blocks_per_sm(LPA))
+    k_steps(Dev d, const int4* plan, unsigned long long* flags, unsigned seq, int max_steps) {
+  constexpr int T = step_threads(LPA);
+  __shared__ __align__(16) Rep R;
+  __shared__ int dead;
+  __shared__ uint32_t s_max[T / 32];
+  __shared__ double s_red[kPostCommitThreads / 32][13], s_acc[13];
+  const int4 pl = plan[blockIdx.x];
+  StepGroup g;
+  g.r = pl.x;
+  g.rank = pl.y;
+  g.nb = pl.z;
+  g.flags = flags + pl.w;
+  g.stride = gridDim.x;
+  g.seq = seq;
+  g.dead = &dead;
+  g.s_max = s_max;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  static_assert(sizeof(Rep) % 8 == 0, "the record is copied in 8-byte words");
+  constexpr int kRepWords = (int)(sizeof(Rep) / 8);
+  {
+    const unsigned long long* src = reinterpret_cast<const unsigned long long*>(d.reps + g.r);
+    unsigned long long* dst = reinterpret_cast<unsigned long long*>(&R);
+    for (int k = threadIdx.x; k < kRepWords; k += T) dst[k] = src[k];
+  }
+  if (threadIdx.x == 0) dead = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(d.kcount + kKForce, 1ull);
+  __syncthreads();
+  g.c0 = (int)((int64_t)g.rank * R.nchunks / g.nb);
+  g.c1 = (int)((int64_t)(g.rank + 1) * R.nchunks / g.nb);
+  const int64_t left = R.active ? R.stop_step - R.step : 0;
+  const int steps = (int)(left < max_steps ? left : max_steps);
+  if (steps <= 0) return;  // the same in every block of the group
+  if (!R.next_valid) {
+    if (g.rank == 0 && threadIdx.x == 0) atomicOr(&d.reps[g.r].status, kStatusStaleScalars);
+    return;
+  }
+  float4* const home = d.pos;
+  for (int k = 0; k < steps; ++k) {
+    // pre-force: this step's positions go to the other buffer
+    float4* const from = d.pos;
+    d.pos = d.tpos;
+    d.tpos = from;
+    uint32_t d2bits = 0;
+    int bad = 0;
+    const bool deferred = R.defer != 0;
+    for (int c = g.c0 + threadIdx.x / kChunk; c < g.c1; c += LPA) {
+      const int local = c * kChunk + threadIdx.x % kChunk, s = R.slot_base + local;
+      if (local < R.natoms)
+        pre_atom(d, R, R.next, s, deferred, from[s], d.vel[s], d.force[s], d.ref[s], d2bits, bad);
+    }
+    if (bad) atomicOr(&d.reps[g.r].status, kStatusNonFinite);
+    warp_max_u32(d2bits);
+    if (lane == 0) s_max[warp] = d2bits;
+    __syncthreads();
+    uint32_t m = 0;
+    if (threadIdx.x == 0)
+      for (int w = 0; w < T / 32; ++w) m = max(m, s_max[w]);
+    if (!group_sync(g, m, &m)) break;
+    // commit, on this block's copy of the record
+    if (threadIdx.x == 0) {
+      R.maxdisp_bits = max(R.maxdisp_bits, m);
+      commit_state<false>(R, R.next);
+      R.defer = post_needed(R) ? 0 : 1;
+    }
+    __syncthreads();
+    if (R.rebuild_now == kListRebuild && !rebuild_group<LPA>(d, R, g)) break;
+    const bool defer = R.defer != 0;
+    if (need_ev(R))
+      forces_group<true, KB, LPA>(d, R, g);
+    else
+      forces_group<false, KB, LPA>(d, R, g);
+    if (defer) {
+      if (threadIdx.x == 0) {
+        step_scalars<false>(R, R.next);
+        R.next_valid = 1;
+      }
+    } else {
+      for (int c = g.c0; c < g.c1; ++c) {
+        const int local = c * kChunk + threadIdx.x, s = R.slot_base + local;
+        const bool have = threadIdx.x < kChunk && local < R.natoms;
+        const float4 v = have ? d.vel[s] : make_float4(0, 0, 0, 1), f = have ? d.force[s] : make_float4(0, 0, 0, 0);
+        post_chunk(d, R, R.chunk_base + c, s, have, v, f, 1);
+        __syncthreads();  // the block partials' staging is free again
+      }
+      if (!group_sync(g)) break;
+      reduce_partials<T>(d, R, need_ev(R) ? 0 : 7, s_red, s_acc);
+      if (threadIdx.x == 0) post_commit_state(R, s_acc, 1);
+      __syncthreads();
+      if (g.rank == 0 && warp == 0 && stress_step(R)) acf_sample(d, R, g.r);
+    }
+    __syncthreads();  // the record is complete
+  }
+  if (dead && threadIdx.x == 0) atomicOr(&d.reps[g.r].status, kStatusTimeout);
+  if (d.pos != home)  // no block reads the other buffer any more
+    for (int c = g.c0 + threadIdx.x / kChunk; c < g.c1; c += LPA) {
+      const int local = c * kChunk + threadIdx.x % kChunk, s = R.slot_base + local;
+      if (local < R.natoms) home[s] = d.pos[s];
+    }
+  if (g.rank == 0) {
+    // the record, less its status word (raised in place by any block)
+    const unsigned* src = reinterpret_cast<const unsigned*>(&R);
+    unsigned* dst = reinterpret_cast<unsigned*>(d.reps + g.r);
+    constexpr int skip = (int)(offsetof(Rep, status) / 4);
+    for (int w = threadIdx.x; w < 2 * kRepWords; w += T)
+      if (w != skip) dst[w] = src[w];
   }
 }
 
@@ -2616,19 +3244,14 @@ __global__ void __launch_bounds__(kChunk) k_bin_g(Dev d) {
   count_launch(d, kKBin);
   const int4 ci = d.chunk_rep[blockIdx.x];
   if (ci.x < 0 || d.reps[ci.x].rebuild_now != 1) return;
-  bin_chunk(d, d.reps[ci.x], ci.w);
+  bin_chunk(d, d.reps[ci.x], ci.w, threadIdx.x);
 }
 
 __global__ void __launch_bounds__(kChunk) k_scatter_g(Dev d) {
   count_launch(d, kKScatter);
   const int4 ci = d.chunk_rep[blockIdx.x];
   if (ci.x < 0 || d.reps[ci.x].rebuild_now != 1) return;
-  const Rep& R = d.reps[ci.x];
-  const int local = ci.w * kChunk + threadIdx.x;
-  if (local >= R.natoms) return;
-  const int s = R.slot_base + local;
-  const int at = atomicAdd(&d.cell_fill[R.cell_base + d.key[s]], 1);
-  d.bucket[R.slot_base + at] = local;
+  scatter_chunk(d, d.reps[ci.x], ci.w, threadIdx.x);
 }
 
 __global__ void __launch_bounds__(32 * kCellGroup) k_cellsort_g(Dev d) {
@@ -2644,14 +3267,14 @@ __global__ void __launch_bounds__(kChunk) k_permute_g(Dev d) {
   count_launch(d, kKPermute);
   const int4 ci = d.chunk_rep[blockIdx.x];
   if (ci.x < 0 || d.reps[ci.x].rebuild_now != 1) return;
-  permute_chunk(d, d.reps[ci.x], ci.w);
+  permute_chunk(d, d.reps[ci.x], ci.w, threadIdx.x);
 }
 
 __global__ void __launch_bounds__(kChunk) k_topo_g(Dev d) {
   count_launch(d, kKTopo);
   const int4 ci = d.chunk_rep[blockIdx.x];
   if (ci.x < 0 || d.reps[ci.x].rebuild_now != 1) return;
-  topo_chunk(d, d.reps[ci.x], ci.w);
+  topo_chunk(d, d.reps[ci.x], ci.w, threadIdx.x);
 }
 
 __global__ void __launch_bounds__(kNbrThreads) k_neighbors_g(Dev d) {
@@ -2661,7 +3284,7 @@ __global__ void __launch_bounds__(kNbrThreads) k_neighbors_g(Dev d) {
   if (R.rebuild_now != 1) return;
   const int G = R.G;
   if ((int)blockIdx.x >= G * G * G) return;
-  neighbors_cell_ballot(d, R, blockIdx.x);
+  neighbors_cell_ballot<kNbrWin, kNbrWarps>(d, R, &R.status, blockIdx.x);
 }
 
 // ---------------------------------------------------------------- launchers
@@ -2684,6 +3307,31 @@ int resident_grid(K kernel, int threads) {
   return num_sms() * (per_sm > 0 ? per_sm : 1);
 }
 }  // namespace
+
+int steps_resident_blocks(int lpa) {
+  static const int n1 = std::min(resident_grid(k_steps<1, 1>, step_threads(1)), resident_grid(k_steps<2, 1>, step_threads(1)));
+  static const int n4 = std::min(resident_grid(k_steps<1, 4>, step_threads(4)), resident_grid(k_steps<2, 4>, step_threads(4)));
+  return lpa == 4 ? n4 : n1;
+}
+
+bool steps_variant(int force_variant) { return force_variant != 9 && force_variant != 10; }
+
+void launch_steps(const Dev& d, const int4* plan, int blocks, int lpa, unsigned long long* flags, unsigned seq,
+                  int force_variant, int max_steps, cudaStream_t st) {
+  const bool two = force_variant == 1 || force_variant == 3 || force_variant == 5;
+  void (*const kernel)(Dev, const int4*, unsigned long long*, unsigned, int) =
+      lpa == 4 ? (two ? k_steps<2, 4> : k_steps<1, 4>) : (two ? k_steps<2, 1> : k_steps<1, 1>);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = blocks;
+  cfg.blockDim = step_threads(lpa);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;  // every block resident: they wait for one another
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  FMD_CUDA(cudaLaunchKernelEx(&cfg, kernel, d, plan, flags, seq, max_steps));
+}
 
 // The pre-force update of every chunk, one block per chunk.  (A resident
 // grid streaming the chunks through shared memory by asynchronous copies
