@@ -13,6 +13,7 @@
 // raises a flag instead of truncating silently; the caller owns all memory.
 #include <cub/cub.cuh>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <mutex>
@@ -20,6 +21,7 @@
 
 #include "dev_common.cuh"
 #include "host.h"
+#include "verlet_cells.cuh"
 
 namespace fmd {
 namespace launch {
@@ -58,19 +60,22 @@ inline VerletGeom verlet_geom(float L, float rcs) {
 }
 
 struct VerletScratch {
-  int* cid;
   int* cid_sorted;
-  int* aid;
   int* sorted;
   int* start;
   int* end;
+  int* cid;
+  int* aid;
   void* cub;
+  float4* spos;
   size_t cub_bytes;
   size_t total;
 };
 
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
+// The sort's input and temporary storage come last: once it is done the
+// positions in sorted order take their place.
 VerletScratch verlet_carve(void* base, int n, int ncell) {
   VerletScratch s{};
   size_t cub_bytes = 0;
@@ -82,15 +87,17 @@ VerletScratch verlet_carve(void* base, int n, int ncell) {
     off += align256(bytes);
     return q;
   };
-  s.cid = (int*)take(sizeof(int) * n);
   s.cid_sorted = (int*)take(sizeof(int) * n);
-  s.aid = (int*)take(sizeof(int) * n);
   s.sorted = (int*)take(sizeof(int) * n);
   s.start = (int*)take(sizeof(int) * ncell);
   s.end = (int*)take(sizeof(int) * ncell);
+  const size_t reuse = off;
+  s.cid = (int*)take(sizeof(int) * n);
+  s.aid = (int*)take(sizeof(int) * n);
   s.cub = take(cub_bytes);
   s.cub_bytes = cub_bytes;
-  s.total = off;
+  s.spos = p ? (float4*)(p + reuse) : nullptr;
+  s.total = std::max(off, reuse + align256(sizeof(float4) * n));
   return s;
 }
 
@@ -206,15 +213,28 @@ __global__ void k_lj(const float4* __restrict__ pos, float4* __restrict__ force,
     const float4 pi = pos[i];
     const int ti = __float_as_int(pi.w);
     const int nn = __ldg(&cnt[i]);
-    for (int k = 0; k < nn; ++k) {
-      const int j = __ldg(&nbr[(size_t)k * n + i]);
-      const float4 pj = __ldg(&pos[j]);
-      const float dx = min_image_f(pi.x - pj.x, L, inv_L);
-      const float dy = min_image_f(pi.y - pj.y, L, inv_L);
-      const float dz = min_image_f(pi.z - pj.z, L, inv_L);
-      const float r2 = dx * dx + dy * dy + dz * dz;
-      if (r2 < rc2 && r2 > 1e-10f)
-        lj_ref_pair(__ldg(&lj[ti * ntypes + __float_as_int(pj.w)]), dx, dy, dz, r2, fx, fy, fz, pe, v);
+    // batches of B entries: the list words (a batch ahead), then the
+    // positions, then the pairs in list order
+    constexpr int B = 4;
+    const int* const row = nbr + i;
+    int jn[B];
+#pragma unroll
+    for (int q = 0; q < B; ++q) jn[q] = q < nn ? __ldg(row + (size_t)q * n) : i;
+    for (int k = 0; k < nn; k += B) {
+      float4 pj[B];
+#pragma unroll
+      for (int q = 0; q < B; ++q) pj[q] = __ldg(&pos[jn[q]]);
+#pragma unroll
+      for (int q = 0; q < B; ++q) jn[q] = k + B + q < nn ? __ldg(row + (size_t)(k + B + q) * n) : i;
+#pragma unroll
+      for (int q = 0; q < B; ++q) {
+        const float dx = min_image_f(pi.x - pj[q].x, L, inv_L);
+        const float dy = min_image_f(pi.y - pj[q].y, L, inv_L);
+        const float dz = min_image_f(pi.z - pj[q].z, L, inv_L);
+        const float r2 = dx * dx + dy * dy + dz * dz;
+        if (k + q < nn && r2 < rc2 && r2 > 1e-10f)
+          lj_ref_pair(__ldg(&lj[ti * ntypes + __float_as_int(pj[q].w)]), dx, dy, dz, r2, fx, fy, fz, pe, v);
+      }
     }
     force[i] = make_float4(fx, fy, fz, pe);
   }
@@ -549,12 +569,23 @@ void verlet_build_into(const void* pos, int32_t natoms, float box_L, const int32
     k_assign<<<gr, kBlock, 0, st>>>((const float4*)pos, s.cid, s.aid, natoms, g.inv_cell, g.nx);
     FMD_CUDA_LAUNCH();
     size_t cb = s.cub_bytes;
-    FMD_CUDA(cub::DeviceRadixSort::SortPairs(s.cub, cb, s.cid, s.cid_sorted, s.aid, s.sorted, natoms, 0, 32, st));
-    FMD_CUDA(cudaMemsetAsync(s.start, 0, sizeof(int) * g.ncell, st));
-    FMD_CUDA(cudaMemsetAsync(s.end, 0, sizeof(int) * g.ncell, st));
+    FMD_CUDA(cub::DeviceRadixSort::SortPairs(s.cub, cb, s.cid, s.cid_sorted, s.aid, s.sorted, natoms, 0,
+                                             cells::key_bits(g.ncell), st));
+    // start and end are one range of the scratch
+    FMD_CUDA(cudaMemsetAsync(s.start, 0, (char*)(s.end + g.ncell) - (char*)s.start, st));
+    const float rcs2 = rc_skin * rc_skin;
+    if (cells::list_by_cells(natoms, g.nx)) {
+      cells::k_sorted<float4, float><<<gr, kBlock, 0, st>>>((const float4*)pos, s.sorted, s.cid_sorted, s.start, s.end,
+                                                            s.spos, natoms);
+      FMD_CUDA_LAUNCH();
+      cells::k_list_cells<float4, float><<<g.ncell, cells::kThreads, 0, st>>>(
+          s.spos, s.start, s.end, excl_off, excl_list, neighbors, num_neighbors, natoms, g.nx, rcs2, box_L,
+          1.0f / box_L, max_neighbors, overflow_flag, 1);
+      FMD_CUDA_LAUNCH();
+      return;
+    }
     k_ranges<<<gr, kBlock, 0, st>>>(s.cid_sorted, s.start, s.end, natoms);
     FMD_CUDA_LAUNCH();
-    const float rcs2 = rc_skin * rc_skin;
     k_build<<<gr, kBlock, 0, st>>>((const float4*)pos, s.sorted, s.cid_sorted, s.start, s.end, excl_off, excl_list,
                                    neighbors, num_neighbors, natoms, g.nx, rcs2, box_L, 1.0f / box_L, max_neighbors,
                                    overflow_flag);
