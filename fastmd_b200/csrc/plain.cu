@@ -26,6 +26,7 @@
 #include "dev_common.cuh"
 #include "engine.h"
 #include "nhc.h"
+#include "verlet_cells.cuh"
 
 namespace fmd {
 namespace plain {
@@ -345,55 +346,88 @@ __device__ __forceinline__ void block_add_virial(double v[6], double* virial) {
   }
 }
 
-// lj.cu:4-107 in FP64: force[i] overwritten with (F, pe_i).
+// lj.cu:4-107 in FP64: force[i] overwritten with (F, pe_i).  LPA lanes of a
+// warp share an atom, 32 / LPA lanes apart (a list row is read in whole
+// sectors): lane group g takes entries g, g + LPA, ..., and the groups' sums
+// are added by a shuffle tree.  A list walk is a chain of dependent loads, so
+// one thread per atom left a few thousand atoms waiting on memory: 12,000
+// atoms, 77 us with one lane.
+template <int LPA>
 __global__ void k_lj(const double4* pos, double4* force, double* virial, const double2* lj, const int* nbr,
                      const int* cnt, int n, int ntypes, double rc2, double L, double inv_L, int clamp) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr int APW = 32 / LPA;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31, g = lane / APW;
+  const int i = (t >> 5) * APW + lane % APW;
   double fx = 0.0, fy = 0.0, fz = 0.0, pe = 0.0;
   double v[6] = {0, 0, 0, 0, 0, 0};
   if (i < n) {
     const double4 pi = pos[i];
     const int ti = type_of(pi);
     const int nn = cnt[i];
-    for (int k = 0; k < nn; ++k) {
-      const int j = nbr[(size_t)k * n + i];
-      const double4 pj = pos[j];
-      const double dx = min_image(pi.x - pj.x, L, inv_L);
-      const double dy = min_image(pi.y - pj.y, L, inv_L);
-      const double dz = min_image(pi.z - pj.z, L, inv_L);
-      const double r2 = dx * dx + dy * dy + dz * dz;
-      if (r2 < rc2 && r2 > 1e-10) {
-        const double2 p = lj[ti * ntypes + type_of(pj)];
-        const double eps = p.x, sig = p.y;
-        const double sig2 = sig * sig;
-        const double r2inv = 1.0 / r2;
-        const double sr2 = sig2 * r2inv;
-        const double sr6 = sr2 * sr2 * sr2;
-        const double sr12 = sr6 * sr6;
-        double fr = 24.0 * eps * r2inv * (2.0 * sr12 - sr6);
-        if (clamp) fr = fmin(fmax(fr, -1000.0), 1000.0);
-        const double fxij = fr * dx, fyij = fr * dy, fzij = fr * dz;
-        fx += fxij;
-        fy += fyij;
-        fz += fzij;
-        pe += 0.5 * 4.0 * eps * (sr12 - sr6);
-        v[0] += 0.5 * fxij * dx;
-        v[1] += 0.5 * fxij * dy;
-        v[2] += 0.5 * fxij * dz;
-        v[3] += 0.5 * fyij * dy;
-        v[4] += 0.5 * fyij * dz;
-        v[5] += 0.5 * fzij * dz;
+    constexpr int B = 2;  // entries in flight per lane, the next ones' words a batch ahead
+    int jn[B];
+#pragma unroll
+    for (int q = 0; q < B; ++q) jn[q] = g + q * LPA < nn ? nbr[(size_t)(g + q * LPA) * n + i] : i;
+    for (int k = g; k < nn; k += B * LPA) {
+      double4 pj[B];
+#pragma unroll
+      for (int q = 0; q < B; ++q) pj[q] = pos[jn[q]];
+#pragma unroll
+      for (int q = 0; q < B; ++q) {
+        const int kn = k + (B + q) * LPA;
+        jn[q] = kn < nn ? nbr[(size_t)kn * n + i] : i;
+      }
+#pragma unroll
+      for (int q = 0; q < B; ++q) {
+        const double dx = min_image(pi.x - pj[q].x, L, inv_L);
+        const double dy = min_image(pi.y - pj[q].y, L, inv_L);
+        const double dz = min_image(pi.z - pj[q].z, L, inv_L);
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        if (k + q * LPA < nn && r2 < rc2 && r2 > 1e-10) {
+          const double2 p = lj[ti * ntypes + type_of(pj[q])];
+          const double eps = p.x, sig = p.y;
+          const double sig2 = sig * sig;
+          const double r2inv = 1.0 / r2;
+          const double sr2 = sig2 * r2inv;
+          const double sr6 = sr2 * sr2 * sr2;
+          const double sr12 = sr6 * sr6;
+          double fr = 24.0 * eps * r2inv * (2.0 * sr12 - sr6);
+          if (clamp) fr = fmin(fmax(fr, -1000.0), 1000.0);
+          const double fxij = fr * dx, fyij = fr * dy, fzij = fr * dz;
+          fx += fxij;
+          fy += fyij;
+          fz += fzij;
+          pe += 0.5 * 4.0 * eps * (sr12 - sr6);
+          v[0] += 0.5 * fxij * dx;
+          v[1] += 0.5 * fxij * dy;
+          v[2] += 0.5 * fxij * dz;
+          v[3] += 0.5 * fyij * dy;
+          v[4] += 0.5 * fyij * dz;
+          v[5] += 0.5 * fzij * dz;
+        }
       }
     }
-    force[i] = make_double4(fx, fy, fz, pe);
   }
+#pragma unroll
+  for (int o = 16; o >= APW; o >>= 1) {
+    fx += __shfl_xor_sync(0xFFFFFFFFu, fx, o);
+    fy += __shfl_xor_sync(0xFFFFFFFFu, fy, o);
+    fz += __shfl_xor_sync(0xFFFFFFFFu, fz, o);
+    pe += __shfl_xor_sync(0xFFFFFFFFu, pe, o);
+  }
+  if (i < n && g == 0) force[i] = make_double4(fx, fy, fz, pe);
   block_add_virial(v, virial);
 }
 
+// Lanes per atom: as many as keep the atoms' threads within one resident
+// wave (148 SMs of 1,024 threads); larger systems fill the GPU without.
+constexpr int kLjThreads = 148 * 1024;
+
 // fene.cu:4-101 in FP64 with atomic scatter; over-stretch reported.
-__global__ void k_fene(const double4* pos, double4* force, double* virial, const int2* bonds, const int* btype,
-                       const double4* fp, int nb, double L, double inv_L, int clamp, int* status) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void fene_block(const double4* pos, double4* force, double* virial, const int2* bonds,
+                                           const int* btype, const double4* fp, int nb, double L, double inv_L,
+                                           int clamp, int* status, int block) {
+  const int b = block * blockDim.x + threadIdx.x;
   double v[6] = {0, 0, 0, 0, 0, 0};
   if (b < nb) {
     const int2 bd = bonds[b];
@@ -442,9 +476,9 @@ __global__ void k_fene(const double4* pos, double4* force, double* virial, const
 }
 
 // angle.cu:4-108 in FP64 with atomic scatter.
-__global__ void k_angle(const double4* pos, double4* force, double* virial, const int4* angles, const double2* ap,
-                        int na, double L, double inv_L) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void angle_block(const double4* pos, double4* force, double* virial, const int4* angles,
+                                            const double2* ap, int na, double L, double inv_L, int block) {
+  const int a = block * blockDim.x + threadIdx.x;
   double v[6] = {0, 0, 0, 0, 0, 0};
   if (a < na) {
     const int4 an = angles[a];
@@ -497,6 +531,16 @@ __global__ void k_angle(const double4* pos, double4* force, double* virial, cons
     v[5] = fiz * dzij + fkz * dzkj;
   }
   block_add_virial(v, virial);
+}
+
+// Bonds and angles in one launch: the first bond_blocks blocks take the bonds.
+__global__ void k_bonded(const double4* pos, double4* force, double* virial, const int2* bonds, const int* btype,
+                         const double4* fp, int nb, int bond_blocks, const int4* angles, const double2* ap, int na,
+                         double L, double inv_L, int clamp, int* status) {
+  if ((int)blockIdx.x < bond_blocks)
+    fene_block(pos, force, virial, bonds, btype, fp, nb, L, inv_L, clamp, status, blockIdx.x);
+  else
+    angle_block(pos, force, virial, angles, ap, na, L, inv_L, blockIdx.x - bond_blocks);
 }
 
 __global__ void k_cap(double4* force, int n, double cap) {
@@ -655,12 +699,15 @@ class PlainEngine final : public SimEngine {
     scid_.alloc(n_);
     aid_.alloc(n_);
     sorted_.alloc(n_);
+    spos_.alloc(n_);
     cstart_.alloc(cell_cap_);
     cend_.alloc(cell_cap_);
     size_t tb = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, tb, (int*)nullptr, (int*)nullptr, (int*)nullptr, (int*)nullptr, n_);
     cub_tmp_.alloc(tb);
     maxdr2_.alloc_zero(1);
+    disp_.alloc(sizeof(double));
+    FMD_CUDA(cudaEventCreateWithFlags(&disp_ready_, cudaEventDisableTiming));
     virial_.alloc_zero(6);
     status_.alloc_zero(1);
     red_.alloc_zero(8);
@@ -703,6 +750,7 @@ class PlainEngine final : public SimEngine {
   }
 
   ~PlainEngine() override {
+    if (disp_ready_) cudaEventDestroy(disp_ready_);
     if (st_) cudaStreamDestroy(st_);
   }
 
@@ -928,14 +976,23 @@ class PlainEngine final : public SimEngine {
     k_assign_cells<<<g, kBlock, 0, st_>>>(pos_, cid_, aid_, n_, inv_cell, nx);
     FMD_CUDA_LAUNCH();
     size_t tb = cub_tmp_.bytes();
-    FMD_CUDA(cub::DeviceRadixSort::SortPairs(cub_tmp_.p, tb, cid_.p, scid_.p, aid_.p, sorted_.p, n_, 0, 32, st_));
+    FMD_CUDA(cub::DeviceRadixSort::SortPairs(cub_tmp_.p, tb, cid_.p, scid_.p, aid_.p, sorted_.p, n_, 0,
+                                             cells::key_bits(ncell), st_));
     FMD_CUDA(cudaMemsetAsync(cstart_, 0, ncell * sizeof(int), st_));
     FMD_CUDA(cudaMemsetAsync(cend_, 0, ncell * sizeof(int), st_));
-    k_cell_ranges<<<g, kBlock, 0, st_>>>(scid_, cstart_, cend_, n_);
-    FMD_CUDA_LAUNCH();
-    k_verlet<<<g, kBlock, 0, st_>>>(pos_, sorted_, scid_, cstart_, cend_, nb_ ? eoff_.p : nullptr,
-                                    nb_ ? elist_.p : nullptr, nbr_, cnt_, n_, nx, rcs_ * rcs_, L_, 1.0 / L_,
-                                    max_nbr_, status_);
+    if (cells::list_by_cells(n_, nx)) {
+      cells::k_sorted<double4, double><<<g, kBlock, 0, st_>>>(pos_, sorted_, scid_, cstart_, cend_, spos_, n_);
+      FMD_CUDA_LAUNCH();
+      cells::k_list_cells<double4, double><<<ncell, cells::kThreads, 0, st_>>>(
+          spos_, cstart_, cend_, nb_ ? eoff_.p : nullptr, nb_ ? elist_.p : nullptr, nbr_, cnt_, n_, nx, rcs_ * rcs_, L_,
+          1.0 / L_, max_nbr_, status_, kStatusOverflow);
+    } else {
+      k_cell_ranges<<<g, kBlock, 0, st_>>>(scid_, cstart_, cend_, n_);
+      FMD_CUDA_LAUNCH();
+      k_verlet<<<g, kBlock, 0, st_>>>(pos_, sorted_, scid_, cstart_, cend_, nb_ ? eoff_.p : nullptr,
+                                      nb_ ? elist_.p : nullptr, nbr_, cnt_, n_, nx, rcs_ * rcs_, L_, 1.0 / L_,
+                                      max_nbr_, status_);
+    }
     FMD_CUDA_LAUNCH();
     FMD_CUDA(cudaMemcpyAsync(ref_, pos_, n_ * sizeof(double4), cudaMemcpyDeviceToDevice, st_));
     ++rebuilds_;
@@ -943,20 +1000,19 @@ class PlainEngine final : public SimEngine {
 
   void forces(double cap) {
     FMD_CUDA(cudaMemsetAsync(virial_, 0, 6 * sizeof(double), st_));
-    k_lj<<<div_up(n_, kBlock), kBlock, 0, st_>>>(pos_, force_, virial_, lj_, nbr_, cnt_, n_, cfg_.ntypes,
-                                                 cfg_.rc * cfg_.rc, L_, 1.0 / L_, 1);
+    const int lanes = n_ * 8ll <= kLjThreads ? 8 : n_ * 4ll <= kLjThreads ? 4 : n_ * 2ll <= kLjThreads ? 2 : 1;
+    auto* const lj_kernel = lanes == 8 ? k_lj<8> : lanes == 4 ? k_lj<4> : lanes == 2 ? k_lj<2> : k_lj<1>;
+    lj_kernel<<<div_up((long long)div_up(n_, 32 / lanes) * 32, kBlock), kBlock, 0, st_>>>(
+        pos_, force_, virial_, lj_, nbr_, cnt_, n_, cfg_.ntypes, cfg_.rc * cfg_.rc, L_, 1.0 / L_, 1);
     FMD_CUDA_LAUNCH();
     if (cap > 0) {  // push-off caps the non-bonded force only
       k_cap<<<div_up(n_, kBlock), kBlock, 0, st_>>>(force_, n_, cap);
       FMD_CUDA_LAUNCH();
     }
-    if (nb_) {
-      k_fene<<<div_up(nb_, kBlock), kBlock, 0, st_>>>(pos_, force_, virial_, bonds_, btype_, fene_, nb_, L_,
-                                                      1.0 / L_, 1, status_);
-      FMD_CUDA_LAUNCH();
-    }
-    if (na_) {
-      k_angle<<<div_up(na_, kBlock), kBlock, 0, st_>>>(pos_, force_, virial_, angles_, angp_, na_, L_, 1.0 / L_);
+    const int gb = div_up(nb_, kBlock), ga = div_up(na_, kBlock);
+    if (gb + ga) {
+      k_bonded<<<gb + ga, kBlock, 0, st_>>>(pos_, force_, virial_, bonds_, btype_, fene_, nb_, gb, angles_, angp_, na_,
+                                            L_, 1.0 / L_, 1, status_);
       FMD_CUDA_LAUNCH();
     }
   }
@@ -1039,19 +1095,27 @@ class PlainEngine final : public SimEngine {
     }
     FMD_CUDA_LAUNCH();
     // Rebuild test on the host every step (skin_trigger.cuh:18-33, main.cu:484-528).
+    // The forces are queued on the list in use before the displacement is
+    // known, so the host's wait and the next launches pass while they run; a
+    // step that turns out to rebuild evaluates them again on its new list.
     ++since_;
-    unsigned long long bits = 0;
-    FMD_CUDA(cudaMemcpyAsync(&bits, maxdr2_, sizeof(bits), cudaMemcpyDeviceToHost, st_));
-    FMD_CUDA(cudaStreamSynchronize(st_));
-    double maxd2;
-    std::memcpy(&maxd2, &bits, sizeof(double));
-    const double hs = 0.5 * cfg_.skin;
-    if (maxd2 > hs * hs || since_ >= 20) {
-      FMD_CUDA(cudaMemsetAsync(maxdr2_, 0, sizeof(bits), st_));
+    bool rebuilds = since_ >= 20;
+    if (!rebuilds) {
+      FMD_CUDA(cudaMemcpyAsync(disp_.p, maxdr2_, sizeof(double), cudaMemcpyDeviceToHost, st_));
+      FMD_CUDA(cudaEventRecord(disp_ready_, st_));
+      forces(cap);
+      FMD_CUDA(cudaEventSynchronize(disp_ready_));
+      double maxd2;
+      std::memcpy(&maxd2, disp_.p, sizeof(double));
+      const double hs = 0.5 * cfg_.skin;
+      rebuilds = maxd2 > hs * hs;
+    }
+    if (rebuilds) {
+      FMD_CUDA(cudaMemsetAsync(maxdr2_, 0, sizeof(unsigned long long), st_));
       since_ = 0;
       rebuild();
+      forces(cap);
     }
-    forces(cap);
     if (ensemble == FMD_LANGEVIN) {
       k_kick<<<g, kBlock, 0, st_>>>(vel_, force_, pos_, params(), hdt);
     } else if (ensemble == FMD_NVT_NH) {
@@ -1088,7 +1152,7 @@ class PlainEngine final : public SimEngine {
   int64_t step_ = 0, rebuilds_ = 0;
   int32_t since_ = 0;
   cudaStream_t st_ = nullptr;
-  DevBuf<double4> pos_, vel_, force_, ref_;
+  DevBuf<double4> pos_, vel_, force_, ref_, spos_;
   DevBuf<int> image_;
   DevBuf<double> mass_;
   DevBuf<double2> lj_;
@@ -1101,6 +1165,8 @@ class PlainEngine final : public SimEngine {
   DevBuf<int> nbr_, cnt_, cid_, scid_, aid_, sorted_, cstart_, cend_;
   DevBuf<char> cub_tmp_;
   DevBuf<unsigned long long> maxdr2_;
+  PinBuf disp_;  // its host copy, and the event after the copy
+  cudaEvent_t disp_ready_ = nullptr;
   DevBuf<double> virial_, red_;
   DevBuf<int> status_;
   DevBuf<NHScalars> nh_;
