@@ -20,12 +20,12 @@
 namespace fmd {
 namespace mixed {
 
-// Chunks per resident block up to which k_steps takes a batch (one where a
-// replica has a Nose-Hoover chain).  Measured per 200 steps, graph against
-// resident: 200 x 1,000 beads (2 chunks per block) 21.9 / 19.0 ms, 64 uneven
-// replicas of 342,000 beads in all (4 per block) 40.4 / 38.3 ms; 16 x 30,000
-// NVT (5 per block) 42.4 / 52.2 ms.
-constexpr int kResidentChunks = 4;
+// Chunks per resident block up to which k_steps takes a batch, without and with
+// Nose-Hoover chains.  Measured per 200 steps, graph against resident: 200 x
+// 1,000 beads (2 chunks per block) 21.9 / 18.5 ms, 64 uneven replicas of
+// 342,000 beads in all (3) 40.4 / 27.1 ms, 64 x 30,000 (13) 100 / 131 ms --
+// the lines cross between 5 and 6; 16 x 30,000 NVT (4) 42.3 / 42.3 ms.
+constexpr int kResidentChunks = 5, kResidentChained = 3;
 constexpr int kResidentSteps = 1000;  // steps per k_steps launch
 constexpr int kReadPiece = 32768;     // atoms per piece of a state readout (2 MB)
 
@@ -725,7 +725,7 @@ int Batch::resident_lanes(F runs, int64_t* chunks) const {
   if (graph_steps_ <= 0 || groups == 0) return 0;
   const int lpa = *chunks <= steps_resident_blocks(4) ? 4 : 1;
   const int cap = steps_resident_blocks(lpa);
-  return groups <= cap && *chunks <= (int64_t)(chained ? 1 : kResidentChunks) * cap ? lpa : 0;
+  return groups <= cap && *chunks <= (int64_t)(chained ? kResidentChained : kResidentChunks) * cap ? lpa : 0;
 }
 
 // The replicas with steps left as groups of resident blocks (k_steps): the

@@ -969,8 +969,22 @@ constexpr int kNbrWarps = kNbrThreads / 32;
 constexpr int kNbrWin = 1024;     // staged candidates per window (a multiple of 64)
 constexpr int kNbrGroup = 64;     // home atoms per pass
 
+// Shared staging of one home cell's list.
+constexpr int kNbrExcl = 1 + kMaxBondsPerAtom;  // the atom itself and its bonded partners
 template <int WIN, int WARPS>
-__device__ __forceinline__ void neighbors_cell_ballot(const Dev& d, const Rep& R, int* status, int lc) {
+struct ListStage {
+  float4 c[WIN];                   // candidates of the window
+  float4 hp[kNbrGroup];            // home atoms' positions
+  int xk[kNbrGroup][kNbrExcl];     // and their excluded candidates (index, or -1)
+  uint32_t xm[WARPS][WIN / 32];    // per warp: excluded candidates of the window
+  int ns[27], off[28], cnt[kNbrGroup];
+  float sx[27], sy[27], sz[27];
+  uint32_t code[27];
+};
+
+template <int WIN, int WARPS>
+__device__ __forceinline__ void neighbors_cell_ballot(const Dev& d, const Rep& R, int* status, int lc,
+                                                      ListStage<WIN, WARPS>& st) {
   const int G = R.G;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (G < 3) return;  // boxes under three cells per axis: k_neighbors_small
@@ -983,14 +997,16 @@ __device__ __forceinline__ void neighbors_cell_ballot(const Dev& d, const Rep& R
   const float rcs = (float)(R.rc + R.skin);
   const float rcs2 = rcs * rcs;
 
-  __shared__ float4 s_c[WIN];
-  __shared__ int s_ns[27], s_off[28], s_cnt[kNbrGroup];
-  __shared__ float s_sx[27], s_sy[27], s_sz[27];
-  __shared__ uint32_t s_code[27];
-  constexpr int kExcl = 1 + kMaxBondsPerAtom;  // the atom itself and its bonded partners
-  __shared__ float4 s_hp[kNbrGroup];            // home atoms' positions
-  __shared__ int s_xk[kNbrGroup][kExcl];        // and their excluded candidates (index, or -1)
-  __shared__ uint32_t s_xm[WARPS][WIN / 32];  // per warp: excluded candidates of the window
+  auto &s_c = st.c;
+  auto& s_ns = st.ns;
+  auto& s_off = st.off;
+  auto& s_cnt = st.cnt;
+  auto &s_sx = st.sx, &s_sy = st.sy, &s_sz = st.sz;
+  auto &s_code = st.code;
+  auto &s_hp = st.hp;
+  auto &s_xk = st.xk;
+  auto &s_xm = st.xm;
+  constexpr int kExcl = kNbrExcl;
   for (int k = threadIdx.x; k < WARPS * (WIN / 32); k += blockDim.x) (&s_xm[0][0])[k] = 0u;
   const int hx = lc % G, hy = (lc / G) % G, hz = lc / (G * G);
   if (warp == 0) {
@@ -1288,8 +1304,9 @@ __global__ void __launch_bounds__(kNbrThreads, MINB) k_neighbors(Dev d) {
     cur.seek(item);
     __syncthreads();  // the previous item's shared staging is no longer read
     if (V == 0) {
+      __shared__ ListStage<kNbrWin, kNbrWarps> st;
       Rep& R = d.reps[rb_rep(d, cur.i)];
-      neighbors_cell_ballot<kNbrWin, kNbrWarps>(d, R, &R.status, item - cur.lo);
+      neighbors_cell_ballot(d, R, &R.status, item - cur.lo, st);
     } else
       neighbors_row(d, d.reps[rb_rep(d, cur.i)], item - cur.lo);
   }
@@ -1872,25 +1889,35 @@ __device__ __forceinline__ void bonded_terms(const Dev& d, const Rep& R, int s, 
 // PF: 0 = list words loaded with the batch, 1 = the next batch's words
 // loaded ahead into registers, D >= 2 = the ring of D batches (per-chunk
 // kernel; the work-list kernel then loads ahead into registers).
+// A force block's shared tables: the shift vectors of all entries (SH = 0) or
+// the per-axis values, and the replica's pair parameters.
+template <int SH>
+struct ForceTables {
+  float4 shift[SH == 0 ? kShiftCodes : 1];
+  float axis[5];
+  float eps24[kMaxTypes * kMaxTypes], sig2[kMaxTypes * kMaxTypes];
+};
+
 // R: the replica's record, or a block's copy of it; ci the chunk's entry.
+// The tables are filled here, the pair parameters (s_eps24, s_sig2) where they
+// are not those of R itself.
 template <bool EV, int B, int PF, int KB, bool LISTED, int SH, bool P2>
-__device__ __forceinline__ void force_chunk_of(const Dev& d, const Rep& R, const int4 ci, int chunk) {
+__device__ __forceinline__ void force_chunk_of(const Dev& d, const Rep& R, const int4 ci, int chunk, float4* s_shift,
+                                               float* s_axis, float* s_eps24, float* s_sig2) {
   constexpr bool RING = PF >= 2 && !LISTED;
   constexpr bool PFR = PF != 0;  // register look-ahead in the loops below
   static_assert(!RING || B == 4, "the ring stages batches of 4 rows");
   constexpr bool ev = EV;
   const int r = ci.x;
-  __shared__ float4 s_shift[SH == 0 ? kShiftCodes : 1];
-  __shared__ float s_axis[5];
-  __shared__ float s_eps24[kMaxTypes * kMaxTypes], s_sig2[kMaxTypes * kMaxTypes];
   const int nt = R.ntypes;
   const int G = R.G;
   const float h = R.h, inv_h = 1.0f / h;
   const float dL = (float)(R.L - (double)G * (double)h);
-  for (int k = threadIdx.x; k < nt * nt; k += blockDim.x) {
-    s_eps24[k] = R.lj_eps24[k];
-    s_sig2[k] = R.lj_sig2[k];
-  }
+  if (s_eps24 != R.lj_eps24)
+    for (int k = threadIdx.x; k < nt * nt; k += blockDim.x) {
+      s_eps24[k] = R.lj_eps24[k];
+      s_sig2[k] = R.lj_sig2[k];
+    }
   if (SH == 0 && threadIdx.x < kShiftCodes) {
     const int c = threadIdx.x;
     const int ax = c / 25, ay = (c / 5) % 5, az = c % 5;
@@ -1998,7 +2025,8 @@ __device__ __forceinline__ void force_chunk(const Dev& d, int chunk, bool skip_r
   if (!R.adv) return;
   if (need_ev(R) != EV) return;
   if (skip_rebuilt && R.rebuild_now) return;
-  force_chunk_of<EV, B, PF, KB, LISTED, SH, P2>(d, R, ci, chunk);
+  __shared__ ForceTables<SH> tb;
+  force_chunk_of<EV, B, PF, KB, LISTED, SH, P2>(d, R, ci, chunk, tb.shift, tb.axis, tb.eps24, tb.sig2);
 }
 
 // The list filter alone: the entries of the atom's rc + skin list (nn
@@ -2314,9 +2342,8 @@ __device__ __forceinline__ int filter_quads(const uint32_t* lst, int nn, uint32_
 // Forces without energies of one chunk by a block of 4 kChunk threads, four
 // lanes per atom; LISTED: the replica's pruned list is due (or it keeps none).
 template <int KB, bool LISTED>
-__device__ __forceinline__ void force_chunk_quads(const Dev& d, const Rep& R, int r, int c) {
-  __shared__ float s_axis[5];
-  __shared__ float s_eps24[kMaxTypes * kMaxTypes], s_sig2[kMaxTypes * kMaxTypes];
+__device__ __forceinline__ void force_chunk_quads(const Dev& d, const Rep& R, int r, int c, float* s_axis) {
+  const float *const s_eps24 = R.lj_eps24, *const s_sig2 = R.lj_sig2;  // R is the block's shared copy
   const int lane = threadIdx.x & 31, q = lane >> 3, src = lane & 7;
   const int nt = R.ntypes;
   const int G = R.G;
@@ -2332,10 +2359,6 @@ __device__ __forceinline__ void force_chunk_quads(const Dev& d, const Rep& R, in
   int nn = valid ? (pruned ? d.pcnt[s] : d.ncnt[s]) : 0;
   const uint32_t bw = valid ? d.bnd[(size_t)s * kMaxBondsPerAtom + q] : 0u;
   const uint2 aw = valid ? d.ang[(size_t)s * kMaxAnglesPerAtom + q] : make_uint2(0u, 0u);
-  for (int k = threadIdx.x; k < nt * nt; k += blockDim.x) {
-    s_eps24[k] = R.lj_eps24[k];
-    s_sig2[k] = R.lj_sig2[k];
-  }
   if (threadIdx.x < 5)
     s_axis[threadIdx.x] = shift_term(axis_code_e(threadIdx.x), axis_code_k(threadIdx.x), h, dL);
   __syncthreads();
@@ -2488,8 +2511,7 @@ void launch_prune(const Dev& d, cudaStream_t st);
 // kernel for replicas with tables only; explicit roundings keep the energy
 // flavour's forces identical to the plain one's.
 template <bool EV>
-__device__ __forceinline__ void table_chunk(const Dev& d, const Rep& R, const int4 ci, int chunk) {
-  __shared__ float4 s_shift[kShiftCodes];
+__device__ __forceinline__ void table_chunk(const Dev& d, const Rep& R, const int4 ci, int chunk, float4* s_shift) {
   const int G = R.G;
   const float h = R.h;
   const float dL = (float)(R.L - (double)G * (double)h);
@@ -2609,7 +2631,8 @@ __global__ void __launch_bounds__(kChunk) k_table(Dev d, int sel) {
   const Rep& R = d.reps[ci.x];
   if (!R.adv || R.ntables == 0 || need_ev(R) != EV) return;
   if ((sel == 1 && R.rebuild_now) || (sel == 2 && !R.rebuild_now)) return;
-  table_chunk<EV>(d, R, ci, blockIdx.x);
+  __shared__ float4 s_shift[kShiftCodes];
+  table_chunk<EV>(d, R, ci, blockIdx.x, s_shift);
 }
 
 void launch_table(const Dev& d, int nchunks, bool ev, int sel, cudaStream_t st) {
@@ -2620,30 +2643,26 @@ void launch_table(const Dev& d, int nchunks, bool ev, int sel, cudaStream_t st) 
 }
 
 // ---------------------------------------------------------------- post-force
-// The final half kick (kick == 1) and the KE-tensor partials of one chunk,
-// on its loaded velocity and force.
-__device__ __forceinline__ void post_chunk(const Dev& d, const Rep& R, int chunk, int s, bool have, float4 v,
-                                           const float4 f, int kick) {
-  double vals[7] = {0, 0, 0, 0, 0, 0, 0};
-  if (have) {
-    if (kick == 1) {
-      const double dt = (R.mode == kModePushoff) ? R.push_dt : R.dt;
-      const float hm = (float)(0.5 * dt) * v.w;
-      v.x = fmaf(hm, f.x, v.x);
-      v.y = fmaf(hm, f.y, v.y);
-      v.z = fmaf(hm, f.z, v.z);
-      d.vel[s] = v;
-    }
-    const double m = 1.0 / (double)v.w;
-    const double vx = v.x, vy = v.y, vz = v.z;
-    vals[0] = m * vx * vx;
-    vals[1] = m * vx * vy;
-    vals[2] = m * vx * vz;
-    vals[3] = m * vy * vy;
-    vals[4] = m * vy * vz;
-    vals[5] = m * vz * vz;
+// The final half kick (kick == 1) of the atom in slot s on its loaded
+// velocity and force, and its KE tensor.
+__device__ __forceinline__ void post_atom(const Dev& d, const Rep& R, int s, float4 v, const float4 f, int kick,
+                                          double* vals) {
+  if (kick == 1) {
+    const double dt = (R.mode == kModePushoff) ? R.push_dt : R.dt;
+    const float hm = (float)(0.5 * dt) * v.w;
+    v.x = fmaf(hm, f.x, v.x);
+    v.y = fmaf(hm, f.y, v.y);
+    v.z = fmaf(hm, f.z, v.z);
+    d.vel[s] = v;
   }
-  block_partials<kChunk>(vals, 6, d.part + 7 * d.part_stride + chunk, d.part_stride);
+  const double m = 1.0 / (double)v.w;
+  const double vx = v.x, vy = v.y, vz = v.z;
+  vals[0] = m * vx * vx;
+  vals[1] = m * vx * vy;
+  vals[2] = m * vx * vz;
+  vals[3] = m * vy * vy;
+  vals[4] = m * vy * vz;
+  vals[5] = m * vz * vz;
 }
 
 __global__ void __launch_bounds__(kChunk, 7) k_post(Dev d, int kick) {
@@ -2660,7 +2679,9 @@ __global__ void __launch_bounds__(kChunk, 7) k_post(Dev d, int kick) {
   }
   const Rep& R = d.reps[ci.x];
   if (!R.adv || (kick == 1 && R.defer)) return;
-  post_chunk(d, R, chunk, s, have, v, f, kick);
+  double vals[7] = {0, 0, 0, 0, 0, 0, 0};
+  if (have) post_atom(d, R, s, v, f, kick, vals);
+  block_partials<kChunk>(vals, 6, d.part + 7 * d.part_stride + chunk, d.part_stride);
 }
 
 // One pressure-tensor sample into a replica's multiple-tau correlator, by
@@ -2725,6 +2746,9 @@ __device__ __forceinline__ void acf_sample(const Dev& d, const Rep& R, int r) {
 // The post-force commit on a replica's record R (one thread): energies,
 // virial and KE of the step from the replica's reduced partials acc, the
 // post-force chain or barostat, and the scalars of the next pre-force.
+// IN_PLACE: R is in shared memory; the chain is updated and the next scalars
+// are built where they stand.
+template <bool IN_PLACE>
 __device__ __forceinline__ void post_commit_state(Rep& R, const double* acc, int kick) {
   if (need_ev(R)) {
     R.pe = acc[0];
@@ -2736,10 +2760,12 @@ __device__ __forceinline__ void post_commit_state(Rep& R, const double* acc, int
   const int ens = (R.mode == kModePushoff) ? FMD_LANGEVIN : R.ensemble;
   if (need_ev(R)) R.ev_step = R.step;
   R.force_ev = 0;
-  // the chain / barostat state is updated in a local copy and stored
-  // once: in place, its arrays' stores would order every later read of
-  // the record behind them
-  NHScalars nh = R.nh;
+  // In global memory the chain / barostat state is updated in a local copy
+  // and stored once: in place, its arrays' stores would order every later
+  // read of the record behind them.
+  NHScalars local;
+  if (!IN_PLACE) local = R.nh;
+  NHScalars& nh = IN_PLACE ? R.nh : local;
   if (kick == 2) {
     // re-evaluation of the current state: reductions only
   } else if (!kick) {
@@ -2764,12 +2790,13 @@ __device__ __forceinline__ void post_commit_state(Rep& R, const double* acc, int
   } else {
     R.pending_scale = 1.0;
   }
-  R.nh = nh;
+  if (!IN_PLACE) R.nh = local;
   R.thermo_step = R.step;
   R.adv = 0;
   R.rebuild_now = 0;
   // scalars of the next pre-force, computed once here for all its blocks
-  next_scalars(R);
+  if (IN_PLACE) step_scalars<false>(R, R.next);
+  else next_scalars(R);
   R.next_valid = 1;
 }
 
@@ -2809,7 +2836,7 @@ __global__ void __launch_bounds__(kPostCommitThreads) k_post_commit(Dev d, int k
         for (int w = 1; w < nw; ++w) t += s_red[w][q];
         acc[q] = t;
       }
-      post_commit_state(R, acc, kick);
+      post_commit_state<false>(R, acc, kick);
     }
     // Stress steps: the thermo row's pressure tensor, (KE tensor (with the
     // pending thermostat scale) + virial) / V in the current box, feeds the
@@ -2843,12 +2870,26 @@ __global__ void __launch_bounds__(kPostCommitThreads) k_post_commit(Dev d, int k
 //
 // LPA lanes per atom (blocks of LPA * kChunk threads): 4 for batches whose
 // every chunk has a resident block of that width, 1 beyond.
-constexpr int kStepWin = 704;       // list candidates staged per window: one 27-cell stencil of a melt
+constexpr int kStepWin = 704;       // list candidates staged per window
 constexpr int kStepSpin = 1 << 22;  // polls of a group barrier before the replica is given up (seconds)
 constexpr int step_threads(int lpa) { return lpa * kChunk; }
-// 6 blocks of 128 threads (80 registers: the energy flavour and the list
-// build do not spill), 2 blocks of 512 (64 registers)
-constexpr int step_blocks_per_sm(int lpa) { return lpa == 1 ? 6 : 2; }
+// 8 blocks of 128 threads or 2 of 512: 64 registers
+constexpr int step_blocks_per_sm(int lpa) { return lpa == 1 ? 8 : 2; }
+constexpr int kStepKicks = 4;  // chunks whose post-force partials are staged at a time
+
+// A resident block's shared memory besides the record: the stages of a step
+// use it in turn (small, so that the L1 keeps the rest of the array for the
+// position gathers).
+template <int LPA>
+union StepStage {
+  ListStage<kStepWin, step_threads(LPA) / 32> list;
+  struct {
+    float4 shift[kShiftCodes];
+    float axis[5];
+  } force;
+  double kick[kStepKicks][kChunk / 32][6];
+  double red[kPostCommitThreads / 32][13];
+};
 
 // Relaxed polls (an acquire per poll would drop the SM's L1 lines each time);
 // a fence follows the last.
@@ -2962,7 +3003,7 @@ __device__ __forceinline__ void scan_cells_block(const Dev& d, const Rep& R) {
 // The rebuild of a group's replica: the phases of launch_rebuild with a group
 // barrier in the place of each kernel boundary.
 template <int LPA>
-__device__ __noinline__ bool rebuild_group(const Dev& d, Rep& R, StepGroup& g) {
+__device__ __noinline__ bool rebuild_group(const Dev& d, Rep& R, StepGroup& g, StepStage<LPA>& st) {
   constexpr int T = step_threads(LPA), W = T / 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int t = threadIdx.x % kChunk, cf = g.c0 + threadIdx.x / kChunk;  // LPA chunks at a time
@@ -2990,7 +3031,7 @@ __device__ __noinline__ bool rebuild_group(const Dev& d, Rep& R, StepGroup& g) {
   for (int lc = g.rank; lc < home; lc += g.nb) {
     if (R.G >= 3) {
       __syncthreads();  // the previous cell's staging is no longer read
-      neighbors_cell_ballot<kStepWin, W>(d, R, status, lc);
+      neighbors_cell_ballot(d, R, status, lc, st.list);
     } else {
       const int ov = neighbors_small_box(d, R, lc, lane, 32 * warp, T);
       if (ov) atomicOr(status, ov);
@@ -3000,25 +3041,62 @@ __device__ __noinline__ bool rebuild_group(const Dev& d, Rep& R, StepGroup& g) {
 }
 
 template <bool EV, int KB, int LPA>
-__device__ __forceinline__ void forces_group(const Dev& d, const Rep& R, const StepGroup& g) {
+__device__ __forceinline__ void forces_group(const Dev& d, Rep& R, const StepGroup& g, StepStage<LPA>& st) {
   for (int c = g.c0; c < g.c1; ++c) {
     const int4 ci = make_int4(g.r, R.slot_base + c * kChunk, 0, c);
     const int chunk = R.chunk_base + c;
     if (!EV && LPA == 4) {
       if (R.rebuild_now)
-        force_chunk_quads<KB, true>(d, R, g.r, c);
+        force_chunk_quads<KB, true>(d, R, g.r, c, st.force.axis);
       else
-        force_chunk_quads<KB, false>(d, R, g.r, c);
+        force_chunk_quads<KB, false>(d, R, g.r, c, st.force.axis);
     } else if (R.rebuild_now) {
-      force_chunk_of<EV, 4, true, KB, true, 1, true>(d, R, ci, chunk);
+      force_chunk_of<EV, 4, true, KB, true, 1, true>(d, R, ci, chunk, nullptr, st.force.axis, R.lj_eps24, R.lj_sig2);
     } else {
-      force_chunk_of<EV, 4, true, KB, false, 1, true>(d, R, ci, chunk);
+      force_chunk_of<EV, 4, true, KB, false, 1, true>(d, R, ci, chunk, nullptr, st.force.axis, R.lj_eps24, R.lj_sig2);
     }
     __syncthreads();  // the tables and the block partials' staging are free again
     if (R.ntables) {
-      table_chunk<EV>(d, R, ci, chunk);
+      table_chunk<EV>(d, R, ci, chunk, st.force.shift);
       __syncthreads();
     }
+  }
+}
+
+// The energy flavour and the chain commit out of line: their registers stay
+// out of the plain step's loops.
+template <int KB, int LPA>
+__device__ __noinline__ void forces_group_ev(const Dev& d, Rep& R, const StepGroup& g, StepStage<LPA>& st) {
+  forces_group<true, KB, LPA>(d, R, g, st);
+}
+__device__ __noinline__ void post_commit_shared(Rep& R, const double* acc) { post_commit_state<true>(R, acc, 1); }
+
+// The post-force half kick and KE partials of the group's chunks, LPA chunks
+// side by side and kStepKicks of their partials staged at a time: per chunk
+// the warps' sums in warp order, as block_partials adds them.
+template <int LPA>
+__device__ __forceinline__ void kicks_group(const Dev& d, const Rep& R, const StepGroup& g, StepStage<LPA>& st) {
+  const int lane = threadIdx.x & 31, warp = (threadIdx.x % kChunk) >> 5;
+  for (int c0 = g.c0; c0 < g.c1; c0 += kStepKicks) {
+    const int c1 = min(c0 + kStepKicks, g.c1);
+#pragma unroll 1
+    for (int c = c0 + threadIdx.x / kChunk; c < c1; c += LPA) {
+      const int local = c * kChunk + threadIdx.x % kChunk, s = R.slot_base + local;
+      double vals[6] = {0, 0, 0, 0, 0, 0};
+      if (local < R.natoms) post_atom(d, R, s, d.vel[s], d.force[s], 1, vals);
+#pragma unroll
+      for (int q = 0; q < 6; ++q) vals[q] = warp_sum(vals[q]);
+      if (lane == 0)
+        for (int q = 0; q < 6; ++q) st.kick[c - c0][warp][q] = vals[q];
+    }
+    __syncthreads();
+    if (threadIdx.x < (c1 - c0) * 6) {
+      const int c = threadIdx.x / 6, q = threadIdx.x % 6;
+      double t = 0.0;
+      for (int w = 0; w < kChunk / 32; ++w) t += st.kick[c][w][q];
+      d.part[(7 + q) * d.part_stride + R.chunk_base + c0 + c] = t;
+    }
+    __syncthreads();
   }
 }
 
@@ -3065,7 +3143,8 @@ __global__ void __launch_bounds__(step_threads(LPA), step_blocks_per_sm(LPA))
   __shared__ __align__(16) Rep R;
   __shared__ int dead;
   __shared__ uint32_t s_max[T / 32];
-  __shared__ double s_red[kPostCommitThreads / 32][13], s_acc[13];
+  __shared__ StepStage<LPA> st;
+  __shared__ double s_acc[13];
   const int4 pl = plan[blockIdx.x];
   StepGroup g;
   g.r = pl.x;
@@ -3125,28 +3204,22 @@ __global__ void __launch_bounds__(step_threads(LPA), step_blocks_per_sm(LPA))
       R.defer = post_needed(R) ? 0 : 1;
     }
     __syncthreads();
-    if (R.rebuild_now == kListRebuild && !rebuild_group<LPA>(d, R, g)) break;
+    if (R.rebuild_now == kListRebuild && !rebuild_group<LPA>(d, R, g, st)) break;
     const bool defer = R.defer != 0;
     if (need_ev(R))
-      forces_group<true, KB, LPA>(d, R, g);
+      forces_group_ev<KB, LPA>(d, R, g, st);
     else
-      forces_group<false, KB, LPA>(d, R, g);
+      forces_group<false, KB, LPA>(d, R, g, st);
     if (defer) {
       if (threadIdx.x == 0) {
         step_scalars<false>(R, R.next);
         R.next_valid = 1;
       }
     } else {
-      for (int c = g.c0; c < g.c1; ++c) {
-        const int local = c * kChunk + threadIdx.x, s = R.slot_base + local;
-        const bool have = threadIdx.x < kChunk && local < R.natoms;
-        const float4 v = have ? d.vel[s] : make_float4(0, 0, 0, 1), f = have ? d.force[s] : make_float4(0, 0, 0, 0);
-        post_chunk(d, R, R.chunk_base + c, s, have, v, f, 1);
-        __syncthreads();  // the block partials' staging is free again
-      }
+      kicks_group<LPA>(d, R, g, st);
       if (!group_sync(g)) break;
-      reduce_partials<T>(d, R, need_ev(R) ? 0 : 7, s_red, s_acc);
-      if (threadIdx.x == 0) post_commit_state(R, s_acc, 1);
+      reduce_partials<T>(d, R, need_ev(R) ? 0 : 7, st.red, s_acc);
+      if (threadIdx.x == 0) post_commit_shared(R, s_acc);
       __syncthreads();
       if (g.rank == 0 && warp == 0 && stress_step(R)) acf_sample(d, R, g.r);
     }
@@ -3284,7 +3357,8 @@ __global__ void __launch_bounds__(kNbrThreads) k_neighbors_g(Dev d) {
   if (R.rebuild_now != 1) return;
   const int G = R.G;
   if ((int)blockIdx.x >= G * G * G) return;
-  neighbors_cell_ballot<kNbrWin, kNbrWarps>(d, R, &R.status, blockIdx.x);
+  __shared__ ListStage<kNbrWin, kNbrWarps> st;
+  neighbors_cell_ballot(d, R, &R.status, blockIdx.x, st);
 }
 
 // ---------------------------------------------------------------- launchers
@@ -3308,7 +3382,36 @@ int resident_grid(K kernel, int threads) {
 }
 }  // namespace
 
+constexpr int kForceCarveoutPct = 16;  // percent of the SM's shared-memory maximum
+
+// The force kernels use 4 KB of shared memory per block: ask for the
+// smallest shared-memory carve-out, leaving the rest of the SM's unified
+// L1 / shared array to cache the neighbor-position gathers.
+template <typename K>
+void prefer_l1(K kernel, int pct = kForceCarveoutPct) {
+  FMD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct));
+}
+
+// The carve-out that holds a resident block's shared memory as often as the
+// block fits an SM; the rest of the array is L1 for the position gathers (the
+// driver's own choice left it 28 KB).
+template <typename K>
+void steps_carveout(K kernel, int blocks_per_sm) {
+  cudaFuncAttributes a;
+  FMD_CUDA(cudaFuncGetAttributes(&a, kernel));
+  const int kb = (int)((a.sharedSizeBytes + 1023) / 1024 + 1) * blocks_per_sm;
+  prefer_l1(kernel, std::min(100, (100 * kb + 227) / 228));
+}
+
 int steps_resident_blocks(int lpa) {
+  static const bool carved = [] {
+    steps_carveout(k_steps<1, 1>, step_blocks_per_sm(1));
+    steps_carveout(k_steps<2, 1>, step_blocks_per_sm(1));
+    steps_carveout(k_steps<1, 4>, step_blocks_per_sm(4));
+    steps_carveout(k_steps<2, 4>, step_blocks_per_sm(4));
+    return true;
+  }();
+  (void)carved;
   static const int n1 = std::min(resident_grid(k_steps<1, 1>, step_threads(1)), resident_grid(k_steps<2, 1>, step_threads(1)));
   static const int n4 = std::min(resident_grid(k_steps<1, 4>, step_threads(4)), resident_grid(k_steps<2, 4>, step_threads(4)));
   return lpa == 4 ? n4 : n1;
@@ -3560,7 +3663,6 @@ void launch_rebuild(const Dev& d, int nreps, int nbr_variant, cudaStream_t st, b
 // The energy flavour of a variant walks the list in the same batches with
 // the same compensated adds, so its forces are bit-identical: energy steps
 // and host re-evaluations do not perturb a trajectory.
-constexpr int kForceCarveoutPct = 16;  // percent of the SM's shared-memory maximum
 
 // The variant's two kernels: one block per chunk, and the work-list form.
 // Parameters: list entries per batch, blocks per SM, next batch's list words
@@ -3591,14 +3693,6 @@ void force_kernels(int variant, void (**per_chunk)(Dev, int), void (**listed)(De
     default: FMD_FORCE_VARIANT(4, 8, true, 1, 0, false, 1) break;
   }
 #undef FMD_FORCE_VARIANT
-}
-
-// The force kernels use 4 KB of shared memory per block: ask for the
-// smallest shared-memory carve-out, leaving the rest of the SM's unified
-// L1 / shared array to cache the neighbor-position gathers.
-template <typename K>
-void prefer_l1(K kernel, int pct = kForceCarveoutPct) {
-  FMD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct));
 }
 
 // The ring variants hold 4-8 KB of list rows per block besides the 2 KB of

@@ -14,13 +14,14 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <cstdint>
 
 namespace fmd {
 namespace cells {
 
 constexpr int kThreads = 128, kWarps = kThreads / 32;
-constexpr int kWin = 512;   // candidates staged per window (a multiple of 32)
+constexpr int kWin = 768;   // candidates staged per window (a multiple of 32): one 27-cell stencil of a dense melt
 constexpr int kGroup = 64;  // home atoms per pass
 
 // Cells hold four atoms or more on average, and the 27 cells are distinct.
@@ -59,6 +60,9 @@ template <bool NEAR, typename V4, typename Real>
 __device__ __forceinline__ int test_window(const V4* s_c, int wn, V4 pi, int i, int excluded, int ne, Real rcs2,
                                            Real L, Real inv_L, int* nbr, int64_t n, int max_nbr, int count, int lane) {
   const uint32_t below = (1u << lane) - 1u;
+  // room for every lane of every batch: no test per hit
+  const bool roomy = count + ((wn + 31) & ~31) <= max_nbr;
+  int* const out = nbr + i;
 #pragma unroll 2
   for (int c0 = 0; c0 < wn; c0 += 32) {
     const V4 c = s_c[c0 + lane];
@@ -70,14 +74,14 @@ __device__ __forceinline__ int test_window(const V4* s_c, int wn, V4 pi, int i, 
     }
     const Real r2 = dx * dx + dy * dy + dz * dz;
     const int j = to_index(c.w);
-    bool hit = r2 < rcs2 && j != i && c0 + lane < wn;
+    bool hit = r2 < rcs2 && j != i;  // the window's padding is NaN: never
     for (int e = 0; e < ne; ++e) {  // every lane takes part in the shuffles
       const int out = __shfl_sync(0xFFFFFFFFu, excluded, e);
       hit &= out != j;
     }
     const uint32_t m = __ballot_sync(0xFFFFFFFFu, hit);
     const int at = count + __popc(m & below);
-    if (hit && at < max_nbr) nbr[at * n + i] = j;
+    if (hit && (roomy || at < max_nbr)) out[at * n] = j;
     count += __popc(m);
   }
   return count;
@@ -135,6 +139,13 @@ __global__ void __launch_bounds__(kThreads) k_list_cells(const V4* spos, const i
           near = near && near_home(p);
           s_c[k - w0] = p;
         }
+      }
+      const int padded = (wn + 31) & ~31;
+      if (wn + (int)threadIdx.x < padded) {
+        V4 none;
+        none.x = none.y = none.z = (Real)NAN;
+        none.w = from_index(-1, Real());
+        s_c[wn + threadIdx.x] = none;
       }
       near = __syncthreads_and(near);
       for (int a = warp; a < gn; a += kWarps) {
