@@ -709,58 +709,70 @@ void Batch::check_status(int r, bool throw_on_fault) {
   throw Error(FMD_ERR_FAULT, "replica fault");
 }
 
-// Lanes per atom with which k_steps takes the replicas for which runs(r)
-// holds, 0 where the graph's grids are the better form; their chunks in all.
+// How k_steps takes the replicas for which runs(r) holds, if it does: with a
+// block per tile where all fit the GPU at once, else with the fewest chunks
+// per block for which every group does; beyond kResidentChunks of them the
+// graph's grids are the better form.
 template <typename F>
-int Batch::resident_lanes(F runs, int64_t* chunks) const {
-  int groups = 0;
+Batch::Resident Batch::resident_form(F runs) const {
+  Resident f;
+  int groups = 0, atoms = 0, most = 0;
+  int64_t tiles = 0, chunks = 0;
   bool chained = false;  // a Nose-Hoover chain: a second barrier and a reduction every step
-  *chunks = 0;
   for (int r = 0; r < max_reps_; ++r) {
     if (!runs(r)) continue;
-    *chunks += h_reps_[r].nchunks;
-    chained |= h_reps_[r].mode == kModeRun && h_reps_[r].ensemble != FMD_LANGEVIN;
+    const Rep& R = h_reps_[r];
     ++groups;
+    tiles += step_tiles(R.natoms, R.nchunks);
+    chunks += R.nchunks;
+    atoms = std::max(atoms, R.natoms);
+    most = std::max(most, R.nchunks);
+    chained |= R.mode == kModeRun && R.ensemble != FMD_LANGEVIN;
   }
-  if (graph_steps_ <= 0 || groups == 0) return 0;
-  const int lpa = *chunks <= steps_resident_blocks(4) ? 4 : 1;
-  const int cap = steps_resident_blocks(lpa);
-  return groups <= cap && *chunks <= (int64_t)(chained ? kResidentChained : kResidentChunks) * cap ? lpa : 0;
+  if (graph_steps_ <= 0 || groups == 0) return f;
+  if (tiles <= steps_resident_blocks(true, 0)) {
+    f.fits = f.quads = true;
+    return f;
+  }
+  const int64_t stage = ((int64_t)atoms * 16 + 1023) / 1024 * 1024;
+  f.stage = stage <= kStepStageBytes ? (int)stage : 0;
+  const int cap = steps_resident_blocks(false, f.stage);
+  if (groups > cap || chunks > (int64_t)(chained ? kResidentChained : kResidentChunks) * cap) return f;
+  for (f.per_block = (int)((chunks + cap - 1) / cap); f.per_block < most; ++f.per_block) {
+    int64_t blocks = 0;
+    for (int r = 0; r < max_reps_; ++r)
+      if (runs(r)) blocks += (h_reps_[r].nchunks + f.per_block - 1) / f.per_block;
+    if (blocks <= cap) break;
+  }
+  f.fits = true;
+  return f;
 }
 
-// The replicas with steps left as groups of resident blocks (k_steps): the
-// fewest chunks per block for which every group fits the GPU at once.  False
-// where the step graph is used instead.
+// The replicas with steps left as groups of resident blocks; false where the
+// step graph is used instead.
 bool Batch::plan_resident() {
   if (!steps_variant(force_variant_)) return false;
   auto runs = [&](int r) { return info_[r].used && h_reps_[r].active && h_reps_[r].step < h_reps_[r].stop_step; };
-  int64_t chunks = 0;
-  const int lpa = resident_lanes(runs, &chunks);
-  if (!lpa) return false;
-  const int cap = steps_resident_blocks(lpa);
-  int most = 0;
-  for (int r = 0; r < max_reps_; ++r)
-    if (runs(r)) most = std::max(most, h_reps_[r].nchunks);
-  int per = (int)((chunks + cap - 1) / cap);
-  for (; per < most; ++per) {
-    int64_t blocks = 0;
-    for (int r = 0; r < max_reps_; ++r)
-      if (runs(r)) blocks += (h_reps_[r].nchunks + per - 1) / per;
-    if (blocks <= cap) break;
-  }
+  resident_ = resident_form(runs);
+  if (!resident_.fits) return false;
   new_plan_.clear();
   for (int r = 0; r < max_reps_; ++r) {
     if (!runs(r)) continue;
-    const int nb = (h_reps_[r].nchunks + per - 1) / per, first = (int)new_plan_.size();
+    const Rep& R = h_reps_[r];
+    const int nb = resident_.quads ? step_tiles(R.natoms, R.nchunks)
+                                   : (R.nchunks + resident_.per_block - 1) / resident_.per_block;
+    const int first = (int)new_plan_.size();
     for (int b = 0; b < nb; ++b) new_plan_.push_back(make_int4(r, b, nb, first));
   }
-  const size_t room = std::max(steps_resident_blocks(1), steps_resident_blocks(4));
-  if (plan_.n < room) {
+  if (plan_.n < new_plan_.size()) {
+    const size_t room = std::max({(int)new_plan_.size(), steps_resident_blocks(true, 0), steps_resident_blocks(false, 0)});
+    FMD_CUDA(cudaStreamSynchronize(st_));
     plan_.alloc(room);
     flags_.alloc(2 * room);
+    tiles_.alloc(6 * room);
+    count_.alloc((size_t)max_reps_ * kStepCountWords);
     h_plan_.clear();
   }
-  lpa_ = lpa;
   const bool same = new_plan_.size() == h_plan_.size() &&
                     std::memcmp(new_plan_.data(), h_plan_.data(), h_plan_.size() * sizeof(int4)) == 0;
   if (!same) {
@@ -778,7 +790,8 @@ void Batch::advance(int64_t nsteps) {
   if (plan_resident()) {
     while (nsteps > 0) {
       const int k = (int)std::min<int64_t>(nsteps, kResidentSteps);
-      launch_steps(d, plan_, (int)h_plan_.size(), lpa_, flags_, seq_, force_variant_, k, st_);
+      launch_steps(d, plan_, (int)h_plan_.size(), resident_.quads, resident_.stage, StepSync{flags_, count_, tiles_},
+                   max_reps_, seq_, force_variant_, k, st_);
       seq_ += (unsigned)k * kStepBarriers;
       nsteps -= k;
     }
@@ -991,8 +1004,7 @@ int Batch::autotune(int iters, double* ms_out, int cap) {
   int best = 0;
   double best_ms = 0;
   // a batch that k_steps takes keeps to the variants built in that form
-  int64_t chunks = 0;
-  const bool resident = resident_lanes([&](int r) { return info_[r].used && h_reps_[r].active; }, &chunks) != 0;
+  const bool resident = resident_form([&](int r) { return info_[r].used && h_reps_[r].active; }).fits;
   for (int v = 0; v < kForceVariants; ++v) {
     const double ms = time_force(iters, v, true);
     if (ms_out && v < cap) ms_out[v] = ms;

@@ -135,8 +135,14 @@ class Batch {
   void upload_atoms(int r, const double* xyz, const double* vel, const int32_t* image);
   void setup(const std::vector<int>& rs);
   void advance(int64_t nsteps);
+  // The form in which k_steps takes a set of replicas: whether at all, a block
+  // per tile (quads) or per so many chunks, shared bytes for the positions.
+  struct Resident {
+    bool fits = false, quads = false;
+    int per_block = 1, stage = 0;
+  };
   template <typename F>
-  int resident_lanes(F runs, int64_t* chunks) const;
+  Resident resident_form(F runs) const;
   bool plan_resident();
   void ensure_graph();
 
@@ -171,9 +177,11 @@ class Batch {
   std::vector<float2> tab_host_;
   DevBuf<int> rb_;  // rebuild work list
   DevBuf<int4> plan_;      // resident steps: the block plan in use
-  DevBuf<unsigned long long> flags_;  // resident steps: group barrier words
+  DevBuf<unsigned long long> flags_;  // resident steps: group barrier words,
+  DevBuf<unsigned> count_;            // arrivals per replica
+  DevBuf<double> tiles_;              // and tile sums
   unsigned seq_ = 0;                  // and the barriers counted so far
-  int lpa_ = 1;                       // lanes per atom of the plan
+  Resident resident_;                 // form of the plan
   std::vector<int4> h_plan_, new_plan_;
   // state readout: two device and two pinned buffers of a piece of atoms each
   DevBuf<char> read_dev_[2];

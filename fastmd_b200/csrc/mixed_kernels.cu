@@ -28,6 +28,7 @@
 
 #include <algorithm>
 #include <cstddef>
+#include <mutex>
 
 #include "counter_rng.h"
 #include "dev_common.cuh"
@@ -1372,15 +1373,12 @@ __device__ __forceinline__ float3 bonded_dr(float4 pi, float4 pj, int G, float h
                      bonded_axis(w_cz(ui), w_cz(uj), pi.z, pj.z, G, h, inv_h, dL));
 }
 
-// Sums of the first BS threads' values (a block may be wider).
 template <int BS>
 __device__ __forceinline__ void block_partials(double* vals, int nv, double* out, int64_t stride) {
   __shared__ double sm[BS / 32][8];
-  if (threadIdx.x < BS) {
-    for (int c = 0; c < nv; ++c) vals[c] = warp_sum(vals[c]);
-    if ((threadIdx.x & 31) == 0)
-      for (int c = 0; c < nv; ++c) sm[threadIdx.x >> 5][c] = vals[c];
-  }
+  for (int c = 0; c < nv; ++c) vals[c] = warp_sum(vals[c]);
+  if ((threadIdx.x & 31) == 0)
+    for (int c = 0; c < nv; ++c) sm[threadIdx.x >> 5][c] = vals[c];
   __syncthreads();
   if (threadIdx.x < nv) {
     double t = 0.0;
@@ -1900,10 +1898,11 @@ struct ForceTables {
 
 // R: the replica's record, or a block's copy of it; ci the chunk's entry.
 // The tables are filled here, the pair parameters (s_eps24, s_sig2) where they
-// are not those of R itself.
+// are not those of R itself.  pbase: the replica's positions, d.pos from its
+// first slot or a copy of them.
 template <bool EV, int B, int PF, int KB, bool LISTED, int SH, bool P2>
 __device__ __forceinline__ void force_chunk_of(const Dev& d, const Rep& R, const int4 ci, int chunk, float4* s_shift,
-                                               float* s_axis, float* s_eps24, float* s_sig2) {
+                                               float* s_axis, float* s_eps24, float* s_sig2, const float4* pbase) {
   constexpr bool RING = PF >= 2 && !LISTED;
   constexpr bool PFR = PF != 0;  // register look-ahead in the loops below
   static_assert(!RING || B == 4, "the ring stages batches of 4 rows");
@@ -1929,7 +1928,6 @@ __device__ __forceinline__ void force_chunk_of(const Dev& d, const Rep& R, const
     s_axis[threadIdx.x] = shift_term(axis_code_e(threadIdx.x), axis_code_k(threadIdx.x), h, dL);
   __syncthreads();
   const int local = ci.w * kChunk + threadIdx.x;
-  const int base = R.slot_base;
   const int s = ci.y + threadIdx.x;
   const float rc2 = (float)(R.rc * R.rc);
   double vals[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -1940,7 +1938,7 @@ __device__ __forceinline__ void force_chunk_of(const Dev& d, const Rep& R, const
     // the whole warp walks its tile's lists (lanes past natoms with none)
     __shared__ __align__(16) uint32_t s_ring[(kChunk / 32) * (RING ? PF : 1) * 4 * 32];
     const bool valid = local < R.natoms;
-    const float4 pi = valid ? d.pos[s] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 pi = valid ? pbase[local] : make_float4(0.f, 0.f, 0.f, 0.f);
     const int ti = w_type(w_bits(pi.w));
     const bool keeps = R.prune_delta > 0.f;
     const int nn = !valid ? 0
@@ -1952,15 +1950,15 @@ __device__ __forceinline__ void force_chunk_of(const Dev& d, const Rep& R, const
     const uint32_t pad = (uint32_t)local | kPadBits;
     if (nt == 1)
       lj_loop_ring<EV, KB, true, SH, P2, (RING ? PF : 2)>(tile_rows, ring, threadIdx.x & 31, nn, nmax, pad,
-                                                          d.pos + base, pi, s_shift, s_axis, ti, nt, s_eps24, s_sig2,
+                                                          pbase, pi, s_shift, s_axis, ti, nt, s_eps24, s_sig2,
                                                           rc2, fx, fy, fz, acc);
     else
       lj_loop_ring<EV, KB, false, SH, P2, (RING ? PF : 2)>(tile_rows, ring, threadIdx.x & 31, nn, nmax, pad,
-                                                           d.pos + base, pi, s_shift, s_axis, ti, nt, s_eps24,
+                                                           pbase, pi, s_shift, s_axis, ti, nt, s_eps24,
                                                            s_sig2, rc2, fx, fy, fz, acc);
   }
-  if (threadIdx.x < kChunk && local < R.natoms) {
-    const float4 pi = d.pos[s];
+  if (local < R.natoms) {
+    const float4 pi = pbase[local];
     const uint32_t ui = w_bits(pi.w);
     const int ti = w_type(ui);
     static_assert(kListPad % B == 0 && kPrunePad % B == 0, "list padding must cover whole batches");
@@ -1970,7 +1968,6 @@ __device__ __forceinline__ void force_chunk_of(const Dev& d, const Rep& R, const
     const size_t row = (size_t)R.nbr_base + ((size_t)(local >> 5) * R.M) * 32 + (local & 31);
     const int nn = pruned ? (d.pcnt[s] + kPrunePad - 1) & ~(kPrunePad - 1) : (d.ncnt[s] + kListPad - 1) & ~(kListPad - 1);
     const uint32_t* lst = (pruned ? d.pnbr : d.nbr) + row;
-    const float4* pbase = d.pos + base;
     if (RING) {
       // the LJ sums are in already
     } else if (LISTED && keeps) {
@@ -2026,7 +2023,8 @@ __device__ __forceinline__ void force_chunk(const Dev& d, int chunk, bool skip_r
   if (need_ev(R) != EV) return;
   if (skip_rebuilt && R.rebuild_now) return;
   __shared__ ForceTables<SH> tb;
-  force_chunk_of<EV, B, PF, KB, LISTED, SH, P2>(d, R, ci, chunk, tb.shift, tb.axis, tb.eps24, tb.sig2);
+  force_chunk_of<EV, B, PF, KB, LISTED, SH, P2>(d, R, ci, chunk, tb.shift, tb.axis, tb.eps24, tb.sig2,
+                                                d.pos + R.slot_base);
 }
 
 // The list filter alone: the entries of the atom's rc + skin list (nn
@@ -2339,22 +2337,24 @@ __device__ __forceinline__ int filter_quads(const uint32_t* lst, int nn, uint32_
   return pc;
 }
 
-// Forces without energies of one chunk by a block of 4 kChunk threads, four
-// lanes per atom; LISTED: the replica's pruned list is due (or it keeps none).
+// Forces without energies of one tile (32 atoms) by a block of kChunk
+// threads, four lanes per atom; LISTED: the replica's pruned list is due (or
+// it keeps none).  R is the block's shared copy of the record.
 template <int KB, bool LISTED>
-__device__ __forceinline__ void force_chunk_quads(const Dev& d, const Rep& R, int r, int c, float* s_axis) {
-  const float *const s_eps24 = R.lj_eps24, *const s_sig2 = R.lj_sig2;  // R is the block's shared copy
+__device__ __forceinline__ void force_tile_quads(const Dev& d, const Rep& R, int r, int tile, float* s_axis) {
+  const float *const s_eps24 = R.lj_eps24, *const s_sig2 = R.lj_sig2;
   const int lane = threadIdx.x & 31, q = lane >> 3, src = lane & 7;
   const int nt = R.ntypes;
   const int G = R.G;
   const float h = R.h, inv_h = 1.0f / h;
   const float dL = (float)(R.L - (double)G * (double)h);
-  const int local = c * kChunk + (threadIdx.x >> 5) * 8 + src;
+  const int local = tile * kTile + (threadIdx.x >> 5) * 8 + src;
   const int base = R.slot_base, s = base + local;
+  const float4* const pbase = d.pos + base;
   const bool valid = local < R.natoms;
   const bool keeps = R.prune_delta > 0.f, pruned = keeps && !LISTED;
   // the atom's own words, all in flight before the tables' barrier
-  const float4 pi = valid ? d.pos[s] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 pi = valid ? pbase[local] : make_float4(0.f, 0.f, 0.f, 0.f);
   const int tc = valid ? d.tcnt[s] : 0;
   int nn = valid ? (pruned ? d.pcnt[s] : d.ncnt[s]) : 0;
   const uint32_t bw = valid ? d.bnd[(size_t)s * kMaxBondsPerAtom + q] : 0u;
@@ -2368,7 +2368,6 @@ __device__ __forceinline__ void force_chunk_quads(const Dev& d, const Rep& R, in
   const uint32_t pad = (uint32_t)(valid ? local : 0) | kPadBits;
   const size_t row = (size_t)R.nbr_base + ((size_t)(local >> 5) * R.M) * 32 + (local & 31);
   const uint32_t* lst = (pruned ? d.pnbr : d.nbr) + row;
-  const float4* pbase = d.pos + base;
   const int ti = w_type(w_bits(pi.w));
   if (LISTED && keeps) {  // replica-uniform
     const float rcd = (float)(R.rc + (double)R.prune_delta);
@@ -2511,7 +2510,8 @@ void launch_prune(const Dev& d, cudaStream_t st);
 // kernel for replicas with tables only; explicit roundings keep the energy
 // flavour's forces identical to the plain one's.
 template <bool EV>
-__device__ __forceinline__ void table_chunk(const Dev& d, const Rep& R, const int4 ci, int chunk, float4* s_shift) {
+__device__ __forceinline__ void table_chunk(const Dev& d, const Rep& R, const int4 ci, int chunk, float4* s_shift,
+                                            const float4* pbase) {
   const int G = R.G;
   const float h = R.h;
   const float dL = (float)(R.L - (double)G * (double)h);
@@ -2528,14 +2528,13 @@ __device__ __forceinline__ void table_chunk(const Dev& d, const Rep& R, const in
   const float rc2 = (float)(R.rc * R.rc);
   const int nt = R.ntypes;
   double vals[7] = {0, 0, 0, 0, 0, 0, 0};
-  if (threadIdx.x < kChunk && local < R.natoms) {
-    const float4 pi = d.pos[s];
+  if (local < R.natoms) {
+    const float4 pi = pbase[local];
     const int ti = w_type(w_bits(pi.w));
     // the pruned list when the replica keeps one (same layout and bases)
     const bool pruned = R.prune_delta > 0.f;
     const int nn = pruned ? (d.pcnt[s] + kPrunePad - 1) & ~(kPrunePad - 1) : (d.ncnt[s] + kListPad - 1) & ~(kListPad - 1);
     const uint32_t* lst = (pruned ? d.pnbr : d.nbr) + R.nbr_base + ((size_t)(local >> 5) * R.M) * 32 + (local & 31);
-    const float4* pbase = d.pos + R.slot_base;
     float fx = 0, fy = 0, fz = 0, pe = 0, v0 = 0, v1 = 0, v2 = 0, v3 = 0, v4 = 0, v5 = 0;
     // Batches of B entries: the list words (loaded a batch ahead), then the
     // positions, then the table points, each B loads in flight together; the
@@ -2632,7 +2631,7 @@ __global__ void __launch_bounds__(kChunk) k_table(Dev d, int sel) {
   if (!R.adv || R.ntables == 0 || need_ev(R) != EV) return;
   if ((sel == 1 && R.rebuild_now) || (sel == 2 && !R.rebuild_now)) return;
   __shared__ float4 s_shift[kShiftCodes];
-  table_chunk<EV>(d, R, ci, blockIdx.x, s_shift);
+  table_chunk<EV>(d, R, ci, blockIdx.x, s_shift, d.pos + R.slot_base);
 }
 
 void launch_table(const Dev& d, int nchunks, bool ev, int sel, cudaStream_t st) {
@@ -2640,6 +2639,101 @@ void launch_table(const Dev& d, int nchunks, bool ev, int sel, cudaStream_t st) 
     k_table<true><<<nchunks, kChunk, 0, st>>>(d, sel);
   else
     k_table<false><<<nchunks, kChunk, 0, st>>>(d, sel);
+}
+
+// The tabulated pairs of one tile by four lanes per atom (see lj_quads): each
+// lane evaluates the entries of its batches and every lane adds the four
+// lanes' pairs in list order, as table_chunk does; an entry without a table
+// adds an exact zero.
+__device__ __forceinline__ void table_tile_quads(const Dev& d, const Rep& R, int tile, float4* s_shift) {
+  const int G = R.G;
+  const float h = R.h;
+  const float dL = (float)(R.L - (double)G * (double)h);
+  if (threadIdx.x < kShiftCodes) {
+    const int c = threadIdx.x;
+    const int ax = c / 25, ay = (c / 5) % 5, az = c % 5;
+    s_shift[c] = make_float4(shift_term(axis_code_e(ax), axis_code_k(ax), h, dL),
+                             shift_term(axis_code_e(ay), axis_code_k(ay), h, dL),
+                             shift_term(axis_code_e(az), axis_code_k(az), h, dL), 0.0f);
+  }
+  __syncthreads();
+  constexpr int B = 4;
+  const int lane = threadIdx.x & 31, g = lane >> 3, src = lane & 7;
+  const int local = tile * kTile + (threadIdx.x >> 5) * 8 + src;
+  const bool valid = local < R.natoms;
+  const int s = R.slot_base + local, nt = R.ntypes;
+  const float4* const pbase = d.pos + R.slot_base;
+  const float4 pi = valid ? pbase[local] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const int ti = w_type(w_bits(pi.w));
+  const bool pruned = R.prune_delta > 0.f;
+  const int padding = pruned ? kPrunePad : kListPad;
+  int nn = valid ? (pruned ? d.pcnt[s] : d.ncnt[s]) : 0;
+  nn = (nn + padding - 1) & ~(padding - 1);
+  const uint32_t pad = (uint32_t)(valid ? local : 0) | kPadBits;
+  const uint32_t* const lst = (pruned ? d.pnbr : d.nbr) + R.nbr_base + ((size_t)(local >> 5) * R.M) * 32 + (local & 31);
+  const float rc2 = (float)(R.rc * R.rc);
+  const int rounds = __reduce_max_sync(0xFFFFFFFFu, (nn + 4 * B - 1) / (4 * B));
+  float fx = 0, fy = 0, fz = 0;
+  uint32_t wn[B];
+#pragma unroll
+  for (int i = 0; i < B; ++i) wn[i] = g * B < nn ? lst[(size_t)(g * B + i) * 32] : pad;
+  for (int t = 0; t < rounds; ++t) {
+    const int k = (4 * (t + 1) + g) * B;
+    uint32_t w[B];
+    float4 pj[B];
+#pragma unroll
+    for (int i = 0; i < B; ++i) {
+      w[i] = wn[i];
+      wn[i] = k < nn ? lst[(size_t)(k + i) * 32] : pad;
+    }
+#pragma unroll
+    for (int i = 0; i < B; ++i) pj[i] = pbase[w[i] & kIdxMask];
+    float dx[B], dy[B], dz[B], u[B];
+    float2 p0[B], p1[B];
+#pragma unroll
+    for (int i = 0; i < B; ++i) {
+      const float3 sh = entry_shift<0>(w[i], s_shift, nullptr);
+      dx[i] = __fsub_rn(__fsub_rn(pi.x, pj[i].x), sh.x);
+      dy[i] = __fsub_rn(__fsub_rn(pi.y, pj[i].y), sh.y);
+      dz[i] = __fsub_rn(__fsub_rn(pi.z, pj[i].z), sh.z);
+      const float r2 = __fadd_rn(__fadd_rn(__fmul_rn(dx[i], dx[i]), __fmul_rn(dy[i], dy[i])), __fmul_rn(dz[i], dz[i]));
+      const int tid = R.table_of[ti * nt + w_type(w_bits(pj[i].w))];
+      u[i] = 0.f;
+      p0[i] = p1[i] = make_float2(0.f, 0.f);
+      if (r2 < rc2 && r2 > 1e-10f && tid >= 0) {
+        const float rmin = R.tab_rmin[tid], rmax = R.tab_rmax[tid], dr = R.tab_dr[tid], inv_dr = R.tab_inv_dr[tid];
+        const float rr = fminf(fmaxf(__fsqrt_rn(r2), rmin), rmax);
+        int idx = (int)__fmul_rn(__fsub_rn(rr, rmin), inv_dr);
+        idx = max(0, min(idx, R.tab_n[tid] - 2));
+        u[i] = __fmul_rn(__fsub_rn(rr, __fadd_rn(rmin, __fmul_rn((float)idx, dr))), inv_dr);
+        const float2* const points = d.tab + R.tab_off[tid] + idx;
+        p0[i] = __ldg(points);
+        p1[i] = __ldg(points + 1);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < B; ++i) {
+      const float fs = __fadd_rn(p0[i].x, __fmul_rn(u[i], __fsub_rn(p1[i].x, p0[i].x)));
+      dx[i] = __fmul_rn(fs, dx[i]);
+      dy[i] = __fmul_rn(fs, dy[i]);
+      dz[i] = __fmul_rn(fs, dz[i]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int i = 0; i < B; ++i) {
+        fx = __fadd_rn(fx, quad_get(dx[i], src, j));
+        fy = __fadd_rn(fy, quad_get(dy[i], src, j));
+        fz = __fadd_rn(fz, quad_get(dz[i], src, j));
+      }
+  }
+  if (valid && g == 0) {
+    float4 f = d.force[s];  // this lane's own store of the pair pass
+    f.x = __fadd_rn(f.x, fx);
+    f.y = __fadd_rn(f.y, fy);
+    f.z = __fadd_rn(f.z, fz);
+    d.force[s] = f;
+  }
 }
 
 // ---------------------------------------------------------------- post-force
@@ -2868,21 +2962,22 @@ __global__ void __launch_bounds__(kPostCommitThreads) k_post_commit(Dev d, int k
 // that of the per-kernel path's device functions in the same order, so the
 // trajectories are bit-identical to it.
 //
-// LPA lanes per atom (blocks of LPA * kChunk threads): 4 for batches whose
-// every chunk has a resident block of that width, 1 beyond.
-constexpr int kStepWin = 704;       // list candidates staged per window
+// QUADS: one 32-atom tile per block, four lanes per atom, where every tile
+// has a resident block; else one lane per atom and several chunks per block.
+// (Four lanes per atom in blocks of 512 threads, a chunk each, left 124 of the
+// SMs without work on 3,000 beads: 18,500 clocks per force evaluation, bound
+// by issue on the 24 SMs in use.)
+constexpr int kStepWin = 704;       // list candidates staged per window: one 27-cell stencil of a melt
 constexpr int kStepSpin = 1 << 22;  // polls of a group barrier before the replica is given up (seconds)
-constexpr int step_threads(int lpa) { return lpa * kChunk; }
-// 8 blocks of 128 threads or 2 of 512: 64 registers
-constexpr int step_blocks_per_sm(int lpa) { return lpa == 1 ? 8 : 2; }
+constexpr int kStepBlocksPerSM = 8;  // 64 registers
 constexpr int kStepKicks = 4;  // chunks whose post-force partials are staged at a time
+constexpr int kStepFlags = 128;  // blocks of a group up to which each polls every other's word
 
 // A resident block's shared memory besides the record: the stages of a step
 // use it in turn (small, so that the L1 keeps the rest of the array for the
 // position gathers).
-template <int LPA>
 union StepStage {
-  ListStage<kStepWin, step_threads(LPA) / 32> list;
+  ListStage<kStepWin, kChunk / 32> list;
   struct {
     float4 shift[kShiftCodes];
     float axis[5];
@@ -2898,6 +2993,11 @@ __device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long lon
   asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ unsigned ld_relaxed(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
 __device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long long v) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
@@ -2905,36 +3005,58 @@ __device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long 
 // A replica's group of blocks within k_steps.
 struct StepGroup {
   int r, rank, nb;            // replica, this block's rank, blocks
-  int c0, c1;                 // this block's chunks
-  unsigned long long* flags;  // the group's words: barrier number << 32 | value, two sets in turn
+  int a0, a1;                 // this block's slots (replica-local): pre-force, rebuild
+  int c0, c1;                 // its chunks: forces (QUADS: of energy steps), post-force partials
+  unsigned long long* flags;  // small groups: barrier number << 32 | value per block, two sets in turn
   int stride;                 // from one set to the other
-  unsigned seq;               // number of the last barrier
+  unsigned* count;            // larger ones: arrivals since the launch began, then three maxima in turn
+  unsigned seq;               // number of the last barrier, counted on from the launch before
+  unsigned nth;               // barriers of this launch
   int* dead;                  // shared: a barrier ran out of polls
   uint32_t* s_max;            // shared: per-warp maxima
 };
 
 // Barrier over the group's blocks; memory written by them before it is
-// visible after it (the fence also drops this SM's stale L1 lines).  Each
-// block posts its number in its own word and polls every block's, so arrival
-// and release are one store and one load apart; a word carries a value
-// (value: thread 0's), and thread 0 gets the largest back in most.  A block
-// is at most one barrier ahead of another's reads: two sets of words are
-// enough.  False when the wait ran out: the replica is faulted and the block
-// gives up.
+// visible after it (the fence also drops this SM's stale L1 lines).  most: the
+// largest of the blocks' values (thread 0 in, thread 0 out).
+//
+// Up to kStepFlags blocks, each posts its number and value in a word of its
+// own and polls every block's: arrival and release are one store and one
+// load apart.  A block is at most one barrier ahead of another's reads, so
+// two sets of words are enough.  Larger groups count arrivals in one word
+// (polling every block's would be megabytes of loads per round) and take the
+// maximum in one of three, the one of two barriers ahead cleared by rank 0.
+// False when the wait ran out: the replica is faulted and the block gives up.
 __device__ __forceinline__ bool group_sync(StepGroup& g, uint32_t value = 0u, uint32_t* most = nullptr) {
-  const unsigned seq = ++g.seq;
+  const unsigned seq = ++g.seq, nth = ++g.nth;
   __syncthreads();
   uint32_t m = value;
-  if (g.nb > 1) {
+  if (g.nb > kStepFlags) {
+    if (threadIdx.x == 0) {
+      unsigned* const top = g.count + 1;
+      if (most) atomicMax(top + nth % 3, value);
+      __threadfence();
+      atomicAdd(g.count, 1u);
+      for (int polls = 0; (int)(ld_relaxed(g.count) - nth * (unsigned)g.nb) < 0;)
+        if (++polls > kStepSpin) {
+          *g.dead = 1;
+          break;
+        }
+      __threadfence();
+      if (most) m = ld_relaxed(top + nth % 3);
+      if (g.rank == 0) top[(nth + 2) % 3] = 0u;
+    }
+    __syncthreads();
+  } else if (g.nb > 1) {
     unsigned long long* const f = g.flags + (seq & 1u) * g.stride;
     if (threadIdx.x == 0) {
       __threadfence();
       st_relaxed(f + g.rank, ((unsigned long long)seq << 32) | value);
     }
     if ((int)(threadIdx.x & ~31u) < g.nb) {  // the warps that poll
-      for (int i = threadIdx.x; i < g.nb; i += blockDim.x) {
-        unsigned long long w = ld_relaxed(f + i);
-        for (int polls = 0; (int)((unsigned)(w >> 32) - seq) < 0; w = ld_relaxed(f + i))
+      if ((int)threadIdx.x < g.nb) {
+        unsigned long long w = ld_relaxed(f + threadIdx.x);
+        for (int polls = 0; (int)((unsigned)(w >> 32) - seq) < 0; w = ld_relaxed(f + threadIdx.x))
           if (++polls > kStepSpin) {
             *g.dead = 1;
             break;
@@ -2943,13 +3065,14 @@ __device__ __forceinline__ bool group_sync(StepGroup& g, uint32_t value = 0u, ui
       }
       __threadfence();
       if (most) {
+        __syncwarp();
         warp_max_u32(m);
         if ((threadIdx.x & 31) == 0) g.s_max[threadIdx.x >> 5] = m;
       }
     }
     __syncthreads();
     if (most && threadIdx.x == 0)
-      for (int w = 0; w < (int)(blockDim.x >> 5) && 32 * w < g.nb; ++w) m = max(m, g.s_max[w]);
+      for (int w = 0; w < kChunk / 32 && 32 * w < g.nb; ++w) m = max(m, g.s_max[w]);
   }
   if (most) *most = m;
   return *g.dead == 0;
@@ -3002,14 +3125,12 @@ __device__ __forceinline__ void scan_cells_block(const Dev& d, const Rep& R) {
 
 // The rebuild of a group's replica: the phases of launch_rebuild with a group
 // barrier in the place of each kernel boundary.
-template <int LPA>
-__device__ __noinline__ bool rebuild_group(const Dev& d, Rep& R, StepGroup& g, StepStage<LPA>& st) {
-  constexpr int T = step_threads(LPA), W = T / 32;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int t = threadIdx.x % kChunk, cf = g.c0 + threadIdx.x / kChunk;  // LPA chunks at a time
-  for (int c = cf; c < g.c1; c += LPA) bin_chunk(d, R, c, t);
+__device__ __noinline__ bool rebuild_group(const Dev& d, Rep& R, StepGroup& g, StepStage& st) {
+  constexpr int W = kChunk / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, first = g.a0 + threadIdx.x;
+  for (int a = first; a < g.a1; a += kChunk) bin_chunk(d, R, 0, a);
   if (!group_sync(g)) return false;
-  if (g.rank == 0) scan_cells_block<T>(d, R);
+  if (g.rank == 0) scan_cells_block<kChunk>(d, R);
   if (threadIdx.x == 0) {
     int Gn = (int)floor(R.L / ((R.rc + R.skin) * 1.0001));
     Gn = Gn < 1 ? 1 : (Gn > R.G_alloc ? R.G_alloc : Gn);
@@ -3017,14 +3138,14 @@ __device__ __noinline__ bool rebuild_group(const Dev& d, Rep& R, StepGroup& g, S
     R.h = (float)(R.L / Gn);
   }
   if (!group_sync(g)) return false;
-  for (int c = cf; c < g.c1; c += LPA) scatter_chunk(d, R, c, t);
+  for (int a = first; a < g.a1; a += kChunk) scatter_chunk(d, R, 0, a);
   if (!group_sync(g)) return false;
   const int ncell = R.P * R.P * R.P;
   for (int c = g.rank * W + warp; c < ncell; c += g.nb * W) cellsort_cell(d, R, c, lane);
   if (!group_sync(g)) return false;
-  for (int c = cf; c < g.c1; c += LPA) permute_chunk(d, R, c, t);
+  for (int a = first; a < g.a1; a += kChunk) permute_chunk(d, R, 0, a);
   if (!group_sync(g)) return false;
-  for (int c = cf; c < g.c1; c += LPA) topo_chunk(d, R, c, t);
+  for (int a = first; a < g.a1; a += kChunk) topo_chunk(d, R, 0, a);
   if (!group_sync(g)) return false;
   int* const status = &d.reps[g.r].status;
   const int home = R.G * R.G * R.G;
@@ -3033,55 +3154,74 @@ __device__ __noinline__ bool rebuild_group(const Dev& d, Rep& R, StepGroup& g, S
       __syncthreads();  // the previous cell's staging is no longer read
       neighbors_cell_ballot(d, R, status, lc, st.list);
     } else {
-      const int ov = neighbors_small_box(d, R, lc, lane, 32 * warp, T);
+      const int ov = neighbors_small_box(d, R, lc, lane, 32 * warp, kChunk);
       if (ov) atomicOr(status, ov);
     }
   }
   return group_sync(g);
 }
 
-template <bool EV, int KB, int LPA>
-__device__ __forceinline__ void forces_group(const Dev& d, Rep& R, const StepGroup& g, StepStage<LPA>& st) {
+// Forces of the group's chunks, one lane per atom; ST: the replica's
+// positions are first copied to shared memory (small replicas: the gathers'
+// L2 round trips, every step's positions being new to this SM's L1, become
+// shared loads: 200 x 1,000 beads 18.7 -> 17.4 ms per 200 steps).
+template <bool EV, int KB, bool ST>
+__device__ __forceinline__ void forces_group(const Dev& d, Rep& R, const StepGroup& g, StepStage& st) {
+  extern __shared__ float4 s_pos[];
+  const float4* const pbase = ST ? s_pos : d.pos + R.slot_base;
+  if (ST) {
+    const float4* const src = d.pos + R.slot_base;
+    for (int i = threadIdx.x; i < R.natoms; i += kChunk) cp_async16_stream(s_pos + i, src + i);
+    cp_async_wait_all();
+    __syncthreads();
+  }
   for (int c = g.c0; c < g.c1; ++c) {
     const int4 ci = make_int4(g.r, R.slot_base + c * kChunk, 0, c);
     const int chunk = R.chunk_base + c;
-    if (!EV && LPA == 4) {
-      if (R.rebuild_now)
-        force_chunk_quads<KB, true>(d, R, g.r, c, st.force.axis);
-      else
-        force_chunk_quads<KB, false>(d, R, g.r, c, st.force.axis);
-    } else if (R.rebuild_now) {
-      force_chunk_of<EV, 4, true, KB, true, 1, true>(d, R, ci, chunk, nullptr, st.force.axis, R.lj_eps24, R.lj_sig2);
-    } else {
-      force_chunk_of<EV, 4, true, KB, false, 1, true>(d, R, ci, chunk, nullptr, st.force.axis, R.lj_eps24, R.lj_sig2);
-    }
+    if (R.rebuild_now)
+      force_chunk_of<EV, 4, true, KB, true, 1, true>(d, R, ci, chunk, nullptr, st.force.axis, R.lj_eps24, R.lj_sig2, pbase);
+    else
+      force_chunk_of<EV, 4, true, KB, false, 1, true>(d, R, ci, chunk, nullptr, st.force.axis, R.lj_eps24, R.lj_sig2, pbase);
     __syncthreads();  // the tables and the block partials' staging are free again
     if (R.ntables) {
-      table_chunk<EV>(d, R, ci, chunk, st.force.shift);
+      table_chunk<EV>(d, R, ci, chunk, st.force.shift, pbase);
       __syncthreads();
     }
   }
 }
 
+// Forces without energies of the block's tile, four lanes per atom.
+template <int KB>
+__device__ __forceinline__ void forces_tile(const Dev& d, Rep& R, const StepGroup& g, StepStage& st) {
+  if (R.rebuild_now)
+    force_tile_quads<KB, true>(d, R, g.r, g.rank, st.force.axis);
+  else
+    force_tile_quads<KB, false>(d, R, g.r, g.rank, st.force.axis);
+  __syncthreads();  // the tables are free again
+  if (R.ntables) {
+    table_tile_quads(d, R, g.rank, st.force.shift);
+    __syncthreads();
+  }
+}
+
 // The energy flavour and the chain commit out of line: their registers stay
 // out of the plain step's loops.
-template <int KB, int LPA>
-__device__ __noinline__ void forces_group_ev(const Dev& d, Rep& R, const StepGroup& g, StepStage<LPA>& st) {
-  forces_group<true, KB, LPA>(d, R, g, st);
+template <int KB, bool ST>
+__device__ __noinline__ void forces_group_ev(const Dev& d, Rep& R, const StepGroup& g, StepStage& st) {
+  forces_group<true, KB, ST>(d, R, g, st);
 }
 __device__ __noinline__ void post_commit_shared(Rep& R, const double* acc) { post_commit_state<true>(R, acc, 1); }
 
-// The post-force half kick and KE partials of the group's chunks, LPA chunks
-// side by side and kStepKicks of their partials staged at a time: per chunk
-// the warps' sums in warp order, as block_partials adds them.
-template <int LPA>
-__device__ __forceinline__ void kicks_group(const Dev& d, const Rep& R, const StepGroup& g, StepStage<LPA>& st) {
-  const int lane = threadIdx.x & 31, warp = (threadIdx.x % kChunk) >> 5;
+// The post-force half kick and KE partials of the group's chunks, kStepKicks
+// of their partials staged at a time: per chunk the warps' sums in warp
+// order, as block_partials adds them.
+__device__ __forceinline__ void kicks_group(const Dev& d, const Rep& R, const StepGroup& g, StepStage& st) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int c0 = g.c0; c0 < g.c1; c0 += kStepKicks) {
     const int c1 = min(c0 + kStepKicks, g.c1);
 #pragma unroll 1
-    for (int c = c0 + threadIdx.x / kChunk; c < c1; c += LPA) {
-      const int local = c * kChunk + threadIdx.x % kChunk, s = R.slot_base + local;
+    for (int c = c0; c < c1; ++c) {
+      const int local = c * kChunk + threadIdx.x, s = R.slot_base + local;
       double vals[6] = {0, 0, 0, 0, 0, 0};
       if (local < R.natoms) post_atom(d, R, s, d.vel[s], d.force[s], 1, vals);
 #pragma unroll
@@ -3100,15 +3240,27 @@ __device__ __forceinline__ void kicks_group(const Dev& d, const Rep& R, const St
   }
 }
 
-// The replica's partials (values q0 .. 12) summed in k_post_commit's order by
-// a block of T threads: thread t of its kPostCommitThreads adds chunks t,
-// t + kPostCommitThreads, ..., a shuffle tree per warp, then the warp totals
-// in order.
-template <int T>
-__device__ __forceinline__ void reduce_partials(const Dev& d, const Rep& R, int q0, double (*s_red)[13], double* s_acc) {
+// The same of the block's tile by its first warp: a warp's sum of its chunk.
+__device__ __forceinline__ void kicks_tile(const Dev& d, const Rep& R, const StepGroup& g, double* tile_part) {
+  if (threadIdx.x >= 32) return;
+  const int local = g.a0 + threadIdx.x, s = R.slot_base + local;
+  double vals[6] = {0, 0, 0, 0, 0, 0};
+  if (local < R.natoms) post_atom(d, R, s, d.vel[s], d.force[s], 1, vals);
+#pragma unroll
+  for (int q = 0; q < 6; ++q) vals[q] = warp_sum(vals[q]);
+  if (threadIdx.x == 0)
+    for (int q = 0; q < 6; ++q) tile_part[q] = vals[q];
+}
+
+// The replica's partials (values q0 .. 12) summed in k_post_commit's order:
+// thread t of its kPostCommitThreads adds chunks t, t + kPostCommitThreads,
+// ..., a shuffle tree per warp, then the warp totals in order.  tiles: the
+// KE values come from the group's tile sums (6 per tile), four to a chunk.
+__device__ __forceinline__ void reduce_partials(const Dev& d, const Rep& R, int q0, const double* tiles, int ntiles,
+                                                double (*s_red)[13], double* s_acc) {
   const int lane = threadIdx.x & 31;
   constexpr int nw = kPostCommitThreads / 32;
-  for (int vt = threadIdx.x; vt < kPostCommitThreads; vt += T) {
+  for (int vt = threadIdx.x; vt < kPostCommitThreads; vt += kChunk) {
     if (vt - lane >= R.nchunks) {  // warp-uniform: no chunks, zero totals
       if (lane < 13) s_red[vt >> 5][lane] = 0.0;
       continue;
@@ -3116,10 +3268,20 @@ __device__ __forceinline__ void reduce_partials(const Dev& d, const Rep& R, int 
     double acc[13];
 #pragma unroll
     for (int q = 0; q < 13; ++q) acc[q] = 0.0;
-    for (int c = vt; c < R.nchunks; c += kPostCommitThreads)
+    for (int c = vt; c < R.nchunks; c += kPostCommitThreads) {
+      if (tiles) {
+        double t[6] = {0, 0, 0, 0, 0, 0};
+        for (int w = 4 * c; w < min(4 * c + 4, ntiles); ++w)
 #pragma unroll
-      for (int q = 0; q < 13; ++q)
-        if (q >= q0) acc[q] += d.part[q * d.part_stride + R.chunk_base + c];
+          for (int q = 0; q < 6; ++q) t[q] += tiles[6 * w + q];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) acc[7 + q] += t[q];
+      } else {
+#pragma unroll
+        for (int q = 0; q < 13; ++q)
+          if (q >= q0) acc[q] += d.part[q * d.part_stride + R.chunk_base + c];
+      }
+    }
 #pragma unroll
     for (int q = 0; q < 13; ++q) {
       if (q >= q0) acc[q] = warp_sum(acc[q]);
@@ -3136,23 +3298,26 @@ __device__ __forceinline__ void reduce_partials(const Dev& d, const Rep& R, int 
   __syncthreads();
 }
 
-template <int KB, int LPA>
-__global__ void __launch_bounds__(step_threads(LPA), step_blocks_per_sm(LPA))
-    k_steps(Dev d, const int4* plan, unsigned long long* flags, unsigned seq, int max_steps) {
-  constexpr int T = step_threads(LPA);
+template <int KB, bool QUADS, bool ST>
+__global__ void __launch_bounds__(kChunk, kStepBlocksPerSM)
+    k_steps(Dev d, const int4* plan, StepSync sync, unsigned seq, int max_steps) {
+  constexpr int T = kChunk;
   __shared__ __align__(16) Rep R;
   __shared__ int dead;
   __shared__ uint32_t s_max[T / 32];
-  __shared__ StepStage<LPA> st;
+  __shared__ StepStage st;
   __shared__ double s_acc[13];
   const int4 pl = plan[blockIdx.x];
   StepGroup g;
   g.r = pl.x;
   g.rank = pl.y;
   g.nb = pl.z;
-  g.flags = flags + pl.w;
+  g.flags = sync.flags + pl.w;
   g.stride = gridDim.x;
+  g.count = sync.count + kStepCountWords * pl.x;
   g.seq = seq;
+  g.nth = 0;
+  double* const tiles = sync.tiles + 6 * (size_t)pl.w;  // QUADS: the group's tile sums
   g.dead = &dead;
   g.s_max = s_max;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -3166,8 +3331,18 @@ __global__ void __launch_bounds__(step_threads(LPA), step_blocks_per_sm(LPA))
   if (threadIdx.x == 0) dead = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(d.kcount + kKForce, 1ull);
   __syncthreads();
-  g.c0 = (int)((int64_t)g.rank * R.nchunks / g.nb);
-  g.c1 = (int)((int64_t)(g.rank + 1) * R.nchunks / g.nb);
+  if (QUADS) {
+    // a tile per block; the block of a chunk's first tile has the chunk
+    g.c0 = (g.rank + 3) / 4;
+    g.c1 = g.rank / 4 + 1;
+    g.a0 = g.rank * kTile;
+    g.a1 = g.a0 + kTile;
+  } else {
+    g.c0 = (int)((int64_t)g.rank * R.nchunks / g.nb);
+    g.c1 = (int)((int64_t)(g.rank + 1) * R.nchunks / g.nb);
+    g.a0 = g.c0 * kChunk;
+    g.a1 = g.c1 * kChunk;
+  }
   const int64_t left = R.active ? R.stop_step - R.step : 0;
   const int steps = (int)(left < max_steps ? left : max_steps);
   if (steps <= 0) return;  // the same in every block of the group
@@ -3184,10 +3359,9 @@ __global__ void __launch_bounds__(step_threads(LPA), step_blocks_per_sm(LPA))
     uint32_t d2bits = 0;
     int bad = 0;
     const bool deferred = R.defer != 0;
-    for (int c = g.c0 + threadIdx.x / kChunk; c < g.c1; c += LPA) {
-      const int local = c * kChunk + threadIdx.x % kChunk, s = R.slot_base + local;
-      if (local < R.natoms)
-        pre_atom(d, R, R.next, s, deferred, from[s], d.vel[s], d.force[s], d.ref[s], d2bits, bad);
+    for (int local = g.a0 + threadIdx.x; local < min(g.a1, R.natoms); local += T) {
+      const int s = R.slot_base + local;
+      pre_atom(d, R, R.next, s, deferred, from[s], d.vel[s], d.force[s], d.ref[s], d2bits, bad);
     }
     if (bad) atomicOr(&d.reps[g.r].status, kStatusNonFinite);
     warp_max_u32(d2bits);
@@ -3204,21 +3378,28 @@ __global__ void __launch_bounds__(step_threads(LPA), step_blocks_per_sm(LPA))
       R.defer = post_needed(R) ? 0 : 1;
     }
     __syncthreads();
-    if (R.rebuild_now == kListRebuild && !rebuild_group<LPA>(d, R, g, st)) break;
-    const bool defer = R.defer != 0;
-    if (need_ev(R))
-      forces_group_ev<KB, LPA>(d, R, g, st);
+    if (R.rebuild_now == kListRebuild && !rebuild_group(d, R, g, st)) break;
+    const bool defer = R.defer != 0, ev = need_ev(R);
+    if (ev)
+      forces_group_ev<KB, ST>(d, R, g, st);
+    else if (QUADS)
+      forces_tile<KB>(d, R, g, st);
     else
-      forces_group<false, KB, LPA>(d, R, g, st);
+      forces_group<false, KB, ST>(d, R, g, st);
     if (defer) {
       if (threadIdx.x == 0) {
         step_scalars<false>(R, R.next);
         R.next_valid = 1;
       }
     } else {
-      kicks_group<LPA>(d, R, g, st);
+      // on an energy step a chunk's forces are its own block's, tiles or not
+      const bool by_tile = QUADS && !ev;
+      if (by_tile)
+        kicks_tile(d, R, g, tiles + 6 * g.rank);
+      else
+        kicks_group(d, R, g, st);
       if (!group_sync(g)) break;
-      reduce_partials<T>(d, R, need_ev(R) ? 0 : 7, st.red, s_acc);
+      reduce_partials(d, R, ev ? 0 : 7, by_tile ? tiles : nullptr, g.nb, st.red, s_acc);
       if (threadIdx.x == 0) post_commit_shared(R, s_acc);
       __syncthreads();
       if (g.rank == 0 && warp == 0 && stress_step(R)) acf_sample(d, R, g.r);
@@ -3227,9 +3408,9 @@ __global__ void __launch_bounds__(step_threads(LPA), step_blocks_per_sm(LPA))
   }
   if (dead && threadIdx.x == 0) atomicOr(&d.reps[g.r].status, kStatusTimeout);
   if (d.pos != home)  // no block reads the other buffer any more
-    for (int c = g.c0 + threadIdx.x / kChunk; c < g.c1; c += LPA) {
-      const int local = c * kChunk + threadIdx.x % kChunk, s = R.slot_base + local;
-      if (local < R.natoms) home[s] = d.pos[s];
+    for (int local = g.a0 + threadIdx.x; local < min(g.a1, R.natoms); local += T) {
+      const int s = R.slot_base + local;
+      home[s] = d.pos[s];
     }
   if (g.rank == 0) {
     // the record, less its status word (raised in place by any block)
@@ -3392,48 +3573,65 @@ void prefer_l1(K kernel, int pct = kForceCarveoutPct) {
   FMD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct));
 }
 
-// The carve-out that holds a resident block's shared memory as often as the
-// block fits an SM; the rest of the array is L1 for the position gathers (the
-// driver's own choice left it 28 KB).
-template <typename K>
-void steps_carveout(K kernel, int blocks_per_sm) {
-  cudaFuncAttributes a;
-  FMD_CUDA(cudaFuncGetAttributes(&a, kernel));
-  const int kb = (int)((a.sharedSizeBytes + 1023) / 1024 + 1) * blocks_per_sm;
-  prefer_l1(kernel, std::min(100, (100 * kb + 227) / 228));
+namespace {
+using StepKernel = void (*)(Dev, const int4*, StepSync, unsigned, int);
+// form: 0 one lane per atom, 1 with the positions in shared memory, 2 QUADS
+StepKernel step_kernel(bool two, int form) {
+  return form == 2 ? (two ? k_steps<2, true, false> : k_steps<1, true, false>)
+       : form == 1 ? (two ? k_steps<2, false, true> : k_steps<1, false, true>)
+                   : (two ? k_steps<2, false, false> : k_steps<1, false, false>);
 }
+int step_form(bool quads, int stage_bytes) { return quads ? 2 : stage_bytes > 0 ? 1 : 0; }
 
-int steps_resident_blocks(int lpa) {
-  static const bool carved = [] {
-    steps_carveout(k_steps<1, 1>, step_blocks_per_sm(1));
-    steps_carveout(k_steps<2, 1>, step_blocks_per_sm(1));
-    steps_carveout(k_steps<1, 4>, step_blocks_per_sm(4));
-    steps_carveout(k_steps<2, 4>, step_blocks_per_sm(4));
-    return true;
-  }();
-  (void)carved;
-  static const int n1 = std::min(resident_grid(k_steps<1, 1>, step_threads(1)), resident_grid(k_steps<2, 1>, step_threads(1)));
-  static const int n4 = std::min(resident_grid(k_steps<1, 4>, step_threads(4)), resident_grid(k_steps<2, 4>, step_threads(4)));
-  return lpa == 4 ? n4 : n1;
+// Once per device: the carve-out that holds the kernels' shared memory as often
+// as a block fits an SM; the rest of the array is L1 for the gathers.
+void step_attributes() {
+  static std::mutex mu;
+  static bool done[256] = {};
+  int dev = 0;
+  FMD_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lock(mu);
+  if (dev >= 0 && dev < 256 && done[dev]) return;
+  for (int form = 0; form < 3; ++form)
+    for (bool two : {false, true}) {
+      cudaFuncAttributes a;
+      FMD_CUDA(cudaFuncGetAttributes(&a, step_kernel(two, form)));
+      const int kb = (int)((a.sharedSizeBytes + 1023) / 1024 + 1) * kStepBlocksPerSM;
+      prefer_l1(step_kernel(two, form), form == 1 ? 100 : std::min(100, (100 * kb + 227) / 228));
+    }
+  if (dev >= 0 && dev < 256) done[dev] = true;
+}
+}  // namespace
+
+int steps_resident_blocks(bool quads, int stage_bytes) {
+  step_attributes();
+  int n = 0;
+  for (bool two : {false, true}) {
+    int per_sm = 0;
+    FMD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, step_kernel(two, step_form(quads, stage_bytes)),
+                                                           kChunk, stage_bytes));
+    n = two ? std::min(n, per_sm) : per_sm;
+  }
+  return n * num_sms();
 }
 
 bool steps_variant(int force_variant) { return force_variant != 9 && force_variant != 10; }
 
-void launch_steps(const Dev& d, const int4* plan, int blocks, int lpa, unsigned long long* flags, unsigned seq,
-                  int force_variant, int max_steps, cudaStream_t st) {
+void launch_steps(const Dev& d, const int4* plan, int blocks, bool quads, int stage_bytes, const StepSync& sync,
+                  int nreps, unsigned seq, int force_variant, int max_steps, cudaStream_t st) {
+  FMD_CUDA(cudaMemsetAsync(sync.count, 0, sizeof(unsigned) * kStepCountWords * nreps, st));
   const bool two = force_variant == 1 || force_variant == 3 || force_variant == 5;
-  void (*const kernel)(Dev, const int4*, unsigned long long*, unsigned, int) =
-      lpa == 4 ? (two ? k_steps<2, 4> : k_steps<1, 4>) : (two ? k_steps<2, 1> : k_steps<1, 1>);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = blocks;
-  cfg.blockDim = step_threads(lpa);
+  cfg.blockDim = kChunk;
+  cfg.dynamicSmemBytes = stage_bytes;
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeCooperative;  // every block resident: they wait for one another
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  FMD_CUDA(cudaLaunchKernelEx(&cfg, kernel, d, plan, flags, seq, max_steps));
+  FMD_CUDA(cudaLaunchKernelEx(&cfg, step_kernel(two, step_form(quads, stage_bytes)), d, plan, sync, seq, max_steps));
 }
 
 // The pre-force update of every chunk, one block per chunk.  (A resident
