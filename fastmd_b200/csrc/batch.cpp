@@ -730,7 +730,7 @@ Batch::Resident Batch::resident_form(F runs) const {
     chained |= R.mode == kModeRun && R.ensemble != FMD_LANGEVIN;
   }
   if (graph_steps_ <= 0 || groups == 0) return f;
-  if (tiles <= steps_resident_blocks(true, 0)) {
+  if (tiles <= steps_resident_blocks(true, 0) && most <= kStepTileChunks) {
     f.fits = f.quads = true;
     return f;
   }
@@ -768,17 +768,14 @@ bool Batch::plan_resident() {
     const size_t room = std::max({(int)new_plan_.size(), steps_resident_blocks(true, 0), steps_resident_blocks(false, 0)});
     FMD_CUDA(cudaStreamSynchronize(st_));
     plan_.alloc(room);
-    flags_.alloc(2 * room);
     tiles_.alloc(6 * room);
-    count_.alloc((size_t)max_reps_ * kStepCountWords);
+    sync_.alloc((size_t)max_reps_ * kStepCountWords / 2 + 2 * room);
     h_plan_.clear();
   }
   const bool same = new_plan_.size() == h_plan_.size() &&
                     std::memcmp(new_plan_.data(), h_plan_.data(), h_plan_.size() * sizeof(int4)) == 0;
   if (!same) {
     h_plan_ = new_plan_;
-    seq_ = 0;  // no word of another layout stays behind
-    FMD_CUDA(cudaMemsetAsync(flags_, 0, flags_.bytes(), st_));
     FMD_CUDA(cudaMemcpyAsync(plan_, h_plan_.data(), h_plan_.size() * sizeof(int4), cudaMemcpyHostToDevice, st_));
   }
   return true;
@@ -788,11 +785,10 @@ bool Batch::plan_resident() {
 void Batch::advance(int64_t nsteps) {
   const Dev d = dev();
   if (plan_resident()) {
+    const StepSync sync{reinterpret_cast<unsigned*>(sync_.p), sync_.p + (size_t)max_reps_ * kStepCountWords / 2, tiles_};
     while (nsteps > 0) {
       const int k = (int)std::min<int64_t>(nsteps, kResidentSteps);
-      launch_steps(d, plan_, (int)h_plan_.size(), resident_.quads, resident_.stage, StepSync{flags_, count_, tiles_},
-                   max_reps_, seq_, force_variant_, k, st_);
-      seq_ += (unsigned)k * kStepBarriers;
+      launch_steps(d, plan_, (int)h_plan_.size(), resident_.quads, resident_.stage, sync, force_variant_, k, st_);
       nsteps -= k;
     }
     return;

@@ -177,11 +177,9 @@ class Batch {
   std::vector<float2> tab_host_;
   DevBuf<int> rb_;  // rebuild work list
   DevBuf<int4> plan_;      // resident steps: the block plan in use
-  DevBuf<unsigned long long> flags_;  // resident steps: group barrier words,
-  DevBuf<unsigned> count_;            // arrivals per replica
-  DevBuf<double> tiles_;              // and tile sums
-  unsigned seq_ = 0;                  // and the barriers counted so far
-  Resident resident_;                 // form of the plan
+  DevBuf<unsigned long long> sync_;  // resident steps: barrier words per replica and block,
+  DevBuf<double> tiles_;             // and tile sums
+  Resident resident_;       // form of the plan
   std::vector<int4> h_plan_, new_plan_;
   // state readout: two device and two pinned buffers of a piece of atoms each
   DevBuf<char> read_dev_[2];

@@ -368,26 +368,25 @@ void launch_reduce_only(const Dev& d, int nchunks, int nreps, cudaStream_t st, i
 // per tile (step_tiles of each replica), four lanes per atom; else one lane
 // per atom, a group's blocks sharing the replica's chunks, and with
 // stage_bytes > 0 each keeps the replica's positions in that much shared
-// memory (16 bytes per atom of the largest, at most kStepStageBytes).  seq:
-// barriers counted so far, at most kStepBarriers per step of each launch.
+// memory (16 bytes per atom of the largest, at most kStepStageBytes).
 // Force variants with several lanes per atom are not built in this form.
-constexpr unsigned kStepBarriers = 16;
 constexpr int kStepCountWords = 4;
 constexpr int kStepStageBytes = 24 * 1024;  // five blocks per SM
 struct StepSync {
-  unsigned long long* flags;  // 2 words per block, kept between launches
-  unsigned* count;            // kStepCountWords per replica
-  double* tiles;              // 6 per block
+  unsigned* count;  // kStepCountWords per replica
+  unsigned long long* flags;  // 2 per block, behind count in one allocation
+  double* tiles;    // 6 per block
 };
 // Tiles that hold a replica's atoms, and the first of each of its chunks.
 inline int step_tiles(int natoms, int nchunks) {
   const int t = (natoms + kTile - 1) / kTile, c = (kChunk / kTile) * (nchunks - 1) + 1;
   return t > c ? t : c;
 }
+constexpr int kStepTileChunks = 304;  // chunks of a replica stepped by tiles (8 blocks on each of 148 SMs, 4 to a chunk)
 int steps_resident_blocks(bool quads, int stage_bytes);
 bool steps_variant(int force_variant);
 void launch_steps(const Dev& d, const int4* plan, int blocks, bool quads, int stage_bytes, const StepSync& sync,
-                  int nreps, unsigned seq, int force_variant, int max_steps, cudaStream_t st);
+                  int force_variant, int max_steps, cudaStream_t st);
 void launch_prepare(const Dev& d, int nreps, cudaStream_t st);  // 0 setup, 2 re-evaluation
 
 }  // namespace mixed

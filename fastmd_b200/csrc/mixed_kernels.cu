@@ -463,11 +463,12 @@ __global__ void __launch_bounds__(32) k_prepare(Dev d) {
 
 // ---------------------------------------------------------------- rebuild
 // Minimum-image cell shift of j relative to i and the periodic wrap count,
-// for cell coordinates ci, cj and offsets oi, oj (one axis).
+// for cell coordinates ci, cj and offsets oi, oj (one axis; G = 1 or 2, so
+// that the product is the exact quotient by G).
 __device__ __forceinline__ void pair_shift(int ci, int cj, float oi, float oj, int G, float inv_h, int& e, int& k) {
   const int dc = ci - cj;
   const float D = (float)dc + (oi - oj) * inv_h;
-  k = (int)rintf(D / (float)G);
+  k = (int)rintf(D * (G == 1 ? 1.0f : 0.5f));
   e = k * G - dc;
 }
 
@@ -756,7 +757,8 @@ __global__ void __launch_bounds__(kChunk) k_scatter(Dev d) {
   for_rebuild_chunks(d, [&](const Rep& R, int, int ci) { scatter_chunk(d, R, ci, threadIdx.x); });
 }
 
-// Per cell: order members by atom id (deterministic), write the permutation.
+// Per cell: order members by atom id (deterministic), write the permutation
+// and the atoms' new slots.
 // grid (cell blocks, replicas); one warp per cell.  Cells of up to 32
 // members rank in registers with shuffles; larger ones fall back to a loop
 // over the bucket.
@@ -773,7 +775,10 @@ __device__ __forceinline__ void cellsort_cell(const Dev& d, const Rep& R, int c,
       }
       int rank = 0;
       for (int b = 0; b < n; ++b) rank += (__shfl_sync(0xFFFFFFFFu, id, b) < id);
-      if (lane < n) d.perm[R.slot_base + st + rank] = old;
+      if (lane < n) {
+        d.perm[R.slot_base + st + rank] = old;
+        d.slot_of[R.slot_base + id] = st + rank;
+      }
     } else {
       for (int a = lane; a < n; a += 32) {
         const int old = d.bucket[R.slot_base + st + a];
@@ -781,6 +786,7 @@ __device__ __forceinline__ void cellsort_cell(const Dev& d, const Rep& R, int c,
         int rank = 0;
         for (int b = 0; b < n; ++b) rank += (d.timg[R.slot_base + d.bucket[R.slot_base + st + b]].w < id);
         d.perm[R.slot_base + st + rank] = old;
+        d.slot_of[R.slot_base + id] = st + rank;
       }
     }
   }
@@ -815,7 +821,6 @@ __device__ __forceinline__ void permute_chunk(const Dev& d, const Rep& R, int ci
   d.ref[s] = make_float4(p.x, p.y, p.z, __int_as_float(im.w));
   d.vel[s] = d.tvel[old];
   d.img[s] = im;
-  d.slot_of[R.slot_base + im.w] = local;
 }
 
 __global__ void __launch_bounds__(kChunk) k_permute(Dev d) {
@@ -882,13 +887,18 @@ __device__ int neighbors_small_box(const Dev& d, const Rep& R, int lc, int lane,
       const int il = hb + lane;
       const bool act = il < he;
       float4 pi = make_float4(0, 0, 0, 0);
-      int idi = -1;
-      int b0 = 0, b1 = 0;
+      // the bonded partners' ids, loaded once: looked up in memory at every
+      // hit they made a 500-bead replica's rebuild take 2.8 ms
+      int partner[kMaxBondsPerAtom];
+#pragma unroll
+      for (int b = 0; b < kMaxBondsPerAtom; ++b) partner[b] = -1;
       if (act) {
         pi = d.pos[base + il];
-        idi = d.img[base + il].w;
-        b0 = d.boff[base + idi];
-        b1 = d.boff[base + idi + 1];
+        const int idi = d.img[base + il].w;
+        const int b0 = d.boff[base + idi], nb = d.boff[base + idi + 1] - b0;
+#pragma unroll
+        for (int b = 0; b < kMaxBondsPerAtom; ++b)
+          if (b < nb) partner[b] = d.bent[R.bond_base + b0 + b].x;
       }
       int count = 0;
       uint32_t* out = d.nbr + R.nbr_base + ((size_t)(il >> 5) * M) * 32 + (il & 31);
@@ -909,13 +919,18 @@ __device__ int neighbors_small_box(const Dev& d, const Rep& R, int lc, int lane,
             for (int jb = ns; jb < ne; jb += 32) {
               const int jl = jb + lane;
               float4 pj = make_float4(0, 0, 0, 0);
-              if (jl < ne) pj = d.pos[base + jl];
+              int idl = -1;
+              if (jl < ne) {
+                pj = d.pos[base + jl];
+                idl = d.img[base + jl].w;
+              }
               const int m = min(32, ne - jb);
               for (int t = 0; t < m; ++t) {
                 const float jx = __shfl_sync(0xFFFFFFFFu, pj.x, t);
                 const float jy = __shfl_sync(0xFFFFFFFFu, pj.y, t);
                 const float jz = __shfl_sync(0xFFFFFFFFu, pj.z, t);
                 const float jw = __shfl_sync(0xFFFFFFFFu, pj.w, t);
+                const int idj = __shfl_sync(0xFFFFFFFFu, idl, t);
                 const int j = jb + t;
                 if (!act || j == il) continue;
                 int ex, ey, ez, kx, ky, kz;
@@ -933,9 +948,9 @@ __device__ int neighbors_small_box(const Dev& d, const Rep& R, int lc, int lane,
                     overflow |= kStatusCellCapacity;
                     continue;
                   }
-                  const int idj = d.img[base + j].w;
                   bool excl = false;
-                  for (int b = b0; b < b1; ++b) excl |= (d.bent[R.bond_base + b].x == idj);
+#pragma unroll
+                  for (int b = 0; b < kMaxBondsPerAtom; ++b) excl |= partner[b] == idj;
                   if (excl) continue;
                   if (count < M)
                     out[(size_t)count * 32] = (uint32_t)j | entry_code(ax, ay, az);
@@ -972,20 +987,20 @@ constexpr int kNbrGroup = 64;     // home atoms per pass
 
 // Shared staging of one home cell's list.
 constexpr int kNbrExcl = 1 + kMaxBondsPerAtom;  // the atom itself and its bonded partners
-template <int WIN, int WARPS>
+template <int WIN, int MASKS>
 struct ListStage {
   float4 c[WIN];                   // candidates of the window
   float4 hp[kNbrGroup];            // home atoms' positions
   int xk[kNbrGroup][kNbrExcl];     // and their excluded candidates (index, or -1)
-  uint32_t xm[WARPS][WIN / 32];    // per warp: excluded candidates of the window
+  uint32_t xm[MASKS][WIN / 32];    // per home atom in work: excluded candidates of the window
   int ns[27], off[28], cnt[kNbrGroup];
   float sx[27], sy[27], sz[27];
   uint32_t code[27];
 };
 
-template <int WIN, int WARPS>
+template <int WIN, int WARPS, int HOMES = 1>
 __device__ __forceinline__ void neighbors_cell_ballot(const Dev& d, const Rep& R, int* status, int lc,
-                                                      ListStage<WIN, WARPS>& st) {
+                                                      ListStage<WIN, WARPS * HOMES>& st) {
   const int G = R.G;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (G < 3) return;  // boxes under three cells per axis: k_neighbors_small
@@ -1008,7 +1023,7 @@ __device__ __forceinline__ void neighbors_cell_ballot(const Dev& d, const Rep& R
   auto &s_xk = st.xk;
   auto &s_xm = st.xm;
   constexpr int kExcl = kNbrExcl;
-  for (int k = threadIdx.x; k < WARPS * (WIN / 32); k += blockDim.x) (&s_xm[0][0])[k] = 0u;
+  for (int k = threadIdx.x; k < HOMES * WARPS * (WIN / 32); k += blockDim.x) (&s_xm[0][0])[k] = 0u;
   const int hx = lc % G, hy = (lc / G) % G, hz = lc / (G * G);
   if (warp == 0) {
     // the 27 cells (one lane each) and their candidate offsets (warp scan)
@@ -1106,46 +1121,67 @@ __device__ __forceinline__ void neighbors_cell_ballot(const Dev& d, const Rep& R
       const int wnp = (wn + 63) & ~63;
       for (int k = wn + threadIdx.x; k < wnp; k += blockDim.x) s_c[k] = make_float4(1e30f, 1e30f, 1e30f, 0.0f);
       __syncthreads();  // window (and home data) staged
-      for (int a = warp; a < gn; a += WARPS) {
-        const int i = hs + hg + a;
-        const float4 pi = s_hp[a];
-        // this atom's excluded candidates in the window, as bits
-        int xk = -1;
-        if (lane < kExcl) {
-          const int k = s_xk[a][lane] - w0;
-          if (k >= 0 && k < wn) {
-            xk = k;
-            atomicOr(&s_xm[warp][k >> 5], 1u << (k & 31));
+      for (int a0 = warp; a0 < gn; a0 += HOMES * WARPS) {
+        // HOMES home atoms against each candidate (their lists' orders are
+        // their own); lanes without a second atom repeat the first, unwritten
+        float4 pi[HOMES];
+        int xk[HOMES], count[HOMES];
+        uint32_t* out[HOMES];
+        bool live[HOMES];
+#pragma unroll
+        for (int u = 0; u < HOMES; ++u) {
+          const int a = a0 + u * WARPS;
+          live[u] = a < gn;
+          const int i = hs + hg + (live[u] ? a : a0);
+          pi[u] = s_hp[live[u] ? a : a0];
+          // this atom's excluded candidates in the window, as bits
+          xk[u] = -1;
+          if (live[u] && lane < kExcl) {
+            const int k = s_xk[a][lane] - w0;
+            if (k >= 0 && k < wn) {
+              xk[u] = k;
+              atomicOr(&s_xm[HOMES * warp + u][k >> 5], 1u << (k & 31));
+            }
           }
+          count[u] = w0 == 0 || !live[u] ? 0 : s_cnt[a];
+          out[u] = list + ((size_t)(i >> 5) * M) * 32 + (i & 31);
         }
         __syncwarp();
-        int count = w0 == 0 ? 0 : s_cnt[a];
-        uint32_t* out = list + ((size_t)(i >> 5) * M) * 32 + (i & 31);
 #pragma unroll 2
         for (int c0 = 0; c0 < wnp; c0 += 32) {
           const float4 c = s_c[c0 + lane];
-          const float rx = pi.x - c.x, ry = pi.y - c.y, rz = pi.z - c.z;
-          const float r2 = rx * rx + ry * ry + rz * rz;
-          const uint32_t m = __ballot_sync(0xFFFFFFFFu, r2 < rcs2) & ~s_xm[warp][c0 >> 5];
-          const int at = count + __popc(m & lt);
-          if (((m >> lane) & 1u) && at < M) __stcg(out + (size_t)at * 32, __float_as_uint(c.w));
-          count += __popc(m);
+#pragma unroll
+          for (int u = 0; u < HOMES; ++u) {
+            const float rx = pi[u].x - c.x, ry = pi[u].y - c.y, rz = pi[u].z - c.z;
+            const float r2 = rx * rx + ry * ry + rz * rz;
+            const uint32_t m = __ballot_sync(0xFFFFFFFFu, r2 < rcs2) & ~s_xm[HOMES * warp + u][c0 >> 5];
+            const int at = count[u] + __popc(m & lt);
+            if (((m >> lane) & 1u) && at < M && live[u]) __stcg(out[u] + (size_t)at * 32, __float_as_uint(c.w));
+            count[u] += __popc(m);
+          }
         }
         __syncwarp();
-        if (xk >= 0) s_xm[warp][xk >> 5] = 0u;
+#pragma unroll
+        for (int u = 0; u < HOMES; ++u)
+          if (xk[u] >= 0) s_xm[HOMES * warp + u][xk[u] >> 5] = 0u;
         __syncwarp();
-        if (w0 + WIN >= total) {
-          if (count <= M) {
-            const int padded = (count + kListPad - 1) & ~(kListPad - 1);
-            if (lane < padded - count)
-              __stcg(out + (size_t)(count + lane) * 32, (uint32_t)i | kPadBits);
+#pragma unroll
+        for (int u = 0; u < HOMES; ++u) {
+          if (!live[u]) continue;
+          const int a = a0 + u * WARPS, i = hs + hg + a;
+          if (w0 + WIN >= total) {
+            if (count[u] <= M) {
+              const int padded = (count[u] + kListPad - 1) & ~(kListPad - 1);
+              if (lane < padded - count[u])
+                __stcg(out[u] + (size_t)(count[u] + lane) * 32, (uint32_t)i | kPadBits);
+            }
+            if (lane == 0) {
+              d.ncnt[base + i] = min(count[u], M);
+              if (count[u] > M) overflow |= kStatusOverflow;
+            }
+          } else if (lane == 0) {
+            s_cnt[a] = count[u];
           }
-          if (lane == 0) {
-            d.ncnt[base + i] = min(count, M);
-            if (count > M) overflow |= kStatusOverflow;
-          }
-        } else if (lane == 0) {
-          s_cnt[a] = count;
         }
       }
     }
@@ -1307,7 +1343,7 @@ __global__ void __launch_bounds__(kNbrThreads, MINB) k_neighbors(Dev d) {
     if (V == 0) {
       __shared__ ListStage<kNbrWin, kNbrWarps> st;
       Rep& R = d.reps[rb_rep(d, cur.i)];
-      neighbors_cell_ballot(d, R, &R.status, item - cur.lo, st);
+      neighbors_cell_ballot<kNbrWin, kNbrWarps>(d, R, &R.status, item - cur.lo, st);
     } else
       neighbors_row(d, d.reps[rb_rep(d, cur.i)], item - cur.lo);
   }
@@ -2945,7 +2981,7 @@ __global__ void __launch_bounds__(kPostCommitThreads) k_post_commit(Dev d, int k
 // ---------------------------------------------------------------- resident steps
 // Many steps in one launch.  A replica is advanced by a group of resident
 // blocks (a cooperative launch), each owning a contiguous range of its
-// chunks; the group synchronises itself through flags in global memory, so
+// chunks; the group synchronises itself through a counter in global memory, so
 // replicas do not wait for one another and one replica's pre-force or rebuild
 // runs beside another's forces on the same SM.  Every block keeps a copy of
 // the replica's record in shared memory and commits each step on it (the same
@@ -2970,100 +3006,96 @@ __global__ void __launch_bounds__(kPostCommitThreads) k_post_commit(Dev d, int k
 constexpr int kStepWin = 704;       // list candidates staged per window: one 27-cell stencil of a melt
 constexpr int kStepSpin = 1 << 22;  // polls of a group barrier before the replica is given up (seconds)
 constexpr int kStepBlocksPerSM = 8;  // 64 registers
+constexpr int kStepHomes = 2;  // home atoms a warp lists at a time: a resident block is bound by latency
+constexpr int kStepFlags = kChunk;  // blocks of a group beside others up to which each polls every word
 constexpr int kStepKicks = 4;  // chunks whose post-force partials are staged at a time
-constexpr int kStepFlags = 128;  // blocks of a group up to which each polls every other's word
 
 // A resident block's shared memory besides the record: the stages of a step
 // use it in turn (small, so that the L1 keeps the rest of the array for the
 // position gathers).
 union StepStage {
-  ListStage<kStepWin, kChunk / 32> list;
+  ListStage<kStepWin, kStepHomes * kChunk / 32> list;
   struct {
     float4 shift[kShiftCodes];
     float axis[5];
   } force;
   double kick[kStepKicks][kChunk / 32][6];
-  double red[kPostCommitThreads / 32][13];
+  struct {
+    double chunk[6][kStepTileChunks];
+    double red[kPostCommitThreads / 32][13];
+  } sums;
 };
 
-// Relaxed polls (an acquire per poll would drop the SM's L1 lines each time);
-// a fence follows the last.
-__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long* p) {
-  unsigned long long v;
-  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
 __device__ __forceinline__ unsigned ld_relaxed(const unsigned* p) {
   unsigned v;
   asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
 __device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long long v) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+__device__ __forceinline__ void add_release(unsigned* p) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory");
 }
 
 // A replica's group of blocks within k_steps.
 struct StepGroup {
-  int r, rank, nb;            // replica, this block's rank, blocks
-  int a0, a1;                 // this block's slots (replica-local): pre-force, rebuild
-  int c0, c1;                 // its chunks: forces (QUADS: of energy steps), post-force partials
-  unsigned long long* flags;  // small groups: barrier number << 32 | value per block, two sets in turn
-  int stride;                 // from one set to the other
-  unsigned* count;            // larger ones: arrivals since the launch began, then three maxima in turn
-  unsigned seq;               // number of the last barrier, counted on from the launch before
-  unsigned nth;               // barriers of this launch
-  int* dead;                  // shared: a barrier ran out of polls
-  uint32_t* s_max;            // shared: per-warp maxima
+  int r, rank, nb;  // replica, this block's rank, blocks
+  int a0, a1;       // this block's slots (replica-local): pre-force, rebuild
+  int c0, c1;       // its chunks: forces (QUADS: of energy steps), post-force partials
+  bool alone;       // no other group in the grid
+  unsigned* count;  // arrivals since the launch began, then three maxima in turn
+  unsigned long long* flags;  // barrier number << 32 | value per block, two sets in turn (a small group beside others)
+  int stride;       // from one set to the other
+  unsigned nth;     // barriers of this launch
+  int* dead;        // shared: a barrier ran out of polls
+  uint32_t* s_max;  // shared: per-warp maxima
 };
 
 // Barrier over the group's blocks; memory written by them before it is
-// visible after it (the fence also drops this SM's stale L1 lines).  most: the
-// largest of the blocks' values (thread 0 in, thread 0 out).
+// visible after it (the acquire also drops this SM's stale L1 lines).  most:
+// the largest of the blocks' values (thread 0 in, thread 0 out).
 //
-// Up to kStepFlags blocks, each posts its number and value in a word of its
-// own and polls every block's: arrival and release are one store and one
-// load apart.  A block is at most one barrier ahead of another's reads, so
-// two sets of words are enough.  Larger groups count arrivals in one word
-// (polling every block's would be megabytes of loads per round) and take the
-// maximum in one of three, the one of two barriers ahead cleared by rank 0.
+// A group that has the grid to itself counts arrivals in one word, with
+// release and acquiring polls: 2,350 clocks for 94 blocks (each block polling
+// a word of every other took 4,900), 7,000 for 938 (40,000; arrivals spread
+// over 16 words were no faster).  The maximum is taken in one of three words,
+// the one of two barriers ahead cleared by rank 0.  Beside other groups an acquiring poll
+// would drop their L1 lines again and again: small groups there post the
+// barrier's number and the value in a word per block and poll those (a block
+// is at most one barrier ahead of another's reads: two sets of words), which
+// ran 64 uneven replicas 12 % faster per step than the shared counter.
 // False when the wait ran out: the replica is faulted and the block gives up.
 __device__ __forceinline__ bool group_sync(StepGroup& g, uint32_t value = 0u, uint32_t* most = nullptr) {
-  const unsigned seq = ++g.seq, nth = ++g.nth;
+  const unsigned nth = ++g.nth;
   __syncthreads();
-  uint32_t m = value;
-  if (g.nb > kStepFlags) {
+  if (!g.alone && g.nb > 1 && g.nb <= kStepFlags) {
+    unsigned long long* const f = g.flags + (nth & 1u) * g.stride;
+    uint32_t m = value;
     if (threadIdx.x == 0) {
-      unsigned* const top = g.count + 1;
-      if (most) atomicMax(top + nth % 3, value);
-      __threadfence();
-      atomicAdd(g.count, 1u);
-      for (int polls = 0; (int)(ld_relaxed(g.count) - nth * (unsigned)g.nb) < 0;)
-        if (++polls > kStepSpin) {
-          *g.dead = 1;
-          break;
-        }
-      __threadfence();
-      if (most) m = ld_relaxed(top + nth % 3);
-      if (g.rank == 0) top[(nth + 2) % 3] = 0u;
-    }
-    __syncthreads();
-  } else if (g.nb > 1) {
-    unsigned long long* const f = g.flags + (seq & 1u) * g.stride;
-    if (threadIdx.x == 0) {
-      __threadfence();
-      st_relaxed(f + g.rank, ((unsigned long long)seq << 32) | value);
+      fence_gpu();
+      st_relaxed(f + g.rank, ((unsigned long long)nth << 32) | value);
     }
     if ((int)(threadIdx.x & ~31u) < g.nb) {  // the warps that poll
       if ((int)threadIdx.x < g.nb) {
+        int polls = 0;
         unsigned long long w = ld_relaxed(f + threadIdx.x);
-        for (int polls = 0; (int)((unsigned)(w >> 32) - seq) < 0; w = ld_relaxed(f + threadIdx.x))
-          if (++polls > kStepSpin) {
-            *g.dead = 1;
-            break;
-          }
+        for (; (int)((unsigned)(w >> 32) - nth) < 0 && ++polls < kStepSpin; w = ld_relaxed(f + threadIdx.x)) {}
+        if (polls >= kStepSpin) *g.dead = 1;
         m = max(m, (uint32_t)w);
       }
-      __threadfence();
+      fence_gpu();
       if (most) {
         __syncwarp();
         warp_max_u32(m);
@@ -3071,10 +3103,29 @@ __device__ __forceinline__ bool group_sync(StepGroup& g, uint32_t value = 0u, ui
       }
     }
     __syncthreads();
-    if (most && threadIdx.x == 0)
+    if (most && threadIdx.x == 0) {
       for (int w = 0; w < kChunk / 32 && 32 * w < g.nb; ++w) m = max(m, g.s_max[w]);
+      *most = m;
+    }
+  } else if (g.nb > 1) {
+    if (threadIdx.x == 0) {
+      unsigned* const top = g.count + 1;
+      if (most) atomicMax(top + nth % 3, value);
+      add_release(g.count);
+      const unsigned all = nth * (unsigned)g.nb;
+      int polls = 0;
+      if (g.alone) {
+        while ((int)(ld_acquire(g.count) - all) < 0 && ++polls < kStepSpin) {}
+      } else {
+        while ((int)(ld_relaxed(g.count) - all) < 0 && ++polls < kStepSpin) {}
+        fence_gpu();
+      }
+      if (polls >= kStepSpin) *g.dead = 1;
+      if (most) *most = ld_relaxed(top + nth % 3);
+      if (g.rank == 0) top[(nth + 2) % 3] = 0u;
+    }
+    __syncthreads();
   }
-  if (most) *most = m;
   return *g.dead == 0;
 }
 
@@ -3143,16 +3194,17 @@ __device__ __noinline__ bool rebuild_group(const Dev& d, Rep& R, StepGroup& g, S
   const int ncell = R.P * R.P * R.P;
   for (int c = g.rank * W + warp; c < ncell; c += g.nb * W) cellsort_cell(d, R, c, lane);
   if (!group_sync(g)) return false;
-  for (int a = first; a < g.a1; a += kChunk) permute_chunk(d, R, 0, a);
-  if (!group_sync(g)) return false;
-  for (int a = first; a < g.a1; a += kChunk) topo_chunk(d, R, 0, a);
+  for (int a = first; a < g.a1; a += kChunk) {
+    permute_chunk(d, R, 0, a);
+    topo_chunk(d, R, 0, a);  // reads this thread's atom id and the new slots
+  }
   if (!group_sync(g)) return false;
   int* const status = &d.reps[g.r].status;
   const int home = R.G * R.G * R.G;
   for (int lc = g.rank; lc < home; lc += g.nb) {
     if (R.G >= 3) {
       __syncthreads();  // the previous cell's staging is no longer read
-      neighbors_cell_ballot(d, R, status, lc, st.list);
+      neighbors_cell_ballot<kStepWin, W, kStepHomes>(d, R, status, lc, st.list);
     } else {
       const int ov = neighbors_small_box(d, R, lc, lane, 32 * warp, kChunk);
       if (ov) atomicOr(status, ov);
@@ -3252,14 +3304,12 @@ __device__ __forceinline__ void kicks_tile(const Dev& d, const Rep& R, const Ste
     for (int q = 0; q < 6; ++q) tile_part[q] = vals[q];
 }
 
-// The replica's partials (values q0 .. 12) summed in k_post_commit's order:
-// thread t of its kPostCommitThreads adds chunks t, t + kPostCommitThreads,
-// ..., a shuffle tree per warp, then the warp totals in order.  tiles: the
-// KE values come from the group's tile sums (6 per tile), four to a chunk.
-__device__ __forceinline__ void reduce_partials(const Dev& d, const Rep& R, int q0, const double* tiles, int ntiles,
-                                                double (*s_red)[13], double* s_acc) {
+// The replica's partials summed in k_post_commit's order (thread t of its
+// kPostCommitThreads adds chunks t, t + kPostCommitThreads, ..., a shuffle
+// tree per warp, then the warp totals in order), by four warps.
+// From the chunk partials, values q0 .. 12.
+__device__ __forceinline__ void reduce_chunks(const Dev& d, const Rep& R, int q0, double (*s_red)[13]) {
   const int lane = threadIdx.x & 31;
-  constexpr int nw = kPostCommitThreads / 32;
   for (int vt = threadIdx.x; vt < kPostCommitThreads; vt += kChunk) {
     if (vt - lane >= R.nchunks) {  // warp-uniform: no chunks, zero totals
       if (lane < 13) s_red[vt >> 5][lane] = 0.0;
@@ -3268,31 +3318,53 @@ __device__ __forceinline__ void reduce_partials(const Dev& d, const Rep& R, int 
     double acc[13];
 #pragma unroll
     for (int q = 0; q < 13; ++q) acc[q] = 0.0;
-    for (int c = vt; c < R.nchunks; c += kPostCommitThreads) {
-      if (tiles) {
-        double t[6] = {0, 0, 0, 0, 0, 0};
-        for (int w = 4 * c; w < min(4 * c + 4, ntiles); ++w)
+    for (int c = vt; c < R.nchunks; c += kPostCommitThreads)
 #pragma unroll
-          for (int q = 0; q < 6; ++q) t[q] += tiles[6 * w + q];
-#pragma unroll
-        for (int q = 0; q < 6; ++q) acc[7 + q] += t[q];
-      } else {
-#pragma unroll
-        for (int q = 0; q < 13; ++q)
-          if (q >= q0) acc[q] += d.part[q * d.part_stride + R.chunk_base + c];
-      }
-    }
+      for (int q = 0; q < 13; ++q)
+        if (q >= q0) acc[q] += d.part[q * d.part_stride + R.chunk_base + c];
 #pragma unroll
     for (int q = 0; q < 13; ++q) {
       if (q >= q0) acc[q] = warp_sum(acc[q]);
       if (lane == 0) s_red[vt >> 5][q] = acc[q];
     }
   }
+}
+
+// The KE values (7 .. 12) from the group's tile sums (6 per tile, four tiles
+// to a chunk; at most kStepTileChunks chunks): the chunk sums through shared
+// memory, a (value, chunk) per thread, then a tree per 32 chunks and value.
+// (A thread per chunk with all values in registers took 19,000 clocks for
+// 188 chunks.)
+__device__ __forceinline__ void reduce_tiles(const Rep& R, const double* tiles, int ntiles,
+                                             double (*s_chunk)[kStepTileChunks], double (*s_red)[13]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll 2
+  for (int e = threadIdx.x; e < 6 * R.nchunks; e += kChunk) {
+    const int c = e / 6, q = e % 6;
+    double v[4];
+#pragma unroll
+    for (int w = 0; w < 4; ++w) v[w] = 4 * c + w < ntiles ? tiles[6 * (4 * c + w) + q] : 0.0;
+    s_chunk[q][c] = ((v[0] + v[1]) + v[2]) + v[3];
+  }
+  __syncthreads();
+  constexpr int nw = kPostCommitThreads / 32;
+#pragma unroll 3
+  for (int t = warp; t < nw * 6; t += kChunk / 32) {
+    const int vw = t / 6, q = t % 6, c = 32 * vw + lane;
+    const double x = 32 * vw < R.nchunks ? warp_sum(c < R.nchunks ? s_chunk[q][c] : 0.0) : 0.0;
+    if (lane == 0) s_red[vw][7 + q] = x;
+  }
+  if (threadIdx.x < nw)
+    for (int q = 0; q < 7; ++q) s_red[threadIdx.x][q] = 0.0;
+}
+
+// The warp totals in warp order.
+__device__ __forceinline__ void sum_totals(double (*s_red)[13], double* s_acc) {
   __syncthreads();
   if (threadIdx.x < 13) {
     double t = s_red[0][threadIdx.x];
 #pragma unroll
-    for (int w = 1; w < nw; ++w) t += s_red[w][threadIdx.x];
+    for (int w = 1; w < kPostCommitThreads / 32; ++w) t += s_red[w][threadIdx.x];
     s_acc[threadIdx.x] = t;
   }
   __syncthreads();
@@ -3300,7 +3372,7 @@ __device__ __forceinline__ void reduce_partials(const Dev& d, const Rep& R, int 
 
 template <int KB, bool QUADS, bool ST>
 __global__ void __launch_bounds__(kChunk, kStepBlocksPerSM)
-    k_steps(Dev d, const int4* plan, StepSync sync, unsigned seq, int max_steps) {
+    k_steps(Dev d, const int4* plan, StepSync sync, int max_steps) {
   constexpr int T = kChunk;
   __shared__ __align__(16) Rep R;
   __shared__ int dead;
@@ -3312,14 +3384,14 @@ __global__ void __launch_bounds__(kChunk, kStepBlocksPerSM)
   g.r = pl.x;
   g.rank = pl.y;
   g.nb = pl.z;
+  g.alone = (int)gridDim.x == pl.z;
+  g.count = sync.count + kStepCountWords * pl.x;
   g.flags = sync.flags + pl.w;
   g.stride = gridDim.x;
-  g.count = sync.count + kStepCountWords * pl.x;
-  g.seq = seq;
+  g.s_max = s_max;
   g.nth = 0;
   double* const tiles = sync.tiles + 6 * (size_t)pl.w;  // QUADS: the group's tile sums
   g.dead = &dead;
-  g.s_max = s_max;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   static_assert(sizeof(Rep) % 8 == 0, "the record is copied in 8-byte words");
   constexpr int kRepWords = (int)(sizeof(Rep) / 8);
@@ -3399,7 +3471,11 @@ __global__ void __launch_bounds__(kChunk, kStepBlocksPerSM)
       else
         kicks_group(d, R, g, st);
       if (!group_sync(g)) break;
-      reduce_partials(d, R, ev ? 0 : 7, by_tile ? tiles : nullptr, g.nb, st.red, s_acc);
+      if (by_tile)
+        reduce_tiles(R, tiles, g.nb, st.sums.chunk, st.sums.red);
+      else
+        reduce_chunks(d, R, ev ? 0 : 7, st.sums.red);
+      sum_totals(st.sums.red, s_acc);
       if (threadIdx.x == 0) post_commit_shared(R, s_acc);
       __syncthreads();
       if (g.rank == 0 && warp == 0 && stress_step(R)) acf_sample(d, R, g.r);
@@ -3539,7 +3615,7 @@ __global__ void __launch_bounds__(kNbrThreads) k_neighbors_g(Dev d) {
   const int G = R.G;
   if ((int)blockIdx.x >= G * G * G) return;
   __shared__ ListStage<kNbrWin, kNbrWarps> st;
-  neighbors_cell_ballot(d, R, &R.status, blockIdx.x, st);
+  neighbors_cell_ballot<kNbrWin, kNbrWarps>(d, R, &R.status, blockIdx.x, st);
 }
 
 // ---------------------------------------------------------------- launchers
@@ -3574,7 +3650,7 @@ void prefer_l1(K kernel, int pct = kForceCarveoutPct) {
 }
 
 namespace {
-using StepKernel = void (*)(Dev, const int4*, StepSync, unsigned, int);
+using StepKernel = void (*)(Dev, const int4*, StepSync, int);
 // form: 0 one lane per atom, 1 with the positions in shared memory, 2 QUADS
 StepKernel step_kernel(bool two, int form) {
   return form == 2 ? (two ? k_steps<2, true, false> : k_steps<1, true, false>)
@@ -3618,8 +3694,9 @@ int steps_resident_blocks(bool quads, int stage_bytes) {
 bool steps_variant(int force_variant) { return force_variant != 9 && force_variant != 10; }
 
 void launch_steps(const Dev& d, const int4* plan, int blocks, bool quads, int stage_bytes, const StepSync& sync,
-                  int nreps, unsigned seq, int force_variant, int max_steps, cudaStream_t st) {
-  FMD_CUDA(cudaMemsetAsync(sync.count, 0, sizeof(unsigned) * kStepCountWords * nreps, st));
+                  int force_variant, int max_steps, cudaStream_t st) {
+  // the barrier words are one range: counters, then the blocks' words
+  FMD_CUDA(cudaMemsetAsync(sync.count, 0, (char*)(sync.flags + 2 * blocks) - (char*)sync.count, st));
   const bool two = force_variant == 1 || force_variant == 3 || force_variant == 5;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = blocks;
@@ -3631,7 +3708,7 @@ void launch_steps(const Dev& d, const int4* plan, int blocks, bool quads, int st
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  FMD_CUDA(cudaLaunchKernelEx(&cfg, step_kernel(two, step_form(quads, stage_bytes)), d, plan, sync, seq, max_steps));
+  FMD_CUDA(cudaLaunchKernelEx(&cfg, step_kernel(two, step_form(quads, stage_bytes)), d, plan, sync, max_steps));
 }
 
 // The pre-force update of every chunk, one block per chunk.  (A resident
