@@ -20,12 +20,19 @@
 namespace fmd {
 namespace mixed {
 
-// Chunks per resident block up to which k_steps takes a batch, without and with
-// Nose-Hoover chains.  Measured per 200 steps, graph against resident: 200 x
-// 1,000 beads (2 chunks per block) 21.9 / 18.5 ms, 64 uneven replicas of
-// 342,000 beads in all (3) 40.4 / 27.1 ms, 64 x 30,000 (13) 100 / 131 ms --
-// the lines cross between 5 and 6; 16 x 30,000 NVT (4) 42.3 / 42.3 ms.
-constexpr int kResidentChunks = 5, kResidentChained = 3;
+// Chunks (128 atoms) up to which k_steps takes a batch with one lane per atom:
+// a fixed number and so many per replica, more with Nose-Hoover chains.  A
+// resident step takes about 0.054 us per chunk; a graph step about 60 us (100
+// with a chain's post-force kernels), 0.024 us per chunk and 1.2 us per replica
+// (its rebuilds follow one another).  Measured per step, graph against
+// resident: 64 uneven replicas of 342,000 beads in all (2,709 chunks) 202 /
+// 140 us, 200 x 1,000 beads 110 / 85, one replica of 100,000 (782) 65 / 58;
+// 30 x 15,000 (3,540) 182 / 194, 64 x 30,000 503 / 655.  NVT: 16 x 30,000
+// (3,760) 212 / 199, 20 x 15,000 168 / 144; one of 100,000, whose 782 blocks
+// meet twice a step, 80 / 82.  NPT evaluates energies every step: 8 x 40,000
+// 191 / 200, one of 100,000 97 / 100.
+constexpr int kResidentChunks = 2000, kResidentChained = 3300, kResidentPerReplica = 40;
+constexpr int kResidentPerBlock = 5;  // and at most this many chunks per block
 constexpr int kResidentSteps = 1000;  // steps per k_steps launch
 constexpr int kReadPiece = 32768;     // atoms per piece of a state readout (2 MB)
 
@@ -711,14 +718,14 @@ void Batch::check_status(int r, bool throw_on_fault) {
 
 // How k_steps takes the replicas for which runs(r) holds, if it does: with a
 // block per tile where all fit the GPU at once, else with the fewest chunks
-// per block for which every group does; beyond kResidentChunks of them the
-// graph's grids are the better form.
+// per block for which every group does, within the limits at the constants
+// above; beyond them the graph's grids are the better form.
 template <typename F>
 Batch::Resident Batch::resident_form(F runs) const {
   Resident f;
   int groups = 0, atoms = 0, most = 0;
   int64_t tiles = 0, chunks = 0;
-  bool chained = false;  // a Nose-Hoover chain: a second barrier and a reduction every step
+  bool chained = false, npt = false;
   for (int r = 0; r < max_reps_; ++r) {
     if (!runs(r)) continue;
     const Rep& R = h_reps_[r];
@@ -728,6 +735,7 @@ Batch::Resident Batch::resident_form(F runs) const {
     atoms = std::max(atoms, R.natoms);
     most = std::max(most, R.nchunks);
     chained |= R.mode == kModeRun && R.ensemble != FMD_LANGEVIN;
+    npt |= R.mode == kModeRun && R.ensemble == FMD_NPT_NH;
   }
   if (graph_steps_ <= 0 || groups == 0) return f;
   if (tiles <= steps_resident_blocks(true, 0) && most <= kStepTileChunks) {
@@ -737,7 +745,9 @@ Batch::Resident Batch::resident_form(F runs) const {
   const int64_t stage = ((int64_t)atoms * 16 + 1023) / 1024 * 1024;
   f.stage = stage <= kStepStageBytes ? (int)stage : 0;
   const int cap = steps_resident_blocks(false, f.stage);
-  if (groups > cap || chunks > (int64_t)(chained ? kResidentChained : kResidentChunks) * cap) return f;
+  const int64_t limit = (chained ? kResidentChained : kResidentChunks) + (int64_t)kResidentPerReplica * groups;
+  if (groups > cap || npt || (chained && groups == 1) || chunks > std::min<int64_t>(limit, kResidentPerBlock * cap))
+    return f;
   for (f.per_block = (int)((chunks + cap - 1) / cap); f.per_block < most; ++f.per_block) {
     int64_t blocks = 0;
     for (int r = 0; r < max_reps_; ++r)

@@ -3659,15 +3659,30 @@ StepKernel step_kernel(bool two, int form) {
 }
 int step_form(bool quads, int stage_bytes) { return quads ? 2 : stage_bytes > 0 ? 1 : 0; }
 
+// Per device: whether the kernels' attributes are set, and the event after the
+// last k_steps launch of any batch of the process.  Two cooperative grids that
+// each got part of the SMs would wait for one another, so a launch waits for
+// the one before it, whichever stream that is in.
+struct StepDevice {
+  bool attributes = false;
+  cudaEvent_t last = nullptr;
+};
+std::mutex g_step_mu;
+StepDevice g_step_dev[64];
+
+StepDevice& step_device() {
+  int dev = 0;
+  FMD_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) throw Error(FMD_ERR_ARG, "device ordinal out of range");
+  return g_step_dev[dev];
+}
+
 // Once per device: the carve-out that holds the kernels' shared memory as often
 // as a block fits an SM; the rest of the array is L1 for the gathers.
 void step_attributes() {
-  static std::mutex mu;
-  static bool done[256] = {};
-  int dev = 0;
-  FMD_CUDA(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lock(mu);
-  if (dev >= 0 && dev < 256 && done[dev]) return;
+  std::lock_guard<std::mutex> lock(g_step_mu);
+  StepDevice& sd = step_device();
+  if (sd.attributes) return;
   for (int form = 0; form < 3; ++form)
     for (bool two : {false, true}) {
       cudaFuncAttributes a;
@@ -3675,7 +3690,7 @@ void step_attributes() {
       const int kb = (int)((a.sharedSizeBytes + 1023) / 1024 + 1) * kStepBlocksPerSM;
       prefer_l1(step_kernel(two, form), form == 1 ? 100 : std::min(100, (100 * kb + 227) / 228));
     }
-  if (dev >= 0 && dev < 256) done[dev] = true;
+  sd.attributes = true;
 }
 }  // namespace
 
@@ -3708,7 +3723,12 @@ void launch_steps(const Dev& d, const int4* plan, int blocks, bool quads, int st
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
+  std::lock_guard<std::mutex> lock(g_step_mu);
+  StepDevice& sd = step_device();
+  if (!sd.last) FMD_CUDA(cudaEventCreateWithFlags(&sd.last, cudaEventDisableTiming));
+  FMD_CUDA(cudaStreamWaitEvent(st, sd.last, 0));
   FMD_CUDA(cudaLaunchKernelEx(&cfg, step_kernel(two, step_form(quads, stage_bytes)), d, plan, sync, max_steps));
+  FMD_CUDA(cudaEventRecord(sd.last, st));
 }
 
 // The pre-force update of every chunk, one block per chunk.  (A resident

@@ -70,6 +70,13 @@ def test_two_types_with_table_and_stress(tmp_path, ens):
     _same([conf], [_melt(10, 60, seed=5, type_block=10)], (11, 40))
 
 
+@pytest.mark.parametrize("ens", ["langevin", "nvt", "npt"])
+def test_step_graph(ens):
+    # a variant with two lanes per atom is not built in the resident form: the step graph
+    _same([run_conf(ensemble=ENS[ens], nsteps=10_000)] * 2, [_melt(12, 50, seed=6), _melt(3, 43, seed=3)], (60, 45),
+          variant=9)
+
+
 def test_push_off():
     melt = fm.generate_melt(10, 50, density=0.85, seed=9)
     _same([run_conf()], [melt], (1, 5),
