@@ -21,20 +21,20 @@ namespace fmd {
 namespace mixed {
 
 // Chunks (128 atoms) up to which k_steps takes a batch with one lane per atom:
-// a fixed number and so many per replica, more with Nose-Hoover chains.  A
-// resident step takes about 0.054 us per chunk; a graph step about 60 us (100
-// with a chain's post-force kernels), 0.024 us per chunk and 1.2 us per replica
+// a fixed number and so many per replica.  A resident step takes about 0.054 us
+// per chunk (0.060 with Nose-Hoover chains); a graph step about 60 us (100 with
+// the chains' post-force kernels), 0.024 us per chunk and 1.2 us per replica
 // (its rebuilds follow one another).  Measured per step, graph against
 // resident: 64 uneven replicas of 342,000 beads in all (2,709 chunks) 202 /
 // 140 us, 200 x 1,000 beads 110 / 85, one replica of 100,000 (782) 65 / 58;
-// 30 x 15,000 (3,540) 182 / 194, 64 x 30,000 503 / 655.  NVT: 16 x 30,000
-// (3,760) 212 / 199, 20 x 15,000 168 / 144; one of 100,000, whose 782 blocks
-// meet twice a step, 80 / 82.  NPT evaluates energies every step: 8 x 40,000
-// 191 / 200, one of 100,000 97 / 100.
-constexpr int kResidentChunks = 2000, kResidentChained = 3300, kResidentPerReplica = 40;
+// 30 x 15,000 (3,540) 181 / 194, 64 x 30,000 503 / 655.  NVT: 20 x 15,000
+// (2,360) 168 / 144, 16 x 30,000 (3,760) 198 / 225; one of 100,000, whose 782
+// blocks meet twice a step, 80 / 82.  NPT evaluates energies every step: 8 x
+// 40,000 187 / 200, one of 100,000 97 / 100.
+constexpr int kResidentChunks = 2000, kResidentPerReplica = 40;
 constexpr int kResidentPerBlock = 5;  // and at most this many chunks per block
 constexpr int kResidentSteps = 1000;  // steps per k_steps launch
-constexpr int kReadPiece = 32768;     // atoms per piece of a state readout (2 MB)
+constexpr int kReadPiece = 8192;      // atoms per piece of a state readout (480 KB)
 
 // ------------------------------------------------------------- allocator
 int64_t SegAlloc::alloc(int64_t n) {
@@ -745,7 +745,7 @@ Batch::Resident Batch::resident_form(F runs) const {
   const int64_t stage = ((int64_t)atoms * 16 + 1023) / 1024 * 1024;
   f.stage = stage <= kStepStageBytes ? (int)stage : 0;
   const int cap = steps_resident_blocks(false, f.stage);
-  const int64_t limit = (chained ? kResidentChained : kResidentChunks) + (int64_t)kResidentPerReplica * groups;
+  const int64_t limit = kResidentChunks + (int64_t)kResidentPerReplica * groups;
   if (groups > cap || npt || (chained && groups == 1) || chunks > std::min<int64_t>(limit, kResidentPerBlock * cap))
     return f;
   for (f.per_block = (int)((chunks + cap - 1) / cap); f.per_block < most; ++f.per_block) {
@@ -1177,10 +1177,15 @@ void Batch::force_frame(int r, double* xyz, double* box) {
 // (k_read_state): while one piece is copied into the caller's arrays the next
 // crosses the bus.
 void Batch::read_state(int r, double* xyz, double* vel, int32_t* image, bool rewrap) {
-  const int n = rep(r).natoms, piece = std::min(n, kReadPiece);
-  const size_t bytes = (size_t)piece * kReadBytes;
+  const int n = rep(r).natoms, piece = kReadPiece;
   const int pieces = (n + piece - 1) / piece;
-  for (int k = 0; k < std::min(2, pieces); ++k) {
+  // sized for the batch's largest replica, so that reading one after another
+  // allocates once
+  int largest = 0;
+  for (int k = 0; k < max_reps_; ++k)
+    if (info_[k].used) largest = std::max(largest, h_reps_[k].natoms);
+  const size_t bytes = (size_t)std::min(largest, piece) * kReadBytes;
+  for (int k = 0; k < std::min(2, (largest + piece - 1) / piece); ++k) {
     if (read_dev_[k].n < bytes) {
       FMD_CUDA(cudaStreamSynchronize(st_));
       read_dev_[k].alloc(bytes);

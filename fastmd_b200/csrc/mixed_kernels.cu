@@ -20,6 +20,8 @@
 //                and runs the post-force thermostat / barostat.  Langevin
 //                steps inside a graph fold the final half kick into the next
 //                k_pre instead (same operations, same order).
+//   k_steps      small and medium batches: all of the above for many steps in
+//                one launch, a group of resident blocks per replica.
 // Reference algorithm sources: integrate/langevin.cu:34-130,
 // integrate/nose_hoover.cu:86-305, 606-898, force/lj.cu:21-65,
 // force/fene.cu:18-73, force/angle.cu:17-80, neighbor/verlet_list.cu:108-335,

@@ -4,9 +4,11 @@
 // reference's structure on purpose:
 //   - per-atom full Verlet list in the transposed layout neighbors[k*N + i]
 //     built from a cell list with cell edge >= rc + skin (verlet_list.cu:3-376);
-//   - thread-per-atom LJ (lj.cu:4-107), thread-per-bond FENE and
-//     thread-per-angle kernels with atomic scatter (fene.cu:4-101, angle.cu:4-108);
-//   - host-side rebuild test every step (skin_trigger.cuh:18-33, main.cu:484-528).
+//   - LJ over the list (lj.cu:4-107), several lanes per atom in small systems,
+//     thread-per-bond FENE and thread-per-angle terms with atomic scatter in
+//     one launch (fene.cu:4-101, angle.cu:4-108);
+//   - host-side rebuild test every step (skin_trigger.cuh:18-33, main.cu:484-528),
+//     with the forces queued on the list in use while the host waits.
 // Differences from the reference: FP64 throughout; the Philox noise of
 // counter_rng.h instead of cuRAND state; neighbor overflow and FENE
 // over-stretch are reported instead of silently truncated / clamped; the cell

@@ -325,7 +325,8 @@ FMD_API fmd_status fmd_batch_totals(fmd_batch* b, int32_t* active, int64_t* atom
  * the device (a graph step skips the rebuild kernels and a force variant no
  * replica needs): counts[0..12] = pre-force, bin, scan, scatter, cell sort,
  * permute, bonded tables, neighbor list, force, force with energies,
- * post-force, rebuild planning, per-replica commits; n = entries to fill. */
+ * post-force, rebuild planning, per-replica commits; n = entries to fill.
+ * A launch that advances a small batch by many steps counts once, as force. */
 FMD_API fmd_status fmd_batch_mark(fmd_batch* b, int32_t which);
 FMD_API fmd_status fmd_batch_elapsed_ms(fmd_batch* b, double* ms);
 FMD_API fmd_status fmd_batch_time_force(fmd_batch* b, int32_t iters, double* ms_per_launch);

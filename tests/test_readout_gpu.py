@@ -1,4 +1,4 @@
-"""State readout at the edges of its pieces (32,768 atoms) and blocks: positions, velocities and image flags come
+"""State readout at the edges of its pieces (8,192 atoms) and blocks: positions, velocities and image flags come
 back in the order given.  Tolerance: a position is an FP32 offset in a cell edge below 8 sigma, so it is off by at
 most half an ulp of that, 2.4e-7, and the FP64 additions around it."""
 import numpy as np
@@ -10,7 +10,7 @@ from tests.util import run_conf
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [1, 255, 257, 32767, 32768, 32769, 65537])
+@pytest.mark.parametrize("n", [1, 255, 257, 8191, 8192, 8193, 16385, 32769])
 def test_state_reads_back_in_the_order_given(n):
     rng = np.random.default_rng(n)
     m = int(np.ceil(n ** (1 / 3) - 1e-9))
