@@ -9,7 +9,8 @@
 // lanes test 32 candidates and a ballot compacts the hits in candidate order.
 // The thread-per-atom form it stands beside follows two dependent loads per
 // candidate (sorted index -> position) and was bound by their latency: 100,000
-// atoms, rc + skin 2.8 at density 0.85, 212 us.  It remains where cells are
+// atoms, rc + skin 2.8 at density 0.85, 212 us against 115 (now bound by issue,
+// 71 % active).  It remains where cells are
 // mostly empty (list_by_cells): there a block per cell would find nothing to do.
 #pragma once
 #include <cuda_runtime.h>
