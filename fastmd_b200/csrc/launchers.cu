@@ -75,7 +75,8 @@ struct VerletScratch {
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // The sort's input and temporary storage come last: once it is done the
-// positions in sorted order take their place.
+// positions in sorted order take their place, at the next 16-byte boundary (a
+// caller's scratch need only be aligned for int; the size holds the gap).
 VerletScratch verlet_carve(void* base, int n, int ncell) {
   VerletScratch s{};
   size_t cub_bytes = 0;
@@ -96,8 +97,9 @@ VerletScratch verlet_carve(void* base, int n, int ncell) {
   s.aid = (int*)take(sizeof(int) * n);
   s.cub = take(cub_bytes);
   s.cub_bytes = cub_bytes;
-  s.spos = p ? (float4*)(p + reuse) : nullptr;
-  s.total = std::max(off, reuse + align256(sizeof(float4) * n));
+  const size_t gap = (size_t)(-(intptr_t)(p + reuse)) % sizeof(float4);
+  s.spos = p ? (float4*)(p + reuse + gap) : nullptr;
+  s.total = std::max(off, reuse + align256(sizeof(float4) * (n + 1)));
   return s;
 }
 

@@ -463,7 +463,7 @@ FMD_API fmd_status fmd_server_pool_destroy(fmd_server_pool* p);
  * CSR of build_exclusions (lammps_data.cpp:231-253), or NULL.  Unlike the
  * reference, an overflow is reported (FMD_ERR_OVERFLOW after the stream is
  * synchronized when sync != 0) instead of truncated silently.
- * scratch: device memory of fmd_verlet_scratch_bytes() bytes. */
+ * scratch: device memory of fmd_verlet_scratch_bytes() bytes, 4-byte aligned. */
 FMD_API fmd_status fmd_verlet_scratch_bytes(int32_t natoms, float rc_skin, float box_L, size_t* bytes);
 FMD_API fmd_status fmd_launch_verlet_build(const void* pos, int32_t natoms, float box_L,
                                            const int32_t* exclusion_offsets, const int32_t* exclusion_list,
