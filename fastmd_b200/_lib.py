@@ -543,6 +543,10 @@ class Batch:
         _call("fmd_batch_get_variants", self._h, C.byref(a), C.byref(b), C.byref(c), C.byref(d))
         return a.value, b.value, c.value, d.value
 
+    def set_wait_limit(self, polls):
+        """Polls after which a block of a many-step launch gives its replica up (4,194,304 by default)."""
+        _call("fmd_batch_set_wait_limit", self._h, C.c_int32(polls))
+
     def last_forces(self, slot):
         """Forces of the last evaluation as stored (FP32 values, id order), not re-evaluated."""
         f = np.zeros((self._natoms[slot], 3))

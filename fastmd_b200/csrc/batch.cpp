@@ -620,6 +620,7 @@ void Batch::finish_pushoffs() {
   advance(steps);
   FMD_CUDA(cudaStreamSynchronize(st_));
   download_reps();
+  clear_expired();
   complete_pushoffs(pend);
 }
 
@@ -708,6 +709,7 @@ void Batch::check_status(int r, bool throw_on_fault) {
   const Rep& R = h_reps_[r];
   if (R.status == 0) return;
   if (!throw_on_fault) return;
+  if (R.status & kStatusTimeout) throw Error(FMD_ERR_FAULT, "a bounded device wait expired");
   if (R.status & kStatusOverflow) throw Error(FMD_ERR_OVERFLOW, "neighbor list overflow");
   if (R.status & kStatusCellCapacity) throw Error(FMD_ERR_OVERFLOW, "cell grid capacity exceeded");
   if (R.status & kStatusNonFinite) throw Error(FMD_ERR_FAULT, "non-finite state");
@@ -791,11 +793,28 @@ bool Batch::plan_resident() {
   return true;
 }
 
+// Replicas given up by k_steps stop here: their blocks left it at different
+// steps, some perhaps between a rebuild's binning and its scan.  The cell
+// counts such a rebuild leaves behind are cleared, so that a later rebuild
+// indexes within the replica's slots.
+bool Batch::clear_expired() {
+  bool any = false;
+  for (int r = 0; r < max_reps_; ++r) {
+    Rep& R = h_reps_[r];
+    if (!info_[r].used || !R.active || !(R.status & kStatusTimeout)) continue;
+    FMD_CUDA(cudaMemsetAsync(cell_cnt_.p + R.cell_base, 0, (size_t)info_[r].plan.ncell * sizeof(int32_t), st_));
+    R.active = 0;
+    any = true;
+  }
+  return any;
+}
+
 // Queue nsteps steps (each replica stops at its own stop_step, as uploaded).
 void Batch::advance(int64_t nsteps) {
   const Dev d = dev();
   if (plan_resident()) {
-    const StepSync sync{reinterpret_cast<unsigned*>(sync_.p), sync_.p + (size_t)max_reps_ * kStepCountWords / 2, tiles_};
+    const StepSync sync{reinterpret_cast<unsigned*>(sync_.p), sync_.p + (size_t)max_reps_ * kStepCountWords / 2, tiles_,
+                        step_polls_};
     while (nsteps > 0) {
       const int k = (int)std::min<int64_t>(nsteps, kResidentSteps);
       launch_steps(d, plan_, (int)h_plan_.size(), resident_.quads, resident_.stage, sync, force_variant_, k, st_);
@@ -873,9 +892,9 @@ void Batch::run(int64_t nsteps, bool respect_nsteps) {
   advance(need);
   FMD_CUDA(cudaStreamSynchronize(st_));
   download_reps();
-  if (concurrent_pushoff_) complete_done_pushoffs();
   // A faulted replica stops; the others continue.
-  bool changed = false;
+  bool changed = clear_expired();
+  if (concurrent_pushoff_) complete_done_pushoffs();
   for (int r = 0; r < max_reps_; ++r) {
     if (!info_[r].used) continue;
     Rep& R = h_reps_[r];
@@ -1057,6 +1076,11 @@ void Batch::set_variants(int fv, int nv) {
     nbr_variant_ = nv;
     graph_dirty_ = true;
   }
+}
+
+void Batch::set_wait_limit(int polls) {
+  if (polls < 0 || polls > kStepPolls) throw Error(FMD_ERR_ARG, "wait limit out of range");
+  step_polls_ = polls;
 }
 
 void Batch::last_forces(int r, double* f) {

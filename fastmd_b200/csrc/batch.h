@@ -123,6 +123,8 @@ class Batch {
   int force_variant() const { return force_variant_; }
   // Force / neighbor-list kernel variants for the following steps (< 0: keep).
   void set_variants(int force_variant, int nbr_variant);
+  // Polls of a resident step's group barrier before its replica is given up.
+  void set_wait_limit(int polls);
   // Forces of the last evaluation as stored (no re-evaluation), id order.
   void last_forces(int r, double* f);
   void list_stats(int64_t* entries, int32_t* max_per_atom);
@@ -144,6 +146,7 @@ class Batch {
   template <typename F>
   Resident resident_form(F runs) const;
   bool plan_resident();
+  bool clear_expired();
   void ensure_graph();
 
   int device_ = 0;
@@ -180,6 +183,7 @@ class Batch {
   DevBuf<unsigned long long> sync_;  // resident steps: barrier words per replica and block,
   DevBuf<double> tiles_;             // and tile sums
   Resident resident_;       // form of the plan
+  int step_polls_ = kStepPolls;  // of a group barrier
   std::vector<int4> h_plan_, new_plan_;
   // state readout: two device and two pinned buffers of a piece of atoms each
   DevBuf<char> read_dev_[2];

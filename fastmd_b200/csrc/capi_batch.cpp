@@ -310,6 +310,10 @@ FMD_API fmd_status fmd_batch_set_variants(fmd_batch* b, int32_t force_variant, i
   return guarded([&] { B(b).set_variants(force_variant, nbr_variant); });
 }
 
+FMD_API fmd_status fmd_batch_set_wait_limit(fmd_batch* b, int32_t polls) {
+  return guarded([&] { B(b).set_wait_limit(polls); });
+}
+
 FMD_API fmd_status fmd_batch_get_variants(fmd_batch* b, int32_t* force_variant, int32_t* nbr_variant,
                                           int32_t* n_force, int32_t* n_nbr) {
   return guarded([&] {

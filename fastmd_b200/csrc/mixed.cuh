@@ -376,7 +376,9 @@ struct StepSync {
   unsigned* count;  // kStepCountWords per replica
   unsigned long long* flags;  // 2 per block, behind count in one allocation
   double* tiles;    // 6 per block
+  int polls;        // of a group barrier before the replica is given up
 };
+constexpr int kStepPolls = 1 << 22;  // seconds
 // Tiles that hold a replica's atoms, and the first of each of its chunks.
 inline int step_tiles(int natoms, int nchunks) {
   const int t = (natoms + kTile - 1) / kTile, c = (kChunk / kTile) * (nchunks - 1) + 1;

@@ -3006,7 +3006,9 @@ __global__ void __launch_bounds__(kPostCommitThreads) k_post_commit(Dev d, int k
 // SMs without work on 3,000 beads: 18,500 clocks per force evaluation, bound
 // by issue on the 24 SMs in use.)
 constexpr int kStepWin = 704;       // list candidates staged per window: one 27-cell stencil of a melt
-constexpr int kStepSpin = 1 << 22;  // polls of a group barrier before the replica is given up (seconds)
+// The first barrier of a launch also waits for the group's blocks to be given
+// their SMs, which other streams' kernels may hold: this many times the limit.
+constexpr int kStepFirstWait = 64;
 constexpr int kStepBlocksPerSM = 8;  // 64 registers
 constexpr int kStepHomes = 2;  // home atoms a warp lists at a time: a resident block is bound by latency
 constexpr int kStepFlags = kChunk;  // blocks of a group beside others up to which each polls every word
@@ -3061,6 +3063,7 @@ struct StepGroup {
   unsigned long long* flags;  // barrier number << 32 | value per block, two sets in turn (a small group beside others)
   int stride;       // from one set to the other
   unsigned nth;     // barriers of this launch
+  int polls;        // of a barrier before the replica is given up
   int* dead;        // shared: a barrier ran out of polls
   uint32_t* s_max;  // shared: per-warp maxima
 };
@@ -3078,9 +3081,13 @@ struct StepGroup {
 // barrier's number and the value in a word per block and poll those (a block
 // is at most one barrier ahead of another's reads: two sets of words), which
 // ran 64 uneven replicas 12 % faster per step than the shared counter.
-// False when the wait ran out: the replica is faulted and the block gives up.
+// False when the wait ran out: the replica is faulted and the block gives up;
+// the group's other blocks run out at their next barrier at the latest.  What
+// a block does between two barriers uses only what was complete at the first,
+// so it stays within the replica's arrays.
 __device__ __forceinline__ bool group_sync(StepGroup& g, uint32_t value = 0u, uint32_t* most = nullptr) {
   const unsigned nth = ++g.nth;
+  const int limit = nth == 1 ? g.polls * kStepFirstWait : g.polls;
   __syncthreads();
   if (!g.alone && g.nb > 1 && g.nb <= kStepFlags) {
     unsigned long long* const f = g.flags + (nth & 1u) * g.stride;
@@ -3093,8 +3100,8 @@ __device__ __forceinline__ bool group_sync(StepGroup& g, uint32_t value = 0u, ui
       if ((int)threadIdx.x < g.nb) {
         int polls = 0;
         unsigned long long w = ld_relaxed(f + threadIdx.x);
-        for (; (int)((unsigned)(w >> 32) - nth) < 0 && ++polls < kStepSpin; w = ld_relaxed(f + threadIdx.x)) {}
-        if (polls >= kStepSpin) *g.dead = 1;
+        for (; (int)((unsigned)(w >> 32) - nth) < 0 && ++polls < limit; w = ld_relaxed(f + threadIdx.x)) {}
+        if (polls >= limit) *g.dead = 1;
         m = max(m, (uint32_t)w);
       }
       fence_gpu();
@@ -3117,12 +3124,12 @@ __device__ __forceinline__ bool group_sync(StepGroup& g, uint32_t value = 0u, ui
       const unsigned all = nth * (unsigned)g.nb;
       int polls = 0;
       if (g.alone) {
-        while ((int)(ld_acquire(g.count) - all) < 0 && ++polls < kStepSpin) {}
+        while ((int)(ld_acquire(g.count) - all) < 0 && ++polls < limit) {}
       } else {
-        while ((int)(ld_relaxed(g.count) - all) < 0 && ++polls < kStepSpin) {}
+        while ((int)(ld_relaxed(g.count) - all) < 0 && ++polls < limit) {}
         fence_gpu();
       }
-      if (polls >= kStepSpin) *g.dead = 1;
+      if (polls >= limit) *g.dead = 1;
       if (most) *most = ld_relaxed(top + nth % 3);
       if (g.rank == 0) top[(nth + 2) % 3] = 0u;
     }
@@ -3392,6 +3399,7 @@ __global__ void __launch_bounds__(kChunk, kStepBlocksPerSM)
   g.stride = gridDim.x;
   g.s_max = s_max;
   g.nth = 0;
+  g.polls = sync.polls;
   double* const tiles = sync.tiles + 6 * (size_t)pl.w;  // QUADS: the group's tile sums
   g.dead = &dead;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -3420,6 +3428,7 @@ __global__ void __launch_bounds__(kChunk, kStepBlocksPerSM)
   const int64_t left = R.active ? R.stop_step - R.step : 0;
   const int steps = (int)(left < max_steps ? left : max_steps);
   if (steps <= 0) return;  // the same in every block of the group
+  if (R.status & kStatusTimeout) return;  // given up in an earlier launch: its blocks stopped at different steps
   if (!R.next_valid) {
     if (g.rank == 0 && threadIdx.x == 0) atomicOr(&d.reps[g.r].status, kStatusStaleScalars);
     return;

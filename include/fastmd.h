@@ -263,7 +263,8 @@ typedef struct fmd_replica_info {
   int32_t natoms;
   int64_t step;
   int64_t nsteps;          /* run.conf nsteps (target) */
-  int32_t status_word;     /* 0 healthy; bits: 1 overflow, 2 non-finite, 4 FENE overstretch, 8 cell capacity */
+  int32_t status_word;     /* 0 healthy; bits: 1 overflow, 2 non-finite, 4 FENE overstretch, 8 cell capacity,
+                              16 a bounded device wait expired */
   int32_t active;
   double box_L;
   int64_t rebuilds;
@@ -384,6 +385,10 @@ FMD_API fmd_status fmd_batch_set_rebuild_cadence(fmd_batch* b, int32_t slot, int
 FMD_API fmd_status fmd_batch_set_variants(fmd_batch* b, int32_t force_variant, int32_t nbr_variant);
 FMD_API fmd_status fmd_batch_get_variants(fmd_batch* b, int32_t* force_variant, int32_t* nbr_variant,
                                           int32_t* n_force, int32_t* n_nbr);
+/* How often a block of a batch advanced by many steps in one launch polls for
+ * the other blocks of its replica before it gives the replica up (a fault of
+ * that replica alone: status bit 16).  0 to 4,194,304, the default (seconds). */
+FMD_API fmd_status fmd_batch_set_wait_limit(fmd_batch* b, int32_t polls);
 /* Forces of the replica's last force evaluation as stored on the device (FP32
  * values, id order), without re-evaluating them: after a step these are the
  * forces the kernel flavour of that step produced at the positions of
