@@ -33,6 +33,18 @@ namespace mixed {
 // 40,000 187 / 200, one of 100,000 97 / 100.
 constexpr int kResidentChunks = 2000, kResidentPerReplica = 40;
 constexpr int kResidentPerBlock = 5;  // and at most this many chunks per block
+// A resident rebuild walks the replica's home cells, empty ones too, with its
+// own blocks, and one of them scans its P^3 sort cells; the graph's rebuild has
+// the whole GPU.  Measured per step of Langevin chains of ten, graph against
+// resident (home cells per block in brackets): a block per tile, 3,000 beads at
+// density 0.01 33 / 25 us (129), at 0.005 34 / 37 (287), at 0.002 (P = 64) 41 /
+// 102; 12,000 at 0.02 35 / 24 (72), at 0.01 (P = 64) 41 / 55; 8 x 3,000 at 0.01
+// 45 / 40 (129), at 0.005 53 / 54 (287).  Chunks shared by blocks, 60,000 beads
+// at 0.1 41 / 37 (57), at 0.05 (P = 64) 47 / 67; 64 x 1,000 at 0.05 49 / 42 (91),
+// at 0.02 56 / 61 (274); 64 x 3,000 at 0.1 71 / 67 (111), 20 x 10,000 at 0.1
+// 65 / 70 (102).  A melt at 0.85 has at most 6 per chunk of a block.
+constexpr int kResidentAxis = 32;  // sort cells per axis
+constexpr int kTileCells = 200, kBlockCells = 100;  // home cells per block
 constexpr int kResidentSteps = 1000;  // steps per k_steps launch
 constexpr int kReadPiece = 8192;      // atoms per piece of a state readout (480 KB)
 
@@ -740,8 +752,19 @@ Batch::Resident Batch::resident_form(F runs) const {
     npt |= R.mode == kModeRun && R.ensemble == FMD_NPT_NH;
   }
   if (graph_steps_ <= 0 || groups == 0) return f;
+  auto few_cells = [&](int per_block) {  // of every replica, for so many chunks per block (0: a tile)
+    for (int r = 0; r < max_reps_; ++r) {
+      if (!runs(r)) continue;
+      const Rep& R = h_reps_[r];
+      const int64_t home = (int64_t)R.G * R.G * R.G;
+      const int64_t room = per_block ? (int64_t)kBlockCells * ((R.nchunks + per_block - 1) / per_block)
+                                     : (int64_t)kTileCells * step_tiles(R.natoms, R.nchunks);
+      if (R.P > kResidentAxis || home > room) return false;
+    }
+    return true;
+  };
   if (tiles <= steps_resident_blocks(true, 0) && most <= kStepTileChunks) {
-    f.fits = f.quads = true;
+    f.fits = f.quads = few_cells(0);
     return f;
   }
   const int64_t stage = ((int64_t)atoms * 16 + 1023) / 1024 * 1024;
@@ -756,7 +779,7 @@ Batch::Resident Batch::resident_form(F runs) const {
       if (runs(r)) blocks += (h_reps_[r].nchunks + f.per_block - 1) / f.per_block;
     if (blocks <= cap) break;
   }
-  f.fits = true;
+  f.fits = few_cells(f.per_block);
   return f;
 }
 
