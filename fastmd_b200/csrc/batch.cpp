@@ -20,17 +20,36 @@
 namespace fmd {
 namespace mixed {
 
-// Chunks (128 atoms) up to which k_steps takes a batch with one lane per atom:
-// a fixed number and so many per replica.  A resident step takes about 0.054 us
-// per chunk (0.060 with Nose-Hoover chains); a graph step about 60 us (100 with
-// the chains' post-force kernels), 0.024 us per chunk and 1.2 us per replica
-// (its rebuilds follow one another).  Measured per step, graph against
-// resident: 64 uneven replicas of 342,000 beads in all (2,709 chunks) 202 /
-// 140 us, 200 x 1,000 beads 110 / 85, one replica of 100,000 (782) 65 / 58;
-// 30 x 15,000 (3,540) 181 / 194, 64 x 30,000 503 / 655.  NVT: 20 x 15,000
-// (2,360) 168 / 144, 16 x 30,000 (3,760) 198 / 225; one of 100,000, whose 782
-// blocks meet twice a step, 80 / 82.  NPT evaluates energies every step: 8 x
-// 40,000 187 / 200, one of 100,000 97 / 100.
+// Limits up to which k_steps takes a batch with one lane per atom.  A graph
+// step takes about 40 us (60 with Nose-Hoover chains) and 0.037 us per chunk
+// (128 atoms) of the batch, and up to 40 us more where the replicas' rebuilds
+// fall on different steps: each such step then waits for a rebuild's kernels.
+// A resident step takes 7 to 9 us per chunk on the SM that has the most (its
+// load: blocks per SM, rounded up, times chunks per block) and hides a
+// replica's rebuild behind the others' forces, so the balance decides.  251
+// batches were measured in both forms, untuned and autotuned (which lifts the
+// forced rebuild cadence that keeps replicas in step).  Per step, graph against
+// resident, load in brackets:
+//   one replica of 130,000 beads 71 / 68 (7), of 160,000 88 / 94 (10);
+//   over 100 chunks each: 3 x 60,000 95 / 92 (10), 8 x 25,000 98 / 104 (12);
+//   over 13: 20 x 10,000 101 / 98 (12), 80 x 3,500 124 / 112 (16), 120 x 2,400
+//   125 / 130 (18), 45 x 7,000 133 / 139 (18), 90 x 7,250 220 / 259 (40);
+//   smaller: 200 x 1,000 111 / 86 (15), 400 x 600 119 / 106 (18), 500 x 600
+//   138 / 114 (21), 600 x 600 155 / 165 (25), 450 x 1,000 186 / 264 (32); with
+//   chains 160 x 2,400 182 / 168 (24), 600 x 600 206 / 179 (25), 250 x 1,500
+//   180 / 211 (24, six chunks per block), 450 x 1,000 234 / 282 (32);
+//   rebuilds apart: 15 x 13,629 133 / 99 (12), 64 uneven replicas of 342,000
+//   beads in all 184 / 139 (21), 64 x 7,797 180 / 163 (28); with chains
+//   15 uneven of 228,000 136 / 110 (14), 4 x 57,300 123 / 130 (14), 2 uneven of
+//   235,000 125 / 146 (14).
+// One replica with a chain, whose blocks meet twice a step: 100,000 beads
+// 83 / 83, 160,000 107 / 121.  NPT evaluates energies every step: 160,000 123 /
+// 149, 8 x 25,000 136 / 144.
+struct ResidentLoad {
+  static constexpr int kOne = 8, kLarge = 10, kMedium = 16, kSmall = 21, kChained = 25, kApart = 28;
+  static constexpr int kLargeChunks = 100, kMediumChunks = 13, kMediumChained = 24, kApartChained = 200;
+};
+// The chunks in all up to which the form was measured.
 constexpr int kResidentChunks = 2000, kResidentPerReplica = 40;
 constexpr int kResidentPerBlock = 5;  // and at most this many chunks per block
 // A resident rebuild walks the replica's home cells, empty ones too, with its
@@ -733,13 +752,14 @@ void Batch::check_status(int r, bool throw_on_fault) {
 // How k_steps takes the replicas for which runs(r) holds, if it does: with a
 // block per tile where all fit the GPU at once, else with the fewest chunks
 // per block for which every group does, within the limits at the constants
-// above; beyond them the graph's grids are the better form.
+// above; beyond them the graph's grids are the better form.  lifted: as if no
+// replica had a forced rebuild cadence.
 template <typename F>
-Batch::Resident Batch::resident_form(F runs) const {
+Batch::Resident Batch::resident_form(F runs, bool lifted) const {
   Resident f;
   int groups = 0, atoms = 0, most = 0;
   int64_t tiles = 0, chunks = 0;
-  bool chained = false, npt = false;
+  bool chained = false, npt = false, apart = true;
   for (int r = 0; r < max_reps_; ++r) {
     if (!runs(r)) continue;
     const Rep& R = h_reps_[r];
@@ -750,6 +770,7 @@ Batch::Resident Batch::resident_form(F runs) const {
     most = std::max(most, R.nchunks);
     chained |= R.mode == kModeRun && R.ensemble != FMD_LANGEVIN;
     npt |= R.mode == kModeRun && R.ensemble == FMD_NPT_NH;
+    apart &= lifted || R.max_between == kNoForcedRebuild;
   }
   if (graph_steps_ <= 0 || groups == 0) return f;
   auto few_cells = [&](int per_block) {  // of every replica, for so many chunks per block (0: a tile)
@@ -773,13 +794,24 @@ Batch::Resident Batch::resident_form(F runs) const {
   const int64_t limit = kResidentChunks + (int64_t)kResidentPerReplica * groups;
   if (groups > cap || npt || (chained && groups == 1) || chunks > std::min<int64_t>(limit, kResidentPerBlock * cap))
     return f;
+  int64_t blocks = groups;
   for (f.per_block = (int)((chunks + cap - 1) / cap); f.per_block < most; ++f.per_block) {
-    int64_t blocks = 0;
+    blocks = 0;
     for (int r = 0; r < max_reps_; ++r)
       if (runs(r)) blocks += (h_reps_[r].nchunks + f.per_block - 1) / f.per_block;
     if (blocks <= cap) break;
+    blocks = groups;
   }
-  f.fits = few_cells(f.per_block);
+  if (f.per_block > kResidentPerBlock) return f;
+  using Load = ResidentLoad;
+  const int64_t sms = num_sms(), load = (blocks + sms - 1) / sms * f.per_block;
+  const int64_t each = chunks / groups;
+  int64_t heaviest = chained ? Load::kChained : Load::kSmall;
+  if (groups == 1) heaviest = Load::kOne;
+  else if (apart && (!chained || each <= Load::kApartChained)) heaviest = Load::kApart;
+  else if (each > Load::kLargeChunks) heaviest = Load::kLarge;
+  else if (each > (chained ? Load::kMediumChained : Load::kMediumChunks)) heaviest = Load::kMedium;
+  f.fits = load <= heaviest && few_cells(f.per_block);
   return f;
 }
 
@@ -788,7 +820,7 @@ Batch::Resident Batch::resident_form(F runs) const {
 bool Batch::plan_resident() {
   if (!steps_variant(force_variant_)) return false;
   auto runs = [&](int r) { return info_[r].used && h_reps_[r].active && h_reps_[r].step < h_reps_[r].stop_step; };
-  resident_ = resident_form(runs);
+  resident_ = resident_form(runs, false);
   if (!resident_.fits) return false;
   new_plan_.clear();
   for (int r = 0; r < max_reps_; ++r) {
@@ -1051,8 +1083,9 @@ int Batch::autotune(int iters, double* ms_out, int cap) {
   nbr_variant_ = nb;
   int best = 0;
   double best_ms = 0;
-  // a batch that k_steps takes keeps to the variants built in that form
-  const bool resident = resident_form([&](int r) { return info_[r].used && h_reps_[r].active; }).fits;
+  // a batch that k_steps takes (with the cadence lifted, as below) keeps to the
+  // variants built in that form
+  const bool resident = resident_form([&](int r) { return info_[r].used && h_reps_[r].active; }, true).fits;
   for (int v = 0; v < kForceVariants; ++v) {
     const double ms = time_force(iters, v, true);
     if (ms_out && v < cap) ms_out[v] = ms;

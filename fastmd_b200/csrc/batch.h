@@ -144,7 +144,7 @@ class Batch {
     int per_block = 1, stage = 0;
   };
   template <typename F>
-  Resident resident_form(F runs) const;
+  Resident resident_form(F runs, bool lifted) const;
   bool plan_resident();
   bool clear_expired();
   void ensure_graph();

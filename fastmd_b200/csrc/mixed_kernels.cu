@@ -3630,7 +3630,6 @@ __global__ void __launch_bounds__(kNbrThreads) k_neighbors_g(Dev d) {
 }
 
 // ---------------------------------------------------------------- launchers
-namespace {
 int num_sms() {
   int dev = 0;
   FMD_CUDA(cudaGetDevice(&dev));
@@ -3640,6 +3639,7 @@ int num_sms() {
   return cache[dev];
 }
 
+namespace {
 // Blocks of a persistent (grid-stride) kernel: exactly the number that are
 // resident at once, so no block waits for a second wave.
 template <typename K>

@@ -23,11 +23,13 @@ def _chains(nchains, density, length=10):
                          bond_type=np.zeros(len(bonds), np.int32))
 
 
-def _resident(melts, steps=100):
+def _resident(melts, steps=100, apart=False):
     sides = [max(1, int(m.box_L / 2.8)) for m in melts]
     cells = sum((1 << max(0, s - 1).bit_length()) ** 3 for s in sides)  # a capacity of four cells per atom
     b = fm.Batch(max_replicas=len(melts), max_atoms=max(sum(len(m.type) + 256 for m in melts), cells // 4) + 4096)
     slots = [b.add(run_conf(angle=None, nsteps=10_000), desc=m) for m in melts]
+    for s in slots if apart else []:
+        b.set_rebuild_cadence(s, 0)
     before = b.launch_counts()["pre"]
     b.run(steps)
     ran = b.launch_counts()["pre"] - before
@@ -44,3 +46,13 @@ def _resident(melts, steps=100):
 ])
 def test_sparse_boxes(replicas, chains, density, resident):
     assert _resident([_chains(chains, density)] * replicas) == resident
+
+
+@pytest.mark.parametrize("replicas, beads, apart, resident", [
+    (1, 100_000, False, True), (1, 160_000, False, False),
+    (3, 60_000, False, True), (8, 25_000, False, False),
+    (20, 10_000, False, True), (45, 7_000, False, False), (45, 7_000, True, True),
+    (200, 1_000, False, True), (450, 1_000, False, False), (450, 1_000, True, False),
+])
+def test_load(replicas, beads, apart, resident):
+    assert _resident([_chains(beads // 10, 0.3)] * replicas, 50, apart) == resident
