@@ -64,7 +64,11 @@ constexpr int kResidentPerBlock = 5;  // and at most this many chunks per block
 // 65 / 70 (102).  A melt at 0.85 has at most 6 per chunk of a block.
 constexpr int kResidentAxis = 32;  // sort cells per axis
 constexpr int kTileCells = 200, kBlockCells = 100;  // home cells per block
-constexpr int kResidentSteps = 1000;  // steps per k_steps launch
+// Steps per k_steps launch: alone on the device, and beside other batches that
+// step so, which wait 5 to 30 ms for their turn then (a block per tile, and
+// otherwise).  Few launches are better beside ordinary kernels: each waits
+// until all its blocks have room at once.
+constexpr int kResidentSteps = 1000, kTileSteps = 400, kBlockSteps = 200;
 constexpr int kReadPiece = 8192;      // atoms per piece of a state readout (480 KB)
 
 // ------------------------------------------------------------- allocator
@@ -232,6 +236,8 @@ Batch::Batch(const fmd_batch_opts& o, const BatchCaps* exact) {
 }
 
 Batch::~Batch() {
+  if (st_ && ticket_.device >= 0) cudaStreamSynchronize(st_);  // left queued by a run that threw
+  ticket_.finished();
   if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
   for (auto& e : ev_)
     if (e) cudaEventDestroy(e);
@@ -650,6 +656,7 @@ void Batch::finish_pushoffs() {
   upload_reps();
   advance(steps);
   FMD_CUDA(cudaStreamSynchronize(st_));
+  ticket_.finished();
   download_reps();
   clear_expired();
   complete_pushoffs(pend);
@@ -870,9 +877,13 @@ void Batch::advance(int64_t nsteps) {
   if (plan_resident()) {
     const StepSync sync{reinterpret_cast<unsigned*>(sync_.p), sync_.p + (size_t)max_reps_ * kStepCountWords / 2, tiles_,
                         step_polls_};
+    const int form = step_form(resident_.quads, resident_.stage), blocks = (int)h_plan_.size();
+    const int capacity = steps_resident_blocks(resident_.quads, resident_.stage);
     while (nsteps > 0) {
-      const int k = (int)std::min<int64_t>(nsteps, kResidentSteps);
-      launch_steps(d, plan_, (int)h_plan_.size(), resident_.quads, resident_.stage, sync, force_variant_, k, st_);
+      const Turn turn(ticket_, st_, form, blocks, capacity);
+      const int most = turn.alone() ? kResidentSteps : resident_.quads ? kTileSteps : kBlockSteps;
+      const int k = (int)std::min<int64_t>(nsteps, most);
+      launch_steps(d, plan_, blocks, resident_.quads, resident_.stage, sync, force_variant_, k, st_);
       nsteps -= k;
     }
     return;
@@ -946,6 +957,7 @@ void Batch::run(int64_t nsteps, bool respect_nsteps) {
   upload_reps();
   advance(need);
   FMD_CUDA(cudaStreamSynchronize(st_));
+  ticket_.finished();
   download_reps();
   // A faulted replica stops; the others continue.
   bool changed = clear_expired();

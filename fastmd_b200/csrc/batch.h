@@ -9,6 +9,7 @@
 #include "dev_common.cuh"
 #include "host.h"
 #include "mixed.cuh"
+#include "turns.h"
 
 namespace fmd {
 namespace mixed {
@@ -183,6 +184,7 @@ class Batch {
   DevBuf<unsigned long long> sync_;  // resident steps: barrier words per replica and block,
   DevBuf<double> tiles_;             // and tile sums
   Resident resident_;       // form of the plan
+  TurnTicket ticket_;
   int step_polls_ = kStepPolls;  // of a group barrier
   std::vector<int4> h_plan_, new_plan_;
   // state readout: two device and two pinned buffers of a piece of atoms each

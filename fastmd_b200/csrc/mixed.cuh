@@ -386,6 +386,7 @@ inline int step_tiles(int natoms, int nchunks) {
 }
 constexpr int kStepTileChunks = 304;  // chunks of a replica stepped by tiles (8 blocks on each of 148 SMs, 4 to a chunk)
 int num_sms();  // of the current device
+int step_form(bool quads, int stage_bytes);  // grids of one form may run side by side
 int steps_resident_blocks(bool quads, int stage_bytes);
 bool steps_variant(int force_variant);
 void launch_steps(const Dev& d, const int4* plan, int blocks, bool quads, int stage_bytes, const StepSync& sync,

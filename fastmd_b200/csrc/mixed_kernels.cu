@@ -3668,42 +3668,35 @@ StepKernel step_kernel(bool two, int form) {
        : form == 1 ? (two ? k_steps<2, false, true> : k_steps<1, false, true>)
                    : (two ? k_steps<2, false, false> : k_steps<1, false, false>);
 }
-int step_form(bool quads, int stage_bytes) { return quads ? 2 : stage_bytes > 0 ? 1 : 0; }
 
-// Per device: whether the kernels' attributes are set, and the event after the
-// last k_steps launch of any batch of the process.  Two cooperative grids that
-// each got part of the SMs would wait for one another, so a launch waits for
-// the one before it, whichever stream that is in.
-struct StepDevice {
-  bool attributes = false;
-  cudaEvent_t last = nullptr;
-};
 std::mutex g_step_mu;
-StepDevice g_step_dev[64];
+bool g_step_attributes[64];  // per device: set
 
-StepDevice& step_device() {
+// Once per device: the carve-out that holds the kernels' shared memory as often
+// as a block fits an SM, one for both kernels of a form (grids of a form run
+// side by side); the rest of the array is L1 for the gathers.
+void step_attributes() {
+  std::lock_guard<std::mutex> lock(g_step_mu);
   int dev = 0;
   FMD_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) throw Error(FMD_ERR_ARG, "device ordinal out of range");
-  return g_step_dev[dev];
-}
-
-// Once per device: the carve-out that holds the kernels' shared memory as often
-// as a block fits an SM; the rest of the array is L1 for the gathers.
-void step_attributes() {
-  std::lock_guard<std::mutex> lock(g_step_mu);
-  StepDevice& sd = step_device();
-  if (sd.attributes) return;
-  for (int form = 0; form < 3; ++form)
+  if (g_step_attributes[dev]) return;
+  for (int form = 0; form < 3; ++form) {
+    size_t most = 0;
     for (bool two : {false, true}) {
       cudaFuncAttributes a;
       FMD_CUDA(cudaFuncGetAttributes(&a, step_kernel(two, form)));
-      const int kb = (int)((a.sharedSizeBytes + 1023) / 1024 + 1) * kStepBlocksPerSM;
-      prefer_l1(step_kernel(two, form), form == 1 ? 100 : std::min(100, (100 * kb + 227) / 228));
+      most = std::max(most, a.sharedSizeBytes);
     }
-  sd.attributes = true;
+    const int kb = (int)((most + 1023) / 1024 + 1) * kStepBlocksPerSM;
+    for (bool two : {false, true})
+      prefer_l1(step_kernel(two, form), form == 1 ? 100 : std::min(100, (100 * kb + 227) / 228));
+  }
+  g_step_attributes[dev] = true;
 }
 }  // namespace
+
+int step_form(bool quads, int stage_bytes) { return quads ? 2 : stage_bytes > 0 ? 1 : 0; }
 
 int steps_resident_blocks(bool quads, int stage_bytes) {
   step_attributes();
@@ -3734,12 +3727,7 @@ void launch_steps(const Dev& d, const int4* plan, int blocks, bool quads, int st
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  std::lock_guard<std::mutex> lock(g_step_mu);
-  StepDevice& sd = step_device();
-  if (!sd.last) FMD_CUDA(cudaEventCreateWithFlags(&sd.last, cudaEventDisableTiming));
-  FMD_CUDA(cudaStreamWaitEvent(st, sd.last, 0));
   FMD_CUDA(cudaLaunchKernelEx(&cfg, step_kernel(two, step_form(quads, stage_bytes)), d, plan, sync, max_steps));
-  FMD_CUDA(cudaEventRecord(sd.last, st));
 }
 
 // The pre-force update of every chunk, one block per chunk.  (A resident
