@@ -841,16 +841,18 @@ bool Batch::plan_resident() {
   if (plan_.n < new_plan_.size()) {
     const size_t room = std::max({(int)new_plan_.size(), steps_resident_blocks(true, 0), steps_resident_blocks(false, 0)});
     FMD_CUDA(cudaStreamSynchronize(st_));
-    plan_.alloc(room);
+    plan_.release();
+    h_plan_.clear();
     tiles_.alloc(6 * room);
     sync_.alloc((size_t)max_reps_ * kStepCountWords / 2 + 2 * room);
-    h_plan_.clear();
+    plan_.alloc(room);  // last: its size says that all three are there
   }
   const bool same = new_plan_.size() == h_plan_.size() &&
                     std::memcmp(new_plan_.data(), h_plan_.data(), h_plan_.size() * sizeof(int4)) == 0;
   if (!same) {
+    h_plan_.clear();
+    FMD_CUDA(cudaMemcpyAsync(plan_, new_plan_.data(), new_plan_.size() * sizeof(int4), cudaMemcpyHostToDevice, st_));
     h_plan_ = new_plan_;
-    FMD_CUDA(cudaMemcpyAsync(plan_, h_plan_.data(), h_plan_.size() * sizeof(int4), cudaMemcpyHostToDevice, st_));
   }
   return true;
 }
@@ -1280,8 +1282,9 @@ void Batch::read_state(int r, double* xyz, double* vel, int32_t* image, bool rew
   for (int k = 0; k < std::min(2, (largest + piece - 1) / piece); ++k) {
     if (read_dev_[k].n < bytes) {
       FMD_CUDA(cudaStreamSynchronize(st_));
-      read_dev_[k].alloc(bytes);
+      read_dev_[k].release();
       read_pin_[k].alloc(bytes);
+      read_dev_[k].alloc(bytes);  // last: its size says that both are there
     }
     if (!read_ev_[k]) FMD_CUDA(cudaEventCreateWithFlags(&read_ev_[k], cudaEventDisableTiming));
   }
