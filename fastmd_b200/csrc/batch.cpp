@@ -791,13 +791,14 @@ Batch::Resident Batch::resident_form(F runs, bool lifted) const {
     }
     return true;
   };
-  if (tiles <= steps_resident_blocks(true, 0) && most <= kStepTileChunks) {
+  f.capacity = steps_resident_blocks(true, 0);
+  if (tiles <= f.capacity && most <= kStepTileChunks) {
     f.fits = f.quads = few_cells(0);
     return f;
   }
   const int64_t stage = ((int64_t)atoms * 16 + 1023) / 1024 * 1024;
   f.stage = stage <= kStepStageBytes ? (int)stage : 0;
-  const int cap = steps_resident_blocks(false, f.stage);
+  const int cap = f.capacity = steps_resident_blocks(false, f.stage);
   const int64_t limit = kResidentChunks + (int64_t)kResidentPerReplica * groups;
   if (groups > cap || npt || (chained && groups == 1) || chunks > std::min<int64_t>(limit, kResidentPerBlock * cap))
     return f;
@@ -880,9 +881,8 @@ void Batch::advance(int64_t nsteps) {
     const StepSync sync{reinterpret_cast<unsigned*>(sync_.p), sync_.p + (size_t)max_reps_ * kStepCountWords / 2, tiles_,
                         step_polls_};
     const int form = step_form(resident_.quads, resident_.stage), blocks = (int)h_plan_.size();
-    const int capacity = steps_resident_blocks(resident_.quads, resident_.stage);
     while (nsteps > 0) {
-      const Turn turn(ticket_, st_, form, blocks, capacity);
+      const Turn turn(ticket_, st_, form, blocks, resident_.capacity);
       const int most = turn.alone() ? kResidentSteps : resident_.quads ? kTileSteps : kBlockSteps;
       const int k = (int)std::min<int64_t>(nsteps, most);
       launch_steps(d, plan_, blocks, resident_.quads, resident_.stage, sync, force_variant_, k, st_);

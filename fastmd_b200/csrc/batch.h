@@ -139,10 +139,11 @@ class Batch {
   void setup(const std::vector<int>& rs);
   void advance(int64_t nsteps);
   // The form in which k_steps takes a set of replicas: whether at all, a block
-  // per tile (quads) or per so many chunks, shared bytes for the positions.
+  // per tile (quads) or per so many chunks, shared bytes for the positions;
+  // the form's blocks that fit the GPU.
   struct Resident {
     bool fits = false, quads = false;
-    int per_block = 1, stage = 0;
+    int per_block = 1, stage = 0, capacity = 0;
   };
   template <typename F>
   Resident resident_form(F runs, bool lifted) const;
