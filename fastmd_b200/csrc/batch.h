@@ -111,7 +111,8 @@ class Batch {
   int graph_steps() const { return graph_steps_; }
   void set_max_between(int r, int k);
   void set_list_prune(int r, double delta);
-  void set_list_buffer(int r, double skin);
+  // forces: re-evaluated after the rebuild (needed where it moves atoms to new slots).
+  void set_list_buffer(int r, double skin, bool forces = true);
   void mark(int which);
   double elapsed_ms();
   // steady: time the flavour each replica needs on ordinary steps (energies
