@@ -826,7 +826,7 @@ Batch::Resident Batch::resident_form(F runs, bool lifted) const {
 // The replicas with steps left as groups of resident blocks; false where the
 // step graph is used instead.
 bool Batch::plan_resident() {
-  if (!steps_variant(force_variant_)) return false;
+  if (!steps_variant(force_variant_, nbr_variant_)) return false;
   auto runs = [&](int r) { return info_[r].used && h_reps_[r].active && h_reps_[r].step < h_reps_[r].stop_step; };
   resident_ = resident_form(runs, false);
   if (!resident_.fits) return false;
@@ -1083,11 +1083,15 @@ double Batch::time_rebuild(int iters, int v) {
 // then every neighbor-list variant on a full rebuild (the step graph is
 // re-captured with the choices).
 int Batch::autotune(int iters, double* ms_out, int cap) {
+  // a batch that k_steps takes (with the cadence lifted, as below) keeps to the
+  // variants built in that form
+  const bool resident = resident_form([&](int r) { return info_[r].used && h_reps_[r].active; }, true).fits;
   int nb = 0;
   double nb_ms = 0;
   for (int v = 0; v < kNbrVariants; ++v) {
     const double ms = time_rebuild(std::max(1, iters / 5), v);
     nbr_ms_[v] = ms;
+    if (resident && !steps_variant(0, v)) continue;
     if (v == 0 || ms < nb_ms) {
       nb = v;
       nb_ms = ms;
@@ -1097,13 +1101,10 @@ int Batch::autotune(int iters, double* ms_out, int cap) {
   nbr_variant_ = nb;
   int best = 0;
   double best_ms = 0;
-  // a batch that k_steps takes (with the cadence lifted, as below) keeps to the
-  // variants built in that form
-  const bool resident = resident_form([&](int r) { return info_[r].used && h_reps_[r].active; }, true).fits;
   for (int v = 0; v < kForceVariants; ++v) {
     const double ms = time_force(iters, v, true);
     if (ms_out && v < cap) ms_out[v] = ms;
-    if (resident && !steps_variant(v)) continue;
+    if (resident && !steps_variant(v, 0)) continue;
     if (v == 0 || ms < best_ms) {
       best = v;
       best_ms = ms;

@@ -369,7 +369,9 @@ void launch_reduce_only(const Dev& d, int nchunks, int nreps, cudaStream_t st, i
 // per atom, a group's blocks sharing the replica's chunks, and with
 // stage_bytes > 0 each keeps the replica's positions in that much shared
 // memory (16 bytes per atom of the largest, at most kStepStageBytes).
-// Force variants with several lanes per atom are not built in this form.
+// Force variants with several lanes per atom, and the row form of the list
+// (which measures from another origin: a pair at the list's edge may round to
+// the other side, and the sums behind it group otherwise), are not built so.
 constexpr int kStepCountWords = 4;
 constexpr int kStepStageBytes = 24 * 1024;  // five blocks per SM
 struct StepSync {
@@ -388,7 +390,7 @@ constexpr int kStepTileChunks = 304;  // chunks of a replica stepped by tiles (8
 int num_sms();  // of the current device
 int step_form(bool quads, int stage_bytes);  // grids of one form may run side by side
 int steps_resident_blocks(bool quads, int stage_bytes);
-bool steps_variant(int force_variant);
+bool steps_variant(int force_variant, int nbr_variant);
 void launch_steps(const Dev& d, const int4* plan, int blocks, bool quads, int stage_bytes, const StepSync& sync,
                   int force_variant, int max_steps, cudaStream_t st);
 void launch_prepare(const Dev& d, int nreps, cudaStream_t st);  // 0 setup, 2 re-evaluation

@@ -3710,7 +3710,9 @@ int steps_resident_blocks(bool quads, int stage_bytes) {
   return n * num_sms();
 }
 
-bool steps_variant(int force_variant) { return force_variant != 9 && force_variant != 10; }
+bool steps_variant(int force_variant, int nbr_variant) {
+  return force_variant != 9 && force_variant != 10 && nbr_variant != 1;
+}
 
 void launch_steps(const Dev& d, const int4* plan, int blocks, bool quads, int stage_bytes, const StepSync& sync,
                   int force_variant, int max_steps, cudaStream_t st) {
