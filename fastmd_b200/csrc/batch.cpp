@@ -1021,6 +1021,7 @@ double Batch::time_force(int iters, int variant, bool steady) {
   for (int r = 0; r < max_reps_; ++r)
     if (info_[r].used && h_reps_[r].active) {
       h_reps_[r].adv = 1;
+      h_reps_[r].L = h_reps_[r].Lpos;  // the positions' box (a barostat has moved L on)
       if (steady) {
         h_reps_[r].force_ev = 0;
         h_reps_[r].thermo_freq = 0;
@@ -1042,6 +1043,9 @@ double Batch::time_force(int iters, int variant, bool steady) {
   FMD_CUDA_LAUNCH();
   mark(1);
   const double ms = elapsed_ms() / std::max(1, iters);
+  // the forces are left behind, and the next step starts from them
+  if (shape().has_table) launch_forces_only(d, nc, variant, true, st_);
+  FMD_CUDA_LAUNCH();
   h_reps_ = saved;
   upload_reps();
   FMD_CUDA(cudaStreamSynchronize(st_));
@@ -1057,7 +1061,10 @@ double Batch::time_rebuild(int iters, int v) {
   for (int r = 0; r < max_reps_; ++r)
     if (info_[r].used && h_reps_[r].active) rs.push_back(r);
   if (rs.empty()) return 0.0;
+  std::vector<double> L;
   for (int r : rs) {
+    L.push_back(h_reps_[r].L);
+    h_reps_[r].L = h_reps_[r].Lpos;  // the positions' box (a barostat has moved L on)
     h_reps_[r].rebuild_now = 1;  // the rebuild kernels act on replicas marked so
     h_reps_[r].maxdisp_bits = 0;
     h_reps_[r].disp_acc = 0.f;
@@ -1075,6 +1082,9 @@ double Batch::time_rebuild(int iters, int v) {
   FMD_CUDA_LAUNCH();
   mark(1);
   const double ms = elapsed_ms() / std::max(1, iters);
+  download_reps();
+  for (size_t k = 0; k < rs.size(); ++k) h_reps_[rs[k]].L = L[k];
+  upload_reps();
   FMD_CUDA(cudaStreamSynchronize(st_));
   return ms;
 }
