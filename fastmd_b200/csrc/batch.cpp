@@ -61,8 +61,11 @@ constexpr int kResidentPerBlock = 5;  // and at most this many chunks per block
 // 45 / 40 (129), at 0.005 53 / 54 (287).  Chunks shared by blocks, 60,000 beads
 // at 0.1 41 / 37 (57), at 0.05 (P = 64) 47 / 67; 64 x 1,000 at 0.05 49 / 42 (91),
 // at 0.02 56 / 61 (274); 64 x 3,000 at 0.1 71 / 67 (111), 20 x 10,000 at 0.1
-// 65 / 70 (102).  A melt at 0.85 has at most 6 per chunk of a block.
-constexpr int kResidentAxis = 32;  // sort cells per axis
+// 65 / 70 (102).  A melt at 0.85 has at most 6 per chunk of a block.  With a
+// skin too narrow for a pruned list a replica rebuilds every few steps: 3,000
+// beads at 0.01 with skin 0.1 (P = 32) 35 / 37, 35,000 of a melt under NPT
+// (whose cells have room to grow: P = 32) 93 / 114, 31,000 (16) 89 / 83.
+constexpr int kResidentAxis = 32, kNarrowAxis = 16;  // sort cells per axis
 constexpr int kTileCells = 200, kBlockCells = 100;  // home cells per block
 // Steps per k_steps launch: alone on the device, and beside other batches that
 // step so, which wait 5 to 30 ms for their turn then (a block per tile, and
@@ -787,7 +790,7 @@ Batch::Resident Batch::resident_form(F runs, bool lifted) const {
       const int64_t home = (int64_t)R.G * R.G * R.G;
       const int64_t room = per_block ? (int64_t)kBlockCells * ((R.nchunks + per_block - 1) / per_block)
                                      : (int64_t)kTileCells * step_tiles(R.natoms, R.nchunks);
-      if (R.P > kResidentAxis || home > room) return false;
+      if (R.P > (R.prune_delta > 0.f ? kResidentAxis : kNarrowAxis) || home > room) return false;
     }
     return true;
   };

@@ -359,8 +359,7 @@ void launch_forces_only(const Dev& d, int nchunks, int variant, bool has_table, 
 // ev, to the energies and virial partials) the force kernel wrote.  sel: 0
 // every replica, 1 replicas not rebuilding this step, 2 rebuilding ones.
 void launch_table(const Dev& d, int nchunks, bool ev, int sel, cudaStream_t st);
-void launch_reduce_only(const Dev& d, int nchunks, int nreps, cudaStream_t st, int mode);
-// Scalars of the next pre-force for replicas whose copy a host upload made stale.
+void launch_reduce_only(const Dev& d, int nchunks, int nreps, cudaStream_t st, int mode);  // 0 setup, 2 re-evaluation
 // Resident steps (k_steps): each replica with steps left is advanced by its
 // own group of blocks, up to max_steps steps in one cooperative launch.
 // plan: per block {replica, rank in its group, blocks of the group, first
@@ -393,7 +392,8 @@ int steps_resident_blocks(bool quads, int stage_bytes);
 bool steps_variant(int force_variant, int nbr_variant);
 void launch_steps(const Dev& d, const int4* plan, int blocks, bool quads, int stage_bytes, const StepSync& sync,
                   int force_variant, int max_steps, cudaStream_t st);
-void launch_prepare(const Dev& d, int nreps, cudaStream_t st);  // 0 setup, 2 re-evaluation
+// Scalars of the next pre-force for replicas whose copy a host upload made stale.
+void launch_prepare(const Dev& d, int nreps, cudaStream_t st);
 
 }  // namespace mixed
 }  // namespace fmd

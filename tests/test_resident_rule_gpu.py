@@ -23,11 +23,11 @@ def _chains(nchains, density, length=10):
                          bond_type=np.zeros(len(bonds), np.int32))
 
 
-def _resident(melts, steps=100, apart=False):
+def _resident(melts, steps=100, apart=False, skin=0.3):
     sides = [max(1, int(m.box_L / 2.8)) for m in melts]
     cells = sum((1 << max(0, s - 1).bit_length()) ** 3 for s in sides)  # a capacity of four cells per atom
     b = fm.Batch(max_replicas=len(melts), max_atoms=max(sum(len(m.type) + 256 for m in melts), cells // 4) + 4096)
-    slots = [b.add(run_conf(angle=None, nsteps=10_000), desc=m) for m in melts]
+    slots = [b.add(run_conf(angle=None, nsteps=10_000, skin=skin), desc=m) for m in melts]
     for s in slots if apart else []:
         b.set_rebuild_cadence(s, 0)
     before = b.launch_counts()["pre"]
@@ -46,6 +46,12 @@ def _resident(melts, steps=100, apart=False):
 ])
 def test_sparse_boxes(replicas, chains, density, resident):
     assert _resident([_chains(chains, density)] * replicas) == resident
+
+
+@pytest.mark.parametrize("density, skin, resident", [(0.05, 0.1, True), (0.02, 0.1, False), (0.02, 0.15, True)])
+def test_narrow_skins(density, skin, resident):
+    # 16 and 32 sort cells per axis; no pruned list with a skin of 0.1
+    assert _resident([_chains(300, density)], skin=skin) == resident
 
 
 @pytest.mark.parametrize("replicas, beads, apart, resident", [
