@@ -580,7 +580,7 @@ void verlet_build_into(const void* pos, int32_t natoms, float box_L, const int32
       cells::k_sorted<float4, float><<<gr, kBlock, 0, st>>>((const float4*)pos, s.sorted, s.cid_sorted, s.start, s.end,
                                                             s.spos, natoms);
       FMD_CUDA_LAUNCH();
-      cells::k_list_cells<float4, float><<<g.ncell, cells::kThreads, 0, st>>>(
+      cells::k_list_cells<float4, float><<<cells::list_grid(natoms, g.ncell), cells::kThreads, 0, st>>>(
           s.spos, s.start, s.end, excl_off, excl_list, neighbors, num_neighbors, natoms, g.nx, rcs2, box_L,
           1.0f / box_L, max_neighbors, overflow_flag, 1);
       FMD_CUDA_LAUNCH();

@@ -985,7 +985,7 @@ class PlainEngine final : public SimEngine {
     if (cells::list_by_cells(n_, nx)) {
       cells::k_sorted<double4, double><<<g, kBlock, 0, st_>>>(pos_, sorted_, scid_, cstart_, cend_, spos_, n_);
       FMD_CUDA_LAUNCH();
-      cells::k_list_cells<double4, double><<<ncell, cells::kThreads, 0, st_>>>(
+      cells::k_list_cells<double4, double><<<cells::list_grid(n_, ncell), cells::kThreads, 0, st_>>>(
           spos_, cstart_, cend_, nb_ ? eoff_.p : nullptr, nb_ ? elist_.p : nullptr, nbr_, cnt_, n_, nx, rcs_ * rcs_, L_,
           1.0 / L_, max_nbr_, status_, kStatusOverflow);
     } else {

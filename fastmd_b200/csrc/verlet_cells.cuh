@@ -4,7 +4,7 @@
 // sorted order; neighbor/verlet_list.cu:154-327).  Both users are compiled
 // without contraction, so the pair predicate rounds as the reference's.
 //
-// k_list_cells, a block per home cell: the 27 cells' atoms are staged in shared
+// k_list_cells, a block per home cell (list_grid): the 27 cells' atoms are staged in shared
 // memory once for the cell's atoms, a warp takes one home atom at a time, its
 // lanes test 32 candidates and a ballot compacts the hits in candidate order.
 // The thread-per-atom form it stands beside follows two dependent loads per
@@ -27,6 +27,16 @@ constexpr int kGroup = 64;  // home atoms per pass
 
 // Cells hold four atoms or more on average, and the 27 cells are distinct.
 inline bool list_by_cells(int n, int nx) { return nx >= 3 && (int64_t)n >= 4ll * nx * nx * nx; }
+
+// A block per home cell and kGroup of its atoms on average: a box of few cells
+// with many atoms each would leave most SMs without a block (20,000 atoms in 27
+// cells, rc + skin 9: 19.3 ms with one block per cell, 2.9 now, 7.0 with a
+// thread per atom).
+inline dim3 list_grid(int n, int ncell) {
+  const long long per_cell = ((long long)n + ncell - 1) / ncell;
+  const long long groups = (per_cell + kGroup - 1) / kGroup;
+  return dim3((unsigned)ncell, (unsigned)(groups < 65535 ? groups : 65535));
+}
 
 // Key bits of ncell cell numbers (radix passes over the others are left out).
 inline int key_bits(int ncell) {
@@ -94,7 +104,7 @@ __global__ void __launch_bounds__(kThreads) k_list_cells(const V4* spos, const i
                                                          int nx, Real rcs2, Real L, Real inv_L, int max_nbr,
                                                          int* overflow, int overflow_bit) {
   const int hs = start[blockIdx.x], nh = end[blockIdx.x] - hs;
-  if (nh <= 0) return;
+  if (nh <= (int)blockIdx.y * kGroup) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int cx = blockIdx.x % nx, cy = (blockIdx.x / nx) % nx, cz = blockIdx.x / (nx * nx);
   __shared__ V4 s_c[kWin];
@@ -127,7 +137,7 @@ __global__ void __launch_bounds__(kThreads) k_list_cells(const V4* spos, const i
   auto near_home = [&](const V4& p) { return fabs(p.x - ox) < reach && fabs(p.y - oy) < reach && fabs(p.z - oz) < reach; };
   __syncthreads();
   const int total = s_off[27];
-  for (int hg = 0; hg < nh; hg += kGroup) {
+  for (int hg = blockIdx.y * kGroup; hg < nh; hg += gridDim.y * kGroup) {
     const int gn = min(kGroup, nh - hg);
     for (int w0 = 0; w0 < total; w0 += kWin) {
       const int wn = min(kWin, total - w0);

@@ -1,6 +1,6 @@
 """The launcher's Verlet list by cells at the edges of its candidate windows of 768: three cells per axis, so that
 every atom is a candidate of every cell, one atom to either side of one and of two windows, and full lists that span
-three; against the candidate order and FP32 predicate restated in numpy (exact)."""
+three and seven, their cells' atoms shared by up to four blocks; against the candidate order and FP32 predicate restated in numpy (exact)."""
 import ctypes as C
 
 import numpy as np
@@ -12,7 +12,7 @@ from tests.test_list_cells_gpu import F, _expected
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [767, 768, 769, 1536, 1537, 2400])
+@pytest.mark.parametrize("n", [767, 768, 769, 1536, 1537, 2400, 5184, 5200])  # 192 and 193 atoms per cell: three and four blocks
 @pytest.mark.parametrize("dense", [False, True])  # an even box; 300 atoms in one cell (five passes of 64)
 def test_windows(n, dense):
     torch = pytest.importorskip("torch")
