@@ -49,6 +49,15 @@ struct ResidentLoad {
   static constexpr int kOne = 8, kLarge = 10, kMedium = 16, kSmall = 21, kChained = 25, kApart = 28;
   static constexpr int kLargeChunks = 100, kMediumChunks = 13, kMediumChained = 24, kApartChained = 200;
 };
+// With longer lists (a list's capacity M is 160 at density 0.85 and rc + skin
+// 2.8) the graph's force kernel, with more warps per SM and no spills, gains on
+// the resident loops, so the loads count in proportion and the tile form stays
+// up to kTileLists list rows in flight.  Per step at M = 352 (rc 3.5): one of
+// 45,000 beads 72 / 64 (load 3), of 100,000 106 / 113 (6), 20 x 10,000 183 / 204
+// (12); at 480 (rc 4): 64 x 1,000 137 / 119 (4), one of 60,000 101 / 117 (4); by
+// tiles at 480 37,000 beads 83 / 73 (1,157 tiles), at 832 (rc 5) 18,000 beads
+// 115 / 84 (563), 30,000 125 / 132 (938), 64 x 1,000 not by tiles 338 / 360.
+constexpr int kListRef = 160, kListMost = 640, kTileLists = 600'000;
 // The chunks in all up to which the form was measured.
 constexpr int kResidentChunks = 2000, kResidentPerReplica = 40;
 constexpr int kResidentPerBlock = 5;  // and at most this many chunks per block
@@ -768,14 +777,16 @@ template <typename F>
 Batch::Resident Batch::resident_form(F runs, bool lifted) const {
   Resident f;
   int groups = 0, atoms = 0, most = 0;
-  int64_t tiles = 0, chunks = 0;
+  int64_t tiles = 0, chunks = 0, tile_lists = 0, chunk_lists = 0;
   bool chained = false, npt = false, apart = true;
   for (int r = 0; r < max_reps_; ++r) {
     if (!runs(r)) continue;
     const Rep& R = h_reps_[r];
     ++groups;
     tiles += step_tiles(R.natoms, R.nchunks);
+    tile_lists += (int64_t)step_tiles(R.natoms, R.nchunks) * R.M;
     chunks += R.nchunks;
+    chunk_lists += (int64_t)R.nchunks * R.M;
     atoms = std::max(atoms, R.natoms);
     most = std::max(most, R.nchunks);
     chained |= R.mode == kModeRun && R.ensemble != FMD_LANGEVIN;
@@ -796,13 +807,14 @@ Batch::Resident Batch::resident_form(F runs, bool lifted) const {
   };
   f.capacity = steps_resident_blocks(true, 0);
   if (tiles <= f.capacity && most <= kStepTileChunks) {
-    f.fits = f.quads = few_cells(0);
+    f.fits = f.quads = tile_lists <= kTileLists && few_cells(0);
     return f;
   }
   const int64_t stage = ((int64_t)atoms * 16 + 1023) / 1024 * 1024;
   f.stage = stage <= kStepStageBytes ? (int)stage : 0;
   const int cap = f.capacity = steps_resident_blocks(false, f.stage);
   const int64_t limit = kResidentChunks + (int64_t)kResidentPerReplica * groups;
+  if (chunk_lists > kListMost * chunks) return f;
   if (groups > cap || npt || (chained && groups == 1) || chunks > std::min<int64_t>(limit, kResidentPerBlock * cap))
     return f;
   int64_t blocks = groups;
@@ -822,7 +834,7 @@ Batch::Resident Batch::resident_form(F runs, bool lifted) const {
   else if (apart && (!chained || each <= Load::kApartChained)) heaviest = Load::kApart;
   else if (each > Load::kLargeChunks) heaviest = Load::kLarge;
   else if (each > (chained ? Load::kMediumChained : Load::kMediumChunks)) heaviest = Load::kMedium;
-  f.fits = load <= heaviest && few_cells(f.per_block);
+  f.fits = load * std::max(chunk_lists, kListRef * chunks) <= heaviest * kListRef * chunks && few_cells(f.per_block);
   return f;
 }
 

@@ -23,11 +23,12 @@ def _chains(nchains, density, length=10):
                          bond_type=np.zeros(len(bonds), np.int32))
 
 
-def _resident(melts, steps=100, apart=False, skin=0.3):
+def _resident(melts, steps=100, apart=False, skin=0.3, rc=2.5):
     sides = [max(1, int(m.box_L / 2.8)) for m in melts]
     cells = sum((1 << max(0, s - 1).bit_length()) ** 3 for s in sides)  # a capacity of four cells per atom
-    b = fm.Batch(max_replicas=len(melts), max_atoms=max(sum(len(m.type) + 256 for m in melts), cells // 4) + 4096)
-    slots = [b.add(run_conf(angle=None, nsteps=10_000, skin=skin), desc=m) for m in melts]
+    atoms = sum(len(m.type) + 256 for m in melts) * max(1, int(rc / 2) ** 2)  # room for longer lists
+    b = fm.Batch(max_replicas=len(melts), max_atoms=max(atoms, cells // 4) + 4096)
+    slots = [b.add(run_conf(angle=None, nsteps=10_000, skin=skin, rc=rc), desc=m) for m in melts]
     for s in slots if apart else []:
         b.set_rebuild_cadence(s, 0)
     before = b.launch_counts()["pre"]
@@ -52,6 +53,14 @@ def test_sparse_boxes(replicas, chains, density, resident):
 def test_narrow_skins(density, skin, resident):
     # 16 and 32 sort cells per axis; no pruned list with a skin of 0.1
     assert _resident([_chains(300, density)], skin=skin) == resident
+
+
+# at density 0.3 a list has room for 256 entries with rc 4.5, for 416 with 5.5 and for 768 with 7
+@pytest.mark.parametrize("replicas, beads, rc, resident", [
+    (1, 18_000, 7.0, True), (1, 30_000, 7.0, False), (64, 1_000, 7.0, False),  # tiles, too many of them, chunks
+    (20, 5_000, 4.5, True), (20, 10_000, 4.5, False), (1, 100_000, 5.5, False)])
+def test_long_lists(replicas, beads, rc, resident):
+    assert _resident([_chains(beads // 10, 0.3)] * replicas, 20, rc=rc) == resident
 
 
 @pytest.mark.parametrize("replicas, beads, apart, resident", [
